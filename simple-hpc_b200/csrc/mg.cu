@@ -8,9 +8,10 @@
 // needs no host round trip. Every kernel is a template on the element type: double gives the
 // reference's bits; float is the mixed-precision mode's V-cycle (sums and norms still in double).
 // The float V-cycle also has its own tail: the small levels held in shared memory
-// (k_mg_tail_smem), the coarsest solve in one warp with FP64 tree sums (warp_coarse_core).
+// (k_mg_tail_smem). The coarsest solve has a kernel of its own, and a device function inside the
+// tails, with a cell pair per thread in registers (mg_coarse.cuh).
 #include "kernels.hpp"
-#include "blocksum.cuh"
+#include "mg_coarse.cuh"
 
 #include <cooperative_groups.h>
 
@@ -244,69 +245,26 @@ __device__ inline SLevel slevel_at(unsigned char* base, int nx, int ny) {
     return v;
 }
 
-// The float V-cycle's coarse_solve in one warp on a shared-memory level: the same red-black
-// sweeps, stopping test (||b - A x|| < tol ||b|| or 200 sweeps) and mean removals as
-// cta_coarse_solve, but no block barrier per pass, which on a level of a few cells is most of a
-// pass's cost. Its sums are FP64: each lane adds its cells in order and a fixed xor-shuffle tree
-// combines the lanes (not the reference's row chain, which only the FP64 V-cycle needs).
-__device__ void warp_coarse_core(const SLevel& L, double tol, int* sweeps_out) {
-    const int lane = static_cast<int>(threadIdx.x) & 31;
-    const int n = L.nx * L.ny, S = L.S;
-    auto at = [&](int k) {
-        const int I = k / L.ny;
-        return L.at(I, k - I * L.ny);
-    };
-    auto sum = [&](auto f) {
-        double a = 0.0;
-        for (int k = lane; k < n; k += 32) a += f(at(k));
-        return warp_sum(a);
-    };
-    float *sx = L.x, *sb = L.b, *sap = L.ap;
-    const float4* sl = L.l4;
-    auto smooth = [&](int colour) {
-        for (int k = lane; k < n; k += 32) {
-            const int I = k / L.ny, J = k - I * L.ny;
-            if (((I + J) & 1) != colour) continue;
-            const int q = L.at(I, J);
-            const float4 a = sl[q];
-            sx[q] = rb_value(sb[q], a.x * sx[q + 1] + a.y * sx[q - 1] + a.w * sx[q + S] + a.z * sx[q - S], sap[q]);
-        }
-        __syncwarp();
-    };
-    const double dn = static_cast<double>(L.nx) * L.ny;
-    const double mb = sum([&](int q) { return static_cast<double>(sb[q]); }) / dn;
-    for (int k = lane; k < n; k += 32) {
-        const int q = at(k);
-        sb[q] = static_cast<float>(sb[q] - mb);
-    }
-    __syncwarp();
-    const double bb = sum([&](int q) {
-        const double v = sb[q];
-        return v * v;
-    });
-    int sweeps = 0;
-    if (bb > 0.0) {
-        const double bn = sqrt(bb);
-        while (sweeps < 200) {
-            smooth(0);
-            smooth(1);
-            ++sweeps;
-            const double rr = sum([&](int q) {
-                const float4 a = sl[q];
-                const double r = sb[q] - (sap[q] * sx[q] - (a.x * sx[q + 1] + a.y * sx[q - 1] + a.w * sx[q + S] +
-                                                            a.z * sx[q - S]));
-                return r * r;
-            });
-            if (sqrt(rr) < tol * bn) break;
-        }
-    }
-    const double mx = sum([&](int q) { return static_cast<double>(sx[q]); }) / dn;
-    for (int k = lane; k < n; k += 32) {
-        const int q = at(k);
-        sx[q] = static_cast<float>(sx[q] - mx);
-    }
-    __syncwarp();
-    if (lane == 0 && sweeps_out) *sweeps_out = sweeps;
+// The coarsest solve on a shared level by the first coarse_threads() threads of the block: its scratch
+// is the level's own link array, which the solve has read into registers before it writes there (for
+// every level the links take more than the scratch).
+[[maybe_unused]] __device__ void s_coarse_solve(const SLevel& L, double tol, int* sweeps_out) {
+    const CoarseCta team{coarse_threads(L.nx, L.ny)};
+    if (static_cast<int>(threadIdx.x) < team.nt)
+        coarse_solve<float>(
+            team, L.nx, L.ny, 0, L.nx, 0, tol, coarse_smem<float>(L.l4, L.nx, L.nx, L.ny),
+            [&](int I, int J) {
+                const int q = L.at(I, J);
+                const float4 a = L.l4[q];
+                return CoarseCell<float>{a.x, a.y, a.z, a.w, L.ap[q], L.b[q], L.x[q]};
+            },
+            [&](int I, int J, float x, float b) {
+                const int q = L.at(I, J);
+                L.x[q] = x;
+                L.b[q] = b;
+            },
+            sweeps_out);
+    __syncthreads();
 }
 
 // Global level L into the shared level s (links, AP; b and x when `values`; zero elsewhere,
@@ -335,40 +293,6 @@ __device__ void slevel_store(const LevelViewT<float>& L, const SLevel& s) {
         const int I = k / L.ny, J = k - I * L.ny;
         L.x[I * L.stride + J] = s.x[s.at(I, J)];
         L.b[I * L.stride + J] = s.b[s.at(I, J)];
-    }
-}
-
-// The coarsest level of the float V-cycle in a global-memory tail: copied to shared memory, solved
-// by one warp, copied back. Levels of up to kWarpCoarseCells cells with their ring.
-constexpr int kWarpCoarseCells = 1024;
-
-[[maybe_unused]] __device__ void warp_coarse_solve(const LevelViewT<float>& L, double tol, int* sweeps_out) {
-    __shared__ __align__(16) unsigned char sm[kWarpCoarseCells * 28];
-    const SLevel s = slevel_at(sm, L.nx, L.ny);
-    if (threadIdx.x < 32) {
-        const int S = s.S, n2 = (L.nx + 2) * S;
-        for (int k = threadIdx.x; k < n2; k += 32) {
-            const int I = k / S - 1, J = k % S - 1;
-            const bool in = I >= 0 && I < L.nx && J >= 0 && J < L.ny;
-            const int q = I * L.stride + J;
-            float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (in) {
-                const Links<float> a = links(L, q);
-                l = make_float4(a.e, a.w, a.n, a.s);
-            }
-            s.l4[k] = l;
-            s.ap[k] = in ? L.AP[q] : 0.0f;
-            s.b[k] = in ? L.b[q] : 0.0f;
-            s.x[k] = in ? L.x[q] : 0.0f;
-        }
-        __syncwarp();
-        warp_coarse_core(s, tol, sweeps_out);
-        const int n = L.nx * L.ny;
-        for (int k = threadIdx.x; k < n; k += 32) {
-            const int I = k / L.ny, J = k - I * L.ny;
-            L.x[I * L.stride + J] = s.x[s.at(I, J)];
-            L.b[I * L.stride + J] = s.b[s.at(I, J)];
-        }
     }
 }
 
@@ -438,8 +362,7 @@ __global__ void __launch_bounds__(kCoarseThreads)
         }
         s_residual_restrict(L, sl(l + 1));
     }
-    if (threadIdx.x < 32) warp_coarse_core(sl(nl - 1), tol, sweeps_out);
-    __syncthreads();
+    s_coarse_solve(sl(nl - 1), tol, sweeps_out);
     const float om = static_cast<float>(omega);
     for (int l = nl - 2; l >= first; --l) {
         const SLevel L = sl(l);
@@ -602,8 +525,7 @@ __global__ void __launch_bounds__(kCoarseThreads)
             }
             s_residual_restrict(L, gathered(l + 1));
         }
-        if (threadIdx.x < 32) warp_coarse_core(gathered(nl - 1), tol, sweeps_out);
-        __syncthreads();
+        s_coarse_solve(gathered(nl - 1), tol, sweeps_out);
         for (int l = nl - 2; l >= lg; --l) {
             const SLevel L = gathered(l);
             s_prolong(gathered(l + 1), L, om);
@@ -638,93 +560,33 @@ __global__ void __launch_bounds__(kCoarseThreads)
 }
 #endif
 
-// coarse_solve (multigrid.cpp:120-140) of an FP64 level in one warp on a shared-memory copy, bit for
-// bit the passes of cta_coarse_solve: the same per-cell expressions, and det_sum's order (each row
-// added left to right by one lane, then the row sums in order by lane 0, multigrid.cpp:18-34), so
-// the sweep count and every value equal the reference's; but no block barrier per pass, which on a
-// coarsest level of a few cells is most of a pass's cost. sm: coarse64_bytes(nx, ny) bytes.
-__host__ __device__ inline int coarse64_bytes(int nx, int ny) { return (8 * (nx + 2) * (ny + 2) + nx) * 8; }
+// A level in global memory as coarse_solve's cells.
+template <class T> __device__ CoarseCell<T> coarse_load(const LevelViewT<T>& L, int I, int J) {
+    const int q = I * L.stride + J;
+    const Links<T> k = links(L, q);
+    return {k.e, k.w, k.n, k.s, L.AP[q], L.b[q], L.x[q]};
+}
 
-__device__ void warp_coarse_solve64(const LevelViewT<double>& L, double tol, int* sweeps_out, double* sm) {
-    const int lane = static_cast<int>(threadIdx.x) & 31;
-    const int nx = L.nx, ny = L.ny, S = ny + 2, n2 = (nx + 2) * S, n = nx * ny;
-    double *le = sm, *lw = le + n2, *ln = lw + n2, *ls = ln + n2, *ap = ls + n2, *b = ap + n2, *x = b + n2,
-           *r = x + n2, *rows = r + n2;
-    for (int k = lane; k < n2; k += 32) { // the level with its zero ring
-        const int I = k / S - 1, J = k % S - 1;
-        const bool in = I >= 0 && I < nx && J >= 0 && J < ny;
-        const int q = I * L.stride + J;
-        le[k] = in ? L.AE[q] : 0.0;
-        lw[k] = in ? L.AW[q] : 0.0;
-        ln[k] = in ? L.AN[q] : 0.0;
-        ls[k] = in ? L.AS[q] : 0.0;
-        ap[k] = in ? L.AP[q] : 0.0;
-        b[k] = in ? L.b[q] : 0.0;
-        x[k] = in ? L.x[q] : 0.0;
-        r[k] = 0.0;
-    }
-    __syncwarp();
-    auto at = [&](int I, int J) { return (I + 1) * S + J + 1; };
-    auto det_sum = [&](auto f) {
-        for (int I = lane; I < nx; I += 32) {
-            double a = 0.0;
-            for (int J = 0; J < ny; ++J) a += f(at(I, J));
-            rows[I] = a;
-        }
-        __syncwarp();
-        double t = 0.0;
-        if (lane == 0)
-            for (int I = 0; I < nx; ++I) t += rows[I];
-        t = __shfl_sync(0xffffffffu, t, 0);
-        __syncwarp();
-        return t;
-    };
-    auto remove_mean = [&](double* f) {
-        const double m = det_sum([&](int q) { return f[q]; }) / (static_cast<double>(nx) * ny);
-        for (int k = lane; k < n; k += 32) {
-            const int q = at(k / ny, k % ny);
-            f[q] = f[q] - m;
-        }
-        __syncwarp();
-    };
-    auto smooth = [&](int colour) {
-        for (int k = lane; k < n; k += 32) {
-            const int I = k / ny, J = k % ny;
-            if (((I + J) & 1) != colour) continue;
-            const int q = at(I, J);
-            x[q] = rb_value(b[q], le[q] * x[q + 1] + lw[q] * x[q - 1] + ls[q] * x[q + S] + ln[q] * x[q - S], ap[q]);
-        }
-        __syncwarp();
-    };
-    remove_mean(b);
-    const double bb = det_sum([&](int q) {
-        const double v = b[q];
-        return v * v;
-    });
-    int sweeps = 0;
-    if (bb > 0.0) {
-        const double bn = sqrt(bb);
-        while (sweeps < 200) {
-            smooth(0);
-            smooth(1);
-            ++sweeps;
-            const double rr = det_sum([&](int q) { // the residual (cta_residual's expression), squared
-                const double v = b[q] - (ap[q] * x[q] - (le[q] * x[q + 1] + lw[q] * x[q - 1] + ls[q] * x[q + S] +
-                                                         ln[q] * x[q - S]));
-                r[q] = v;
-                return v * v;
-            });
-            if (sqrt(rr) < tol * bn) break;
-        }
-    }
-    remove_mean(x);
-    for (int k = lane; k < n; k += 32) {
-        const int I = k / ny, J = k % ny, q = I * L.stride + J, c = at(I, J);
-        L.x[q] = x[c];
-        L.b[q] = b[c];
-        L.r[q] = r[c];
-    }
-    if (lane == 0 && sweeps_out) *sweeps_out = sweeps;
+// The coarsest level alone, a cell pair per thread: one CTA, or a cluster of them with the rows split
+// into bands.
+struct CoarseBands {
+    int band[17]; // first row of each CTA's band (band[number of CTAs] = nx)
+    int rows;     // rows of the largest band
+};
+template <class T, class Team>
+__global__ void __launch_bounds__(1024) k_mg_coarse_pairs(LevelViewT<T> L, CoarseBands pl, double tol, int* sweeps_out) {
+    extern __shared__ __align__(16) unsigned char tail_dyn[];
+    const Team team{static_cast<int>(blockDim.x)};
+    const int rank = team.rank(), i0 = pl.band[rank];
+    coarse_solve<T>(
+        team, L.nx, L.ny, i0, pl.band[rank + 1] - i0, rank > 0 ? i0 - pl.band[rank - 1] : 0, tol,
+        coarse_smem<T>(tail_dyn, L.nx, pl.rows, L.ny), [&](int I, int J) { return coarse_load(L, I, J); },
+        [&](int I, int J, T x, T b) {
+            const int q = I * L.stride + J;
+            L.x[q] = x;
+            L.b[q] = b;
+        },
+        sweeps_out);
 }
 
 template <class T>
@@ -738,7 +600,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(LevelViewT<T> L, d
 template <class T>
 __global__ void __launch_bounds__(kCoarseThreads)
     k_mg_tail(MgLevelsT<T> lv, int first, int pre, int post, double omega, double tol,
-              double* rowbuf, int* sweeps_out, int warp64) {
+              double* rowbuf, int* sweeps_out, int pairs) {
     extern __shared__ __align__(16) unsigned char tail_dyn[];
     const int nl = lv.n;
     for (int l = first; l + 1 < nl; ++l) {
@@ -749,19 +611,20 @@ __global__ void __launch_bounds__(kCoarseThreads)
         cta_residual(lv.L[l]);
         cta_restrict(lv.L[l], lv.L[l + 1]);
     }
-    bool warp_solve = false;
-    if constexpr (sizeof(T) == 4)
-        warp_solve = (lv.L[nl - 1].nx + 2) * (lv.L[nl - 1].ny + 2) <= kWarpCoarseCells;
-    if (warp_solve) {
-        if constexpr (sizeof(T) == 4)
-            if (threadIdx.x < 32) warp_coarse_solve(lv.L[nl - 1], tol, sweeps_out);
+    if (pairs) {
+        const LevelViewT<T>& L = lv.L[nl - 1];
+        const CoarseCta team{coarse_threads(L.nx, L.ny)};
         __syncthreads();
-    } else if (warp64) {
-        __threadfence_block(); // the other warps' restriction writes, made visible to warp 0
-        __syncthreads();
-        if constexpr (sizeof(T) == 8)
-            if (threadIdx.x < 32)
-                warp_coarse_solve64(lv.L[nl - 1], tol, sweeps_out, reinterpret_cast<double*>(tail_dyn));
+        if (static_cast<int>(threadIdx.x) < team.nt)
+            coarse_solve<T>(
+                team, L.nx, L.ny, 0, L.nx, 0, tol, coarse_smem<T>(tail_dyn, L.nx, L.nx, L.ny),
+                [&](int I, int J) { return coarse_load(L, I, J); },
+                [&](int I, int J, T x, T b) {
+                    const int q = I * L.stride + J;
+                    L.x[q] = x;
+                    L.b[q] = b;
+                },
+                sweeps_out);
         __syncthreads();
     } else {
         cta_coarse_solve(lv.L[nl - 1], rowbuf, tol, sweeps_out);
@@ -780,12 +643,88 @@ __global__ void __launch_bounds__(kCoarseThreads)
 // The float tail runs with every level in shared memory when they fit (the 64^2-and-below levels
 // of a square grid take about 170 KB); otherwise, and for double, through global memory.
 constexpr int kTailSmemMax = 200 * 1024;
-// Shared memory for the FP64 warp coarse solve (about 1400 cells with their ring).
-constexpr int kCoarse64Max = 96 * 1024;
+// Shared memory of a pair solve: any level of 1024 threads per CTA takes less.
+constexpr int kCoarseSmemMax = 160 * 1024;
+
+// The coarsest level alone, where its pairs fit: one CTA up to 1024 threads (about 2048 cells), then a
+// cluster of 8 CTAs, then of 16 (about 32768 cells); beyond that (or fewer rows than CTAs) false. One
+// CTA's block barrier is a fraction of a cluster barrier, so it goes first; 8 CTAs are the largest
+// portable cluster. 37 x 37 FP64, 200 sweeps: 0.28 ms (one warp on shared memory: 6.31 ms); 75 x 125
+// FP32, 200 sweeps: 0.23 ms in a cluster of 8 (one CTA on global memory: 5.63 ms).
+template <class T>
+bool launch_coarse_pairs(const LevelViewT<T>& L, double tol, int* sweeps_out, cudaStream_t st) {
+    CoarseBands pl{};
+    auto plan = [&](int ctas) {
+        pl.rows = (L.nx + ctas - 1) / ctas;
+        for (int r = 0; r <= ctas; ++r) pl.band[r] = static_cast<int>(static_cast<long long>(r) * L.nx / ctas);
+        return L.nx >= ctas && static_cast<long long>(pl.rows) * coarse_hp(L.ny) <= 1024 &&
+               coarse_smem_bytes<T>(L.nx, pl.rows, L.ny) <= kCoarseSmemMax;
+    };
+    if (plan(1)) {
+        static PerDeviceOnce attr;
+        attr.get([] {
+            SGPU_CUDA(cudaFuncSetAttribute(k_mg_coarse_pairs<T, CoarseCta>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kCoarseSmemMax));
+            return 0;
+        });
+        k_mg_coarse_pairs<T, CoarseCta><<<1, coarse_threads(L.nx, L.ny), coarse_smem_bytes<T>(L.nx, L.nx, L.ny), st>>>(
+            L, pl, tol, sweeps_out);
+        SGPU_LAUNCH();
+        return true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    // clusters of this size that this device runs (0: none), its attributes set once per device
+    auto available = [&](int ctas) {
+        static PerDeviceOnce attr, fit8, fit16;
+        const int ok = attr.get([] {
+            const bool set = cudaFuncSetAttribute(k_mg_coarse_pairs<T, CoarseCluster>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  kCoarseSmemMax) == cudaSuccess &&
+                             cudaFuncSetAttribute(k_mg_coarse_pairs<T, CoarseCluster>,
+                                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+            if (!set) (void)cudaGetLastError();
+            return set ? 1 : 0;
+        });
+        return ok && (ctas == 8 ? fit8 : fit16).get([&] {
+            cfg.gridDim = dim3(ctas);
+            cfg.blockDim = dim3(1024);
+            cfg.dynamicSmemBytes = kCoarseSmemMax;
+            at[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, k_mg_coarse_pairs<T, CoarseCluster>, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                n = 0;
+            }
+            return n;
+        }) > 0;
+    };
+    for (int ctas : {8, 16}) {
+        if (!plan(ctas) || !available(ctas)) continue;
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(coarse_threads(pl.rows, L.ny));
+        cfg.dynamicSmemBytes = static_cast<std::size_t>(coarse_smem_bytes<T>(L.nx, pl.rows, L.ny));
+        cfg.stream = st;
+        at[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+        SGPU_CUDA(cudaLaunchKernelEx(&cfg, k_mg_coarse_pairs<T, CoarseCluster>, L, pl, tol, sweeps_out));
+        SGPU_LAUNCH();
+        return true;
+    }
+    return false;
+}
 
 template <class T>
 void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double omega, double tol,
                     double* rowbuf, int* sweeps_out, cudaStream_t st) {
+    const LevelViewT<T>& Lc = lv.L[lv.n - 1];
+    if (first == lv.n - 1 && launch_coarse_pairs(Lc, tol, sweeps_out, st)) return;
+    // pair solve inside the tail: a thread of the block per pair
+    const bool pairs = static_cast<long long>(Lc.nx) * coarse_hp(Lc.ny) <= kCoarseThreads;
     if constexpr (sizeof(T) == 4) {
         TailSmem ts{};
         int bytes = 0;
@@ -794,8 +733,7 @@ void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double
             bytes += slevel_bytes(lv.L[l].nx, lv.L[l].ny);
         }
         ts.bytes = bytes;
-        const int nc = lv.L[lv.n - 1].nx * lv.L[lv.n - 1].ny;
-        if (lv.n <= 24 && bytes <= kTailSmemMax && nc <= kWarpCoarseCells) {
+        if (lv.n <= 24 && bytes <= kTailSmemMax && pairs) {
             static PerDeviceOnce attr; // the attribute lives in each device's context
             attr.get([] {
                 SGPU_CUDA(cudaFuncSetAttribute(k_mg_tail_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -807,19 +745,13 @@ void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double
             return;
         }
     }
-    // FP64: the coarsest solve in one warp on a shared-memory copy when the level fits
-    int dyn = 0;
-    if constexpr (sizeof(T) == 8) {
-        const int b = coarse64_bytes(lv.L[lv.n - 1].nx, lv.L[lv.n - 1].ny);
-        if (b <= kCoarse64Max) dyn = b;
-        static PerDeviceOnce attr;
-        attr.get([] {
-            SGPU_CUDA(cudaFuncSetAttribute(k_mg_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kCoarse64Max));
-            return 0;
-        });
-    }
-    k_mg_tail<T><<<1, kCoarseThreads, dyn, st>>>(lv, first, pre, post, omega, tol, rowbuf, sweeps_out, dyn > 0 ? 1 : 0);
+    static PerDeviceOnce attr;
+    attr.get([] {
+        SGPU_CUDA(cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoarseSmemMax));
+        return 0;
+    });
+    const int dyn = pairs ? coarse_smem_bytes<T>(Lc.nx, Lc.nx, Lc.ny) : 0;
+    k_mg_tail<T><<<1, kCoarseThreads, dyn, st>>>(lv, first, pre, post, omega, tol, rowbuf, sweeps_out, pairs ? 1 : 0);
     SGPU_LAUNCH();
 }
 template <class T> void launch_mg_build(const LevelViewT<T>& F, const LevelViewT<T>& C, cudaStream_t st) {
@@ -877,6 +809,7 @@ bool cluster_tail_plan(const MgLevelsT<float>& lv, int first, ClusterTailPlan& p
     int lg = first;
     while (lg < nl - 1 && lv.L[lg].nx * lv.L[lg].ny > kGatherCells) ++lg;
     if (lg == first || lv.L[lg].nx * lv.L[lg].ny > kGatherCells) return false;
+    if (lv.L[nl - 1].nx * coarse_hp(lv.L[nl - 1].ny) > kCoarseThreads) return false; // the coarse solve's pairs
     for (int l = first; l < lg; ++l)
         if (lv.L[l].nx != 2 * lv.L[l + 1].nx || lv.L[l].ny != 2 * lv.L[l + 1].ny) return false;
     const int Lc = lg - 1, nxc = lv.L[Lc].nx;
