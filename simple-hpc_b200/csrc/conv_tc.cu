@@ -275,29 +275,50 @@ __global__ void __launch_bounds__(kThreadsTc)
                      : "memory");
 }
 
-// Weight gradient of a 3x3 convolution: dW[co, t, ci] += sum over pixels p of dZ[p, co] X[p + t, ci],
-// for the taps t0 .. t0 + nt - 1 of this CTA (blockIdx.y) and its chunk of `chunk` pixels
-// (blockIdx.x). GEMM with M = 128 (output channels co < Cout, the rest zero rows), N = nt x Cin
-// (column (t, ci)), K = pixels in stages of kWgPix. Both operands are gathered from the NHWC arrays
-// into the K-major core-matrix layout: a thread takes two consecutive pixels of 8 channels (two
-// 16-byte loads) and writes the 8 channel rows' (p, p + 1) pairs as 4-byte stores. The chunk's
-// result is added into the FP32 dW with atomics (as many adds per weight as pixel chunks).
-constexpr int kWgPix = 32; // pixels (K) per stage: two MMAs of K = 16
+// Weight gradient of a 3x3 convolution: dW[co, t, ci] += sum over pixels p of dZ[p, co] X[p + t, ci].
+// A GEMM with M = output channels (128 lanes; rows from Cout on are whatever lies behind the tile and
+// are never read back), N = Cin per tap (taps side by side in TMEM) and K = pixels.
+//  * Layout. Both operands are stored as they lie in memory, channels innermost ("MN-major"): a plane
+//    per 8 channels, 16 bytes per pixel, pixels of a row contiguous. So a tile row is filled with plain
+//    16-byte copies, and a tap is only another start address: one pixel to the side is 16 bytes, one
+//    row up or down another ring slot. X is brought in once for its nine taps (the gather into K-major
+//    tiles that this replaces read it nine times and transposed it with 4-byte stores: that bound it).
+//  * Split. A CTA takes `cw` columns (a multiple of 16, zero-filled past the image), `rows` rows of one
+//    image and `nt` taps (nt Cin <= 512 TMEM columns); it walks down its rows with a ring of kWgAhead + 3
+//    rows of X and kWgAhead + 1 of dZ, filled by cp.async kWgAhead rows ahead of the MMAs. At most 4096
+//    pixels are accumulated before the FP32 adds into dW (vector reductions).
+// Measured: the 14 weight gradients of a training step on 8 images of 256^2, 0.91 ms against 8.42 ms.
+constexpr int kWgAhead = 2;
+constexpr int kWgXRows = kWgAhead + 3, kWgZRows = kWgAhead + 1;
+
+struct WgradPlan {
+    int cw, rows, nt;         // columns, rows and taps per CTA
+    int ctiles, rchunks;      // column tiles and row chunks per image
+    unsigned z_plane, x_plane; // bytes of one 8-channel plane of a tile row
+    unsigned z_row, x_row;     // bytes of one tile row (all planes)
+    int smem;
+};
+
+// Shared-memory descriptor of an MN-major tile without swizzling: `k8` bytes between groups of 8
+// pixels, `mn8` between planes of 8 channels.
+__device__ __forceinline__ uint64_t smem_desc_mn(unsigned addr, unsigned k8, unsigned mn8) {
+    return smem_desc(addr, k8, mn8);
+}
 
 __global__ void __launch_bounds__(kThreadsTc)
-    k_conv_wgrad_tc(const bf16* __restrict__ X, const bf16* __restrict__ dZ, int N, int H, int W, int Cin,
-                    int Cout, int taps_per_cta, float* __restrict__ dW, int chunk, uint32_t tmem_cols,
-                    unsigned* err) {
+    k_conv_wgrad_tc(const bf16* __restrict__ X, const bf16* __restrict__ dZ, int H, int W, int Cin, int Cout,
+                    WgradPlan pl, float* __restrict__ dW, uint32_t tmem_cols, unsigned* err) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bars[2];
+    __shared__ __align__(8) uint64_t bars[3]; // stages in turn; [2] the end of all MMAs
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int t0 = blockIdx.y * taps_per_cta;
-    const int nt = min(taps_per_cta, 9 - t0);
-    const int ncols = nt * Cin; // N
-    const unsigned a_bytes = kM * kWgPix * 2, b_bytes = static_cast<unsigned>(ncols) * kWgPix * 2;
-    unsigned char* a_buf[2] = {smem, smem + a_bytes};
-    unsigned char* b_buf[2] = {smem + 2 * a_bytes, smem + 2 * a_bytes + b_bytes};
+    const int t0 = blockIdx.y * pl.nt, nt = min(pl.nt, 9 - t0);
+    int bx = static_cast<int>(blockIdx.x);
+    const int x0 = (bx % pl.ctiles) * pl.cw;
+    bx /= pl.ctiles;
+    const int y0 = (bx % pl.rchunks) * pl.rows, n = bx / pl.rchunks;
+    const int nrows = min(pl.rows, H - y0);
+    unsigned char* const xring = smem + kWgZRows * pl.z_row;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -309,64 +330,56 @@ __global__ void __launch_bounds__(kThreadsTc)
     if (tid == 0) {
         bar_init(&bars[0], 1);
         bar_init(&bars[1], 1);
+        bar_init(&bars[2], 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    // Rows co >= Cout of both A buffers stay zero: clear both A buffers once.
-    for (unsigned o = tid * 16u; o < 2 * a_bytes; o += kThreadsTc * 16u)
-        *reinterpret_cast<uint4*>(smem + o) = make_uint4(0u, 0u, 0u, 0u);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = tmem_slot;
 
-    const long npix = static_cast<long>(N) * H * W;
-    const long pbeg = static_cast<long>(blockIdx.x) * chunk;
-    const long pend = min(npix, pbeg + chunk);
-    const int stages = static_cast<int>((pend - pbeg + kWgPix - 1) / kWgPix);
-    const uint32_t idesc = instr_desc(ncols, kM);
-    const int co_groups = Cout / 8, ci_groups = Cin / 8;
-    bool gave_up = false;
-    int issued = 0;
-    // a 16-byte group of 8 channels of pixel p (zero past the chunk), and of the pixel tap t away
-    auto zload = [&](long p, int g) -> uint4 {
-        return p < pend ? __ldg(reinterpret_cast<const uint4*>(dZ + p * Cout) + g) : make_uint4(0u, 0u, 0u, 0u);
-    };
-    auto xload = [&](long p, int t, int g) -> uint4 {
-        if (p >= pend) return make_uint4(0u, 0u, 0u, 0u);
-        const int x = static_cast<int>(p % W), y = static_cast<int>((p / W) % H);
-        const long n = p / (static_cast<long>(W) * H);
-        const int ys = y + t / 3 - 1, xs = x + t % 3 - 1;
-        if (ys < 0 || ys >= H || xs < 0 || xs >= W) return make_uint4(0u, 0u, 0u, 0u);
-        return __ldg(reinterpret_cast<const uint4*>(X + ((n * H + ys) * W + xs) * Cin) + g);
-    };
-    // the pair (k, k + 1) of 8 rows r0 .. r0 + 7 from two 8-channel groups lo (pixel k), hi (k + 1)
-    auto scatter = [&](unsigned char* buf, int r0, int k, uint4 lo, uint4 hi) {
-        const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, h[4] = {hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const uint32_t a = (l[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
-            const uint32_t b = (h[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
-            *reinterpret_cast<uint32_t*>(buf + core_off(r0 + e, k >> 3, kWgPix) + (k & 7) * 2) = a | (b << 16);
+    const int gz = Cout / 8, gx = Cin / 8;
+    const long image = static_cast<long>(n) * H * W;
+    // row y of X, columns x0 - 1 .. x0 + cw, into its ring slot (zeros outside the image)
+    auto load_x = [&](int y) {
+        unsigned char* dst = xring + ((y + 1) % kWgXRows) * pl.x_row;
+        const bool yin = y >= 0 && y < H;
+        const int cnt = (pl.cw + 2) * gx;
+        for (int u = tid; u < cnt; u += kThreadsTc) {
+            const int px = u / gx, g = u - px * gx, x = x0 + px - 1;
+            const bool in = yin && x >= 0 && x < W;
+            cp_async16(dst + g * pl.x_plane + px * 16, in ? X + (image + static_cast<long>(y) * W + x) * Cin + 8 * g : X,
+                       in ? 16u : 0u);
         }
+    };
+    auto load_z = [&](int s) {
+        unsigned char* dst = smem + (s % kWgZRows) * pl.z_row;
+        const int cnt = pl.cw * gz;
+        for (int u = tid; u < cnt; u += kThreadsTc) {
+            const int px = u / gz, g = u - px * gz, x = x0 + px;
+            const bool in = x < W;
+            cp_async16(dst + g * pl.z_plane + px * 16,
+                       in ? dZ + (image + static_cast<long>(y0 + s) * W + x) * Cout + 8 * g : dZ, in ? 16u : 0u);
+        }
+    };
+    auto issue = [&](int s) { // what stage s (row y0 + s) adds to the rings; one group per stage
+        if (s < nrows) {
+            if (s == 0) {
+                load_x(y0 - 1);
+                load_x(y0);
+            }
+            load_x(y0 + s + 1);
+            load_z(s);
+        }
+        cp_async_commit();
     };
 
-    for (int s = 0; s < stages; ++s) {
-        const int b = s & 1;
-        if (s >= 2 && !bar_wait(&bars[b], static_cast<unsigned>(((s - 2) >> 1) & 1), err)) gave_up = true;
-        if (!gave_up) {
-            const long p0 = pbeg + static_cast<long>(s) * kWgPix;
-            // A: (k pair, co group) units
-            for (int u = tid; u < (kWgPix / 2) * co_groups; u += kThreadsTc) {
-                const int k = 2 * (u % (kWgPix / 2)), g = u / (kWgPix / 2);
-                scatter(a_buf[b], 8 * g, k, zload(p0 + k, g), zload(p0 + k + 1, g));
-            }
-            // B: (k pair, tap, ci group) units
-            for (int u = tid; u < (kWgPix / 2) * nt * ci_groups; u += kThreadsTc) {
-                const int k = 2 * (u % (kWgPix / 2)), rest = u / (kWgPix / 2);
-                const int g = rest % ci_groups, t = rest / ci_groups;
-                scatter(b_buf[b], t * Cin + 8 * g, k, xload(p0 + k, t0 + t, g), xload(p0 + k + 1, t0 + t, g));
-            }
-        }
+    const uint32_t idesc = instr_desc(Cin, kM) | (1u << 15) | (1u << 16); // A and B MN-major
+    bool gave_up = false;
+    int issued = 0;
+    for (int s = 0; s < kWgAhead; ++s) issue(s);
+    for (int s = 0; s < nrows; ++s) {
+        cp_async_wait<kWgAhead - 1>(); // this thread's copies of stage s have landed
         fence_async_smem();
         if (__syncthreads_or(gave_up ? 1 : 0)) {
             gave_up = true;
@@ -374,40 +387,52 @@ __global__ void __launch_bounds__(kThreadsTc)
         }
         if (tid == 0) {
             fence_after();
-            const unsigned a0 = smem_addr(a_buf[b]), b0 = smem_addr(b_buf[b]);
-#pragma unroll
-            for (int k = 0; k < kWgPix / 16; ++k) {
-                const uint64_t ad = smem_desc(a0 + 256u * k, 128u, kWgPix * 16u);
-                const uint64_t bd = smem_desc(b0 + 256u * k, 128u, kWgPix * 16u);
-                mma_issue(tmem, ad, bd, idesc, (s > 0 || k > 0) ? 1u : 0u);
+            const unsigned za = smem_addr(smem + (s % kWgZRows) * pl.z_row);
+            for (int tl = 0; tl < nt; ++tl) {
+                const int t = t0 + tl;
+                // tap t of pixel x: row y0 + s + t / 3 - 1, ring column x - x0 + 1 + t % 3 - 1
+                const unsigned xa =
+                    smem_addr(xring + ((y0 + s + t / 3) % kWgXRows) * pl.x_row) + static_cast<unsigned>(t % 3) * 16u;
+                for (int k = 0; k < pl.cw / 16; ++k)
+                    mma_issue(tmem + static_cast<uint32_t>(tl * Cin), smem_desc_mn(za + 256u * k, 128u, pl.z_plane),
+                              smem_desc_mn(xa + 256u * k, 128u, pl.x_plane), idesc, (s > 0 || k > 0) ? 1u : 0u);
             }
-            mma_commit(&bars[b]);
+            mma_commit(&bars[s & 1]);
+            if (s == nrows - 1) mma_commit(&bars[2]);
         }
         issued = s + 1;
+        // stage s + kWgAhead refills the slots that stage s - 1 read last
+        if (s >= 1 && s + kWgAhead < nrows &&
+            !bar_wait(&bars[(s - 1) & 1], static_cast<unsigned>(((s - 1) >> 1) & 1), err))
+            gave_up = true;
+        if (!gave_up) issue(s + kWgAhead);
+        else cp_async_commit();
     }
-    if (issued > 0 && !gave_up) {
-        const int s = issued - 1;
-        if (!bar_wait(&bars[s & 1], static_cast<unsigned>((s >> 1) & 1), err)) gave_up = true;
-    }
+    cp_async_wait<0>();
+    if (!gave_up && !bar_wait(&bars[2], 0u, err)) gave_up = true;
     if (__syncthreads_or(gave_up ? 1 : 0)) {
-        if (tid == 0)
-            for (int s = issued - 1; s >= 0 && s >= issued - 2; --s)
-                bar_wait(&bars[s & 1], static_cast<unsigned>((s >> 1) & 1), err);
+        // wait (bounded) for what is in flight before TMEM and shared memory are given back
+        if (tid == 0 && issued > 0) {
+            if (issued < nrows) mma_commit(&bars[2]);
+            bar_wait(&bars[2], 0u, err);
+        }
     } else if (issued > 0) {
         fence_after();
         const int co = warp * 32 + (tid & 31);
         const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-        for (int c0 = 0; c0 < ncols; c0 += 16) {
-            float v[16];
-            tmem_ld16(tmem + lane_base + static_cast<uint32_t>(c0), v);
-            if (co < Cout) {
+        if (warp * 32 < Cout) // uniform in the warp
+            for (int c0 = 0; c0 < nt * Cin; c0 += 16) { // 16 columns of one tap (Cin is a multiple of 16)
+                float v[16];
+                tmem_ld16(tmem + lane_base + static_cast<uint32_t>(c0), v);
+                if (co < Cout) {
+                    float* dst = dW + (static_cast<long>(co) * 9 + t0) * Cin + c0;
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const int col = c0 + e, t = t0 + col / Cin, ci = col % Cin;
-                    atomicAdd(dW + (static_cast<long>(co) * 9 + t) * Cin + ci, v[e]);
+                    for (int e = 0; e < 16; e += 4)
+                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst + e), "f"(v[e]),
+                                     "f"(v[e + 1]), "f"(v[e + 2]), "f"(v[e + 3])
+                                     : "memory");
                 }
             }
-        }
     }
     fence_before();
     __syncthreads();
@@ -418,6 +443,7 @@ __global__ void __launch_bounds__(kThreadsTc)
 
 // Kernel shared memory available for the stage ring (one CTA's share of an SM).
 constexpr int kConvSmemMax = 200 * 1024;
+constexpr int kWgSmemPair = 110 * 1024; // the weight gradient's share with two CTAs on an SM
 
 // Stages of the forward kernel: kc = Cin (or the largest multiple of 16 dividing it that is <= 128),
 // nt = the taps that keep K = nt kc <= 144, and as many buffers (2 or 3) as the ring allows.
@@ -450,22 +476,44 @@ void launch_conv_wgrad_tc(const bf16* X, const bf16* dZ, int N, int H, int W, in
     const auto misaligned = [](const void* q) { return (reinterpret_cast<std::uintptr_t>(q) & 15u) != 0; };
     if (misaligned(X) || misaligned(dZ))
         throw Error(SGPU_E_INVALID, "tensor-core weight gradient: operands must be 16-byte aligned");
-    const long npix = static_cast<long>(N) * H * W;
-    if (npix <= 0) return;
-    const int taps = std::min(9, std::max(1, 256 / Cin)); // N = taps x Cin <= 256
-    int ncols_max = taps * Cin;
+    if (reinterpret_cast<std::uintptr_t>(dW) & 15u)
+        throw Error(SGPU_E_INVALID, "tensor-core weight gradient: dW must be 16-byte aligned");
+    if (static_cast<long>(N) * H * W <= 0) return;
+    WgradPlan pl{};
+    pl.nt = std::min(9, 512 / Cin); // Cin <= 256: two taps at least
+    pl.nt = (9 + (9 + pl.nt - 1) / pl.nt - 1) / ((9 + pl.nt - 1) / pl.nt); // even groups
+    // the widest column tile whose rings fit (two CTAs per SM where that still leaves 64 columns)
+    auto size = [&](int cw) {
+        pl.cw = cw;
+        pl.z_plane = static_cast<unsigned>(cw) * 16u;
+        pl.x_plane = static_cast<unsigned>(cw + 2) * 16u;
+        pl.z_row = pl.z_plane * (Cout / 8);
+        pl.x_row = pl.x_plane * (Cin / 8);
+        // the A descriptor spans 16 planes from any dZ slot, whatever Cout is
+        const unsigned rings = kWgZRows * pl.z_row + kWgXRows * pl.x_row;
+        pl.smem = static_cast<int>(std::max(rings, (kWgZRows - 1) * pl.z_row + 16u * pl.z_plane));
+        return pl.smem;
+    };
+    int cw = std::min(256, (W + 15) / 16 * 16);
+    while (cw > 16 && size(cw) > (cw > 64 ? kWgSmemPair : kConvSmemMax)) cw = (cw / 2 + 15) / 16 * 16;
+    if (size(cw) > kConvSmemMax)
+        throw Error(SGPU_E_INVALID, "tensor-core weight gradient: row ring exceeds shared memory");
+    pl.ctiles = (W + cw - 1) / cw;
+    // rows per CTA: about two CTAs per SM over the layer, at most 4096 pixels each
+    const long want = std::max(1L, 296L / ((9 + pl.nt - 1) / pl.nt) / pl.ctiles);
+    pl.rows = static_cast<int>(std::max(1L, std::min<long>(4096 / cw, (static_cast<long>(N) * H + want - 1) / want)));
+    pl.rows = std::min(pl.rows, H);
+    pl.rchunks = (H + pl.rows - 1) / pl.rows;
     uint32_t cols = 32;
-    while (cols < static_cast<uint32_t>(ncols_max)) cols <<= 1;
-    const int chunk = 4096;
-    const int smem = 2 * (kM * kWgPix * 2) + 2 * (ncols_max * kWgPix * 2);
+    while (cols < static_cast<uint32_t>(pl.nt * Cin)) cols <<= 1;
     static PerDeviceOnce attr;
     attr.get([] {
-        SGPU_CUDA(cudaFuncSetAttribute(k_conv_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       2 * (kM * kWgPix * 2) + 2 * (256 * kWgPix * 2)));
+        SGPU_CUDA(cudaFuncSetAttribute(k_conv_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmemMax));
         return 0;
     });
-    const dim3 grid(static_cast<unsigned>((npix + chunk - 1) / chunk), static_cast<unsigned>((9 + taps - 1) / taps));
-    k_conv_wgrad_tc<<<grid, kThreadsTc, smem, st>>>(X, dZ, N, H, W, Cin, Cout, taps, dW, chunk, cols, err);
+    const dim3 grid(static_cast<unsigned>(static_cast<long>(N) * pl.rchunks * pl.ctiles),
+                    static_cast<unsigned>((9 + pl.nt - 1) / pl.nt));
+    k_conv_wgrad_tc<<<grid, kThreadsTc, pl.smem, st>>>(X, dZ, H, W, Cin, Cout, pl, dW, cols, err);
     SGPU_LAUNCH();
 }
 
