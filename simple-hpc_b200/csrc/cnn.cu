@@ -35,30 +35,70 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-// W'[ci][tap'][co] = W[co][8 - tap'][ci]: the weights of the input-gradient convolution.
-__global__ void k_flip_weights(const bf16* __restrict__ W, bf16* __restrict__ Wf, int Cout, int Cin) {
-    const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= static_cast<long>(Cout) * 9 * Cin) return;
-    const int ci = static_cast<int>(i % Cin);
-    const int tap = static_cast<int>((i / Cin) % 9);
-    const int co = static_cast<int>(i / (9L * Cin));
-    Wf[(static_cast<long>(ci) * 9 + (8 - tap)) * Cout + co] = W[i];
+// W'[ci][tap'][co] = W[co][8 - tap'][ci]: the weights of every input-gradient convolution, in one launch
+// (blockIdx.y: the convolution).
+struct FlipTable {
+    long off[18];
+    int cin[18], cout[18];
+};
+__global__ void k_flip_weights(const bf16* __restrict__ W, bf16* __restrict__ Wf, FlipTable ft) {
+    const int Cin = ft.cin[blockIdx.y], Cout = ft.cout[blockIdx.y], n = Cout * 9 * Cin;
+    const bf16* src = W + ft.off[blockIdx.y];
+    bf16* dst = Wf + ft.off[blockIdx.y];
+    for (int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); i < n;
+         i += static_cast<int>(gridDim.x * blockDim.x)) {
+        const int ci = i % Cin, tap = (i / Cin) % 9, co = i / (9 * Cin);
+        dst[(static_cast<long>(ci) * 9 + (8 - tap)) * Cout + co] = src[i];
+    }
 }
 
-// dZ = dY where the post-activation output Y > 0, else 0 (ReLU backward, in place allowed).
-__global__ void k_relu_back(const bf16* __restrict__ Y, const bf16* dY, bf16* dZ, long n) {
-    const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dZ[i] = __bfloat162float(Y[i]) > 0.0f ? dY[i] : __float2bfloat16(0.0f);
-}
+// ---- gradients of the layers between the convolutions ----
+//
+// Each of these kernels forms the gradient of one convolution's output, zeroes it where that
+// convolution's ReLU was off and adds its sum over the pixels to the bias gradient: one pass over the
+// activations, where the mask, the bias sum and the skip connection's copy and addition each took
+// theirs. A thread keeps one group of 8 channels (16-byte accesses) and strides over the pixels, so
+// the sums stay in registers until the block adds them up. Bound: HBM (a training step on 8 images of
+// 256^2: 171 us together, against 1.19 ms for the passes they replace).
+constexpr int kBackThreads = 256;
 
-// db[c] += sum over pixels of dZ[p, c].
-__global__ void k_bias_grad(const bf16* __restrict__ dZ, long npix, int C, float* __restrict__ db) {
-    const int c = threadIdx.x;
-    if (c >= C) return;
-    float s = 0.0f;
-    for (long p = blockIdx.x; p < npix; p += gridDim.x) s += __bfloat162float(dZ[p * C + c]);
-    atomicAdd(db + c, s);
+__device__ __forceinline__ float bf_at(const uint4& v, int e) {
+    const uint32_t w = (&v.x)[e >> 1];
+    return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
 }
+__device__ __forceinline__ uint4 pack8(const bf16 (&h)[8]) {
+    uint4 r;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const __nv_bfloat162 p{h[2 * k], h[2 * k + 1]};
+        (&r.x)[k] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+    return r;
+}
+// dst[c] += the block's sum of acc over its threads of channel group g (8 channels each; C in all).
+__device__ __forceinline__ void channel_sums(const float (&acc)[8], int g, bool active, float* s, int C, float* dst) {
+    for (int c = static_cast<int>(threadIdx.x); c < C; c += kBackThreads) s[c] = 0.0f;
+    __syncthreads();
+    if (active)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) atomicAdd(&s[8 * g + e], acc[e]);
+    __syncthreads();
+    for (int c = static_cast<int>(threadIdx.x); c < C; c += kBackThreads) atomicAdd(dst + c, s[c]);
+    __syncthreads();
+}
+// The pixels of a thread: first, and the stride over the grid; groups of 8 channels fastest.
+struct Walk {
+    int g;
+    bool active;
+    long first, step;
+    __device__ __forceinline__ explicit Walk(int groups) {
+        const int per = kBackThreads / groups, k = static_cast<int>(threadIdx.x) / groups;
+        g = static_cast<int>(threadIdx.x) - k * groups;
+        active = k < per;
+        first = static_cast<long>(blockIdx.x) * per + k;
+        step = static_cast<long>(gridDim.x) * per;
+    }
+};
 
 // 2x2 average pooling, 8 channels (16 bytes) per thread, 32-bit indices (images of up to 2^31
 // channel values): the forward pass's pooling.
@@ -89,15 +129,34 @@ __global__ void k_pool8(const bf16* __restrict__ X, bf16* __restrict__ Y, int N,
     reinterpret_cast<uint4*>(Y)[i] = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-// Backward of the 2x2 average pooling.
-__global__ void k_pool_back(const bf16* __restrict__ dY, bf16* __restrict__ dX, int N, int H, int W, int C) {
-    const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= static_cast<long>(N) * H * W * C) return;
-    const int c = static_cast<int>(i % C);
-    const long q = i / C;
-    const int x = static_cast<int>(q % W), y = static_cast<int>((q / W) % H);
-    const long b = q / (static_cast<long>(W) * H);
-    dX[i] = __float2bfloat16(0.25f * __bfloat162float(dY[((b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c]));
+// The output gradient of the convolution before a pooling and a skip connection: 0.25 of the pooled
+// pixel's gradient (dP, H/2 x W/2, C channels) plus the skip part of the concatenation's (dcat, channels
+// [Ca, Ca + C)); Y: the convolution's output.
+__global__ void __launch_bounds__(kBackThreads)
+    k_join_back8(const bf16* __restrict__ dP, const bf16* __restrict__ dcat, int Ca, const bf16* __restrict__ Y,
+                 bf16* __restrict__ dY, int N, int H, int W, int C, float* __restrict__ db) {
+    __shared__ float s[256];
+    const int gc = C / 8, ga = Ca / 8;
+    const Walk w(gc);
+    const long npix = static_cast<long>(N) * H * W;
+    float acc[8] = {};
+    if (w.active)
+        for (long q = w.first; q < npix; q += w.step) {
+            const int x = static_cast<int>(q % W), y = static_cast<int>((q / W) % H);
+            const long b = q / (static_cast<long>(W) * H);
+            const uint4 p = reinterpret_cast<const uint4*>(dP)[((b * (H / 2) + y / 2) * (W / 2) + x / 2) * gc + w.g];
+            const uint4 k = reinterpret_cast<const uint4*>(dcat)[q * (ga + gc) + ga + w.g];
+            const uint4 v = reinterpret_cast<const uint4*>(Y)[q * gc + w.g];
+            bf16 h[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float d = __bfloat162float(__float2bfloat16(0.25f * bf_at(p, e)));
+                h[e] = bf_at(v, e) > 0.0f ? __float2bfloat16(d + bf_at(k, e)) : __float2bfloat16(0.0f);
+                acc[e] += __bfloat162float(h[e]);
+            }
+            reinterpret_cast<uint4*>(dY)[q * gc + w.g] = pack8(h);
+        }
+    channel_sums(acc, w.g, w.active, s, C, db);
 }
 
 // Y (H x W, Ca + Cb channels) = [nearest 2x upsampling of A (H/2 x W/2, Ca channels), B (Cb)], 8
@@ -114,33 +173,36 @@ __global__ void k_up_concat8(const bf16* __restrict__ A, int Ca, const bf16* __r
                : reinterpret_cast<const uint4*>(B)[q * gb + (g - ga)];
 }
 
-// Backward of k_up_concat8: dA = sum over the 4 children, dB = copy. One thread per element of dB
-// (dB has twice as many elements as dA).
-__global__ void k_up_concat_back(const bf16* __restrict__ dY, bf16* __restrict__ dA, int Ca,
-                                 bf16* __restrict__ dB, int Cb, int N, int H, int W) {
-    const int C = Ca + Cb;
-    const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const long nb = static_cast<long>(N) * H * W * Cb;
-    const long na = static_cast<long>(N) * (H / 2) * (W / 2) * Ca;
-    if (i < nb) dB[i] = dY[(i / Cb) * C + Ca + (i % Cb)];
-    if (i < na) {
-        const int c = static_cast<int>(i % Ca);
-        const long q = i / Ca;
-        const int Wo = W / 2, Ho = H / 2;
-        const int x = static_cast<int>(q % Wo), y = static_cast<int>((q / Wo) % Ho);
-        const long b = q / (static_cast<long>(Wo) * Ho);
-        float s = 0.0f;
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx)
-                s += __bfloat162float(dY[((b * H + 2 * y + dy) * W + 2 * x + dx) * C + c]);
-        dA[i] = __float2bfloat16(s);
-    }
-}
-
-// a += b (the skip connection's gradient joins the encoder output's).
-__global__ void k_add_bf16(bf16* __restrict__ a, const bf16* __restrict__ b, long n) {
-    const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = __float2bfloat16(__bfloat162float(a[i]) + __bfloat162float(b[i]));
+// The output gradient of the convolution before an upsampling: the sum over a pixel's four children of
+// the upsampled part (channels [0, Ca)) of the concatenation's gradient (dcat, H x W, Ca + Cb channels);
+// Y: the convolution's output (H/2 x W/2).
+__global__ void __launch_bounds__(kBackThreads)
+    k_up_back8(const bf16* __restrict__ dcat, int Ca, int Cb, const bf16* __restrict__ Y, bf16* __restrict__ dA, int N,
+               int H, int W, float* __restrict__ db) {
+    __shared__ float s[256];
+    const int ga = Ca / 8, gc = (Ca + Cb) / 8, Ho = H / 2, Wo = W / 2;
+    const Walk w(ga);
+    const long npix = static_cast<long>(N) * Ho * Wo;
+    float acc[8] = {};
+    if (w.active)
+        for (long q = w.first; q < npix; q += w.step) {
+            const int x = static_cast<int>(q % Wo), y = static_cast<int>((q / Wo) % Ho);
+            const long b = q / (static_cast<long>(Wo) * Ho);
+            const uint4* src = reinterpret_cast<const uint4*>(dcat) + ((b * H + 2 * y) * W + 2 * x) * gc + w.g;
+            const uint4 c[4] = {src[0], src[gc], src[static_cast<long>(W) * gc], src[static_cast<long>(W) * gc + gc]};
+            const uint4 v = reinterpret_cast<const uint4*>(Y)[q * ga + w.g];
+            bf16 h[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float t = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) t += bf_at(c[k], e);
+                h[e] = bf_at(v, e) > 0.0f ? __float2bfloat16(t) : __float2bfloat16(0.0f);
+                acc[e] += __bfloat162float(h[e]);
+            }
+            reinterpret_cast<uint4*>(dA)[q * ga + w.g] = pack8(h);
+        }
+    channel_sums(acc, w.g, w.active, s, Ca, db);
 }
 
 // 1x1 head: out[p] = b + sum over c of w[c] X[p, c] (FP32).
@@ -152,33 +214,50 @@ __global__ void k_head_fwd(const bf16* __restrict__ X, int C, const float* __res
     for (int c = 0; c < C; ++c) s += w[c] * __bfloat162float(X[p * C + c]);
     out[p] = s;
 }
-// Head backward with the mean-squared error folded in: d = 2 (out - t) / npix; dX = d w; dw, db
-// summed over pixels; loss = sum of (out - t)^2 / npix.
-__global__ void k_head_back_mse(const bf16* __restrict__ X, int C, const float* __restrict__ w,
-                                const float* __restrict__ out, const float* __restrict__ target,
-                                bf16* __restrict__ dX, float* __restrict__ dw, float* __restrict__ db,
-                                float* __restrict__ loss, long npix) {
-    __shared__ float sw[128];
-    __shared__ float sb, sl;
-    const long p = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (threadIdx.x < C) sw[threadIdx.x] = 0.0f;
-    if (threadIdx.x == 0) sb = sl = 0.0f;
-    __syncthreads();
-    if (p < npix) {
-        const float diff = out[p] - target[p];
-        const float d = 2.0f * diff / static_cast<float>(npix);
-        for (int c = 0; c < C; ++c) {
-            dX[p * C + c] = __float2bfloat16(d * w[c]);
-            atomicAdd(&sw[c], d * __bfloat162float(X[p * C + c]));
+// Head backward with the mean-squared error folded in: d = 2 (out - t) / npix; dX = d w, zeroed where X
+// (the last convolution's output) is not positive, its sum to db_conv; dw, db summed over pixels; loss =
+// sum of (out - t)^2 / npix.
+__global__ void __launch_bounds__(kBackThreads)
+    k_head_back_mse(const bf16* __restrict__ X, int C, const float* __restrict__ w, const float* __restrict__ out,
+                    const float* __restrict__ target, bf16* __restrict__ dX, float* __restrict__ dw,
+                    float* __restrict__ db, float* __restrict__ db_conv, float* __restrict__ loss, long npix) {
+    __shared__ float s[256];
+    const int gc = C / 8;
+    const Walk k(gc);
+    float wc[8] = {}, aw[8] = {}, ab[8] = {}, tot[2] = {}; // tot: the sums of d and of the loss
+    if (k.active) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wc[e] = w[8 * k.g + e];
+        for (long p = k.first; p < npix; p += k.step) {
+            const float diff = out[p] - target[p];
+            const float d = 2.0f * diff / static_cast<float>(npix);
+            const uint4 v = reinterpret_cast<const uint4*>(X)[p * gc + k.g];
+            bf16 h[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float x = bf_at(v, e);
+                h[e] = x > 0.0f ? __float2bfloat16(d * wc[e]) : __float2bfloat16(0.0f);
+                aw[e] += d * x;
+                ab[e] += __bfloat162float(h[e]);
+            }
+            reinterpret_cast<uint4*>(dX)[p * gc + k.g] = pack8(h);
+            tot[0] += d;
+            tot[1] += diff * diff / static_cast<float>(npix);
         }
-        atomicAdd(&sb, d);
-        atomicAdd(&sl, diff * diff / static_cast<float>(npix));
+    }
+    channel_sums(aw, k.g, k.active, s, C, dw);
+    channel_sums(ab, k.g, k.active, s, C, db_conv);
+    // one channel group's threads hold each pixel once
+    if (threadIdx.x < 2) s[threadIdx.x] = 0.0f;
+    __syncthreads();
+    if (k.active && k.g == 0) {
+        atomicAdd(&s[0], tot[0]);
+        atomicAdd(&s[1], tot[1]);
     }
     __syncthreads();
-    if (threadIdx.x < C) atomicAdd(dw + threadIdx.x, sw[threadIdx.x]);
     if (threadIdx.x == 0) {
-        atomicAdd(db, sb);
-        atomicAdd(loss, sl);
+        atomicAdd(db, s[0]);
+        atomicAdd(loss, s[1]);
     }
 }
 
@@ -378,7 +457,7 @@ UNet::UNet(int base, int levels, unsigned seed) : base_(base), levels_(levels) {
     SGPU_CUDA(cudaMalloc(&m_, sizeof(float) * nparam_));
     SGPU_CUDA(cudaMalloc(&v_, sizeof(float) * nparam_));
     SGPU_CUDA(cudaMalloc(&wb_, sizeof(bf16) * nparam_));
-    SGPU_CUDA(cudaMalloc(&wf_, sizeof(bf16) * max_conv_weights()));
+    SGPU_CUDA(cudaMalloc(&wf_, sizeof(bf16) * nparam_));
     SGPU_CUDA(cudaMalloc(&loss_, sizeof(float)));
     SGPU_CUDA(cudaMalloc(&err_, sizeof(unsigned)));
     SGPU_CUDA(cudaMemset(err_, 0, sizeof(unsigned)));
@@ -417,12 +496,6 @@ void UNet::free_acts() {
     for (void* p : acts_) cudaFree(p);
     acts_.clear();
     n_ = h_ = wd_ = 0;
-}
-
-long UNet::max_conv_weights() const {
-    long m = 0;
-    for (const auto& c : convs_) m = std::max(m, static_cast<long>(c.cout) * 9 * c.cin);
-    return m;
 }
 
 double UNet::flops_per_pixel() const {
@@ -466,7 +539,6 @@ void UNet::shape(int n, int h, int w) {
     dpool_.assign(L, nullptr);
     cat_.assign(L, nullptr);
     dcat_.assign(L, nullptr);
-    skip_.assign(L, nullptr);
     for (int l = 1; l < L; ++l) {
         pool_[l] = abf(px(l) * (base_ << (l - 1)));
         dpool_[l] = abf(px(l) * (base_ << (l - 1)));
@@ -475,7 +547,6 @@ void UNet::shape(int n, int h, int w) {
         const long c = (base_ << (l + 1)) + (base_ << l);
         cat_[l] = abf(px(l) * c);
         dcat_[l] = abf(px(l) * c);
-        skip_[l] = abf(px(l) * (base_ << l));
     }
     in32_ = static_cast<float*>(alloc(2 * px(0), sizeof(float)));
     out_ = static_cast<float*>(alloc(px(0), sizeof(float)));
@@ -518,22 +589,14 @@ void UNet::forward(cudaStream_t st) {
     SGPU_LAUNCH();
 }
 
-// Gradient through conv c given c.dy (gradient of its post-ReLU output): ReLU mask, weight and bias
-// gradients, and (dx != null) the gradient of its input.
-void UNet::conv_back(const Conv& c, const bf16* x_in, bf16* dx, cudaStream_t st) {
+// Gradient through conv c given c.dy (of its pre-activation): the weight gradient and (dx != null) the
+// gradient of its input, which is another convolution's dy (masked, its bias gradient added) if relu_of.
+void UNet::conv_back(const Conv& c, const bf16* x_in, bf16* dx, const Conv* relu_of, cudaStream_t st) {
     const int h = h_ >> c.level, w = wd_ >> c.level;
-    const long np = px(c.level);
-    k_relu_back<<<blocks(np * c.cout), 256, 0, st>>>(c.y, c.dy, c.dy, np * c.cout);
-    SGPU_LAUNCH();
     launch_conv_wgrad_tc(x_in, c.dy, n_, h, w, c.cin, c.cout, g_ + c.w_off, err_, st);
-    k_bias_grad<<<static_cast<unsigned>(std::min<long>(np, 1024)), std::max(32, c.cout), 0, st>>>(c.dy, np, c.cout,
-                                                                                               g_ + c.b_off);
-    SGPU_LAUNCH();
     if (!dx) return;
-    const long nw = static_cast<long>(c.cout) * 9 * c.cin;
-    k_flip_weights<<<blocks(nw), 256, 0, st>>>(wb_ + c.w_off, wf_, c.cout, c.cin);
-    SGPU_LAUNCH();
-    launch_conv_tc(c.dy, n_, h, w, c.cout, wf_, nullptr, dx, c.cin, 0, err_, st);
+    launch_conv_tc(c.dy, n_, h, w, c.cout, wf_ + c.w_off, nullptr, dx, c.cin, 0, err_, st,
+                   relu_of ? relu_of->y : nullptr, relu_of ? g_ + relu_of->b_off : nullptr);
 }
 
 void UNet::backward(cudaStream_t st) {
@@ -541,23 +604,37 @@ void UNet::backward(cudaStream_t st) {
     const int L = levels_;
     SGPU_CUDA(cudaMemsetAsync(g_, 0, sizeof(float) * nparam_, st));
     SGPU_CUDA(cudaMemsetAsync(loss_, 0, sizeof(float), st));
+    FlipTable ft{};
+    for (std::size_t c = 0; c < convs_.size(); ++c) {
+        ft.off[c] = convs_[c].w_off;
+        ft.cin[c] = convs_[c].cin;
+        ft.cout[c] = convs_[c].cout;
+    }
+    k_flip_weights<<<dim3(32, static_cast<unsigned>(convs_.size())), 256, 0, st>>>(wb_, wf_, ft);
+    SGPU_LAUNCH();
+    // blocks of a strided pass over npix pixels of `channels` channels: at most four per SM
+    auto strided = [](long npix, int channels) {
+        const long per = kBackThreads / (channels / 8);
+        return static_cast<unsigned>(std::min<long>((npix + per - 1) / per, 592));
+    };
     std::size_t k = convs_.size();
     const Conv& last = convs_[k - 1];
-    k_head_back_mse<<<blocks(px(0)), 256, 0, st>>>(last.y, base_, w_ + head_w_, out_, target_, last.dy,
-                                                  g_ + head_w_, g_ + head_b_, loss_, px(0));
+    k_head_back_mse<<<strided(px(0), base_), kBackThreads, 0, st>>>(last.y, base_, w_ + head_w_, out_, target_, last.dy,
+                                                                   g_ + head_w_, g_ + head_b_, g_ + last.b_off, loss_,
+                                                                   px(0));
     SGPU_LAUNCH();
     // Decoder, finest level first (the reverse of the forward order).
     for (int l = 0; l <= L - 2; ++l) {
         k -= 2;
         const Conv& c1 = convs_[k];
         const Conv& c2 = convs_[k + 1];
-        conv_back(c2, c1.y, c1.dy, st);
-        conv_back(c1, cat_[l], dcat_[l], st);
-        // Upsampled part -> the producing convolution's output gradient; skip part -> stashed for
-        // the encoder output of level l.
-        const int ca = base_ << (l + 1), cb = base_ << l;
-        k_up_concat_back<<<blocks(px(l) * cb), 256, 0, st>>>(dcat_[l], convs_[k - 1].dy, ca, skip_[l], cb, n_,
-                                                            h_ >> l, wd_ >> l);
+        conv_back(c2, c1.y, c1.dy, &c1, st);
+        conv_back(c1, cat_[l], dcat_[l], nullptr, st);
+        // The upsampled part is the gradient of the producing convolution's output; the skip part joins
+        // the encoder output of level l below.
+        const Conv& up = convs_[k - 1];
+        k_up_back8<<<strided(px(l + 1), up.cout), kBackThreads, 0, st>>>(dcat_[l], up.cout, base_ << l, up.y, up.dy, n_,
+                                                                       h_ >> l, wd_ >> l, g_ + up.b_off);
         SGPU_LAUNCH();
     }
     // Encoder, coarsest level first.
@@ -566,17 +643,13 @@ void UNet::backward(cudaStream_t st) {
         const Conv& c1 = convs_[k];
         const Conv& c2 = convs_[k + 1];
         if (l < L - 1) {
-            k_add_bf16<<<blocks(px(l) * c2.cout), 256, 0, st>>>(c2.dy, skip_[l], px(l) * c2.cout);
+            k_join_back8<<<strided(px(l), c2.cout), kBackThreads, 0, st>>>(dpool_[l + 1], dcat_[l], base_ << (l + 1),
+                                                                         c2.y, c2.dy, n_, h_ >> l, wd_ >> l, c2.cout,
+                                                                         g_ + c2.b_off);
             SGPU_LAUNCH();
         }
-        conv_back(c2, c1.y, c1.dy, st);
-        conv_back(c1, l == 0 ? in_ : pool_[l], l == 0 ? nullptr : dpool_[l], st);
-        if (l > 0) {
-            const Conv& prev = convs_[k - 1];
-            k_pool_back<<<blocks(px(l - 1) * prev.cout), 256, 0, st>>>(dpool_[l], prev.dy, n_, h_ >> (l - 1),
-                                                                      wd_ >> (l - 1), prev.cout);
-            SGPU_LAUNCH();
-        }
+        conv_back(c2, c1.y, c1.dy, &c1, st);
+        conv_back(c1, l == 0 ? in_ : pool_[l], l == 0 ? nullptr : dpool_[l], nullptr, st);
     }
 }
 

@@ -64,14 +64,14 @@ class UNet {
         int cin, cout, level;
         long w_off = 0, b_off = 0;
         __nv_bfloat16* y = nullptr;  // post-ReLU output
-        __nv_bfloat16* dy = nullptr; // gradient of the output (then of the pre-activation)
+        __nv_bfloat16* dy = nullptr; // gradient of the pre-activation (zero where the ReLU was off)
     };
     void shape(int n, int h, int w);
     void free_acts();
     void refresh_bf16(cudaStream_t st);
     void conv_fwd(const Conv& c, const __nv_bfloat16* x, __nv_bfloat16* y, cudaStream_t st);
-    void conv_back(const Conv& c, const __nv_bfloat16* x_in, __nv_bfloat16* dx, cudaStream_t st);
-    long max_conv_weights() const;
+    // relu_of: the convolution whose output x_in is, if it is a convolution's (dx is then its masked dy).
+    void conv_back(const Conv& c, const __nv_bfloat16* x_in, __nv_bfloat16* dx, const Conv* relu_of, cudaStream_t st);
     long px(int l) const { return static_cast<long>(n_) * (h_ >> l) * (wd_ >> l); }
 
     int base_, levels_;
@@ -79,23 +79,25 @@ class UNet {
     std::vector<Conv> convs_;
     float *w_ = nullptr, *g_ = nullptr, *m_ = nullptr, *v_ = nullptr, *loss_ = nullptr;
     __nv_bfloat16* wb_ = nullptr; // BF16 copy of every parameter
-    __nv_bfloat16* wf_ = nullptr; // flipped weights of one conv (input-gradient pass)
+    __nv_bfloat16* wf_ = nullptr; // flipped weights of every conv (input-gradient pass), at its w_off
     unsigned* err_ = nullptr;      // device word: a tensor-core convolution's bounded wait gave up
     int step_ = 0;
     // activations for the current shape
     int n_ = 0, h_ = 0, wd_ = 0;
     std::vector<void*> acts_;
     __nv_bfloat16* in_ = nullptr;
-    std::vector<__nv_bfloat16*> pool_, dpool_, cat_, dcat_, skip_;
+    std::vector<__nv_bfloat16*> pool_, dpool_, cat_, dcat_;
     float *in32_ = nullptr, *out_ = nullptr, *target_ = nullptr;
 };
 
 // 3x3 convolution, zero padding 1, of NHWC BF16 X [N*H*W][Cin] with W [Cout][9][Cin] (+ bias when not
 // null, ReLU when relu) into Y [N*H*W][Cout], as a tcgen05 implicit GEMM with the accumulator in TMEM
 // (conv_tc.cu). Cin and Cout multiples of 16, Cout <= 256. *err (device) gets a bit if a bounded
-// wait for the MMAs gave up.
+// wait for the MMAs gave up. mask (not null: with db): Y is zeroed where mask [N*H*W][Cout] is not
+// positive, and db[Cout] += the sum of Y over the pixels.
 void launch_conv_tc(const __nv_bfloat16* X, int N, int H, int W, int Cin, const __nv_bfloat16* Wt,
-                    const float* bias, __nv_bfloat16* Y, int Cout, int relu, unsigned* err, cudaStream_t st);
+                    const float* bias, __nv_bfloat16* Y, int Cout, int relu, unsigned* err, cudaStream_t st,
+                    const __nv_bfloat16* mask = nullptr, float* db = nullptr);
 
 // Weight gradient of that convolution, dW [Cout][9][Cin] += sum over pixels of dZ[p, co] X[p + t, ci]
 // (dZ: the pre-activation gradient), as tcgen05 GEMMs over pixel chunks added with FP32 atomics.
