@@ -236,6 +236,13 @@ int stream_seg_rows(const DevParams& p, int sms, int blocks_per_sm = 2, int min_
 // Momentum prep: |R| into cells, AP over the update range, frozen copy xF of x.
 void launch_mom_prep(const DevParams& p, bool v_component, const double* x, const double* oth,
                      const double* pf, double* xF, double* AP, double* cells, cudaStream_t st);
+// A small grid's whole component on one thread-block cluster: |R| into cells, AP over the update range
+// and nsweeps sweeps of x in place; the bits of launch_mom_prep and launch_mom_sweep.
+// mom_cluster_fits: the component fits a cluster's shared memory (about 200^2 cells), and this device
+// runs such clusters.
+bool mom_cluster_fits(const DevParams& p, bool v_component);
+void launch_mom_cluster(const DevParams& p, bool v_component, double* x, const double* oth, const double* pf,
+                        double* AP, double* cells, int nsweeps, cudaStream_t st);
 // One whole multicolour sweep xin -> xout (every cell of xout written).
 void launch_mom_sweep(const DevParams& p, bool v_component, const double* xin, double* xout,
                       const double* xF, const double* oth, const double* pf, int seg_rows,

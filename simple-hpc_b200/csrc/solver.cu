@@ -242,14 +242,24 @@ struct Solver {
         mark(vcomp ? SGPU_PH_BC_V : SGPU_PH_BC_U);
         if (vcomp) launch_bc_v(dp, v, st);
         else launch_bc_u(dp, u, st);
-        mark(vcomp ? SGPU_PH_ASSEMBLE_V : SGPU_PH_ASSEMBLE_U);
         double* cplane = cells + (vcomp ? plane : 0);
+        const bool deferred = defer_sums();
+        const int n = vcomp ? prm.maxit_inner_v : prm.maxit_inner_u;
+        // small grids: assembly, residual and sweeps in one cluster launch (timed as the sweeps)
+        if (n > 0 && mom_cluster_fits(dp, vcomp)) {
+            mark(vcomp ? SGPU_PH_SWEEP_V : SGPU_PH_SWEEP_U);
+            sweep_mark(vcomp, 0, n);
+            launch_mom_cluster(dp, vcomp, x, oth, pf, AP, cplane, n, st);
+            sweep_mark(vcomp, 1, n);
+            mark(vcomp ? SGPU_PH_RESIDUAL_V : SGPU_PH_RESIDUAL_U);
+            momentum_sum(vcomp, res, cplane, deferred);
+            return;
+        }
+        mark(vcomp ? SGPU_PH_ASSEMBLE_V : SGPU_PH_ASSEMBLE_U);
         launch_mom_prep(dp, vcomp, x, oth, pf, xF, AP, cplane, st);
         mark(vcomp ? SGPU_PH_RESIDUAL_V : SGPU_PH_RESIDUAL_U);
-        const bool deferred = defer_sums();
         if (!deferred) momentum_sum(vcomp, res, cplane, false);
         mark(vcomp ? SGPU_PH_SWEEP_V : SGPU_PH_SWEEP_U);
-        const int n = vcomp ? prm.maxit_inner_v : prm.maxit_inner_u;
         double* in = x;
         double* out = tmp;
         sweep_mark(vcomp, 0, n);

@@ -1,0 +1,34 @@
+"""FP64 on small grids, where a component's assembly and sweeps run on one thread-block cluster: every
+cluster size, bands of the fewest rows, ragged columns, both colour counts and sweep counts from one up,
+and the first grid that does not fit. Bit for bit the oracle's."""
+from __future__ import annotations
+
+import pytest
+
+from conftest import bit_equal, config_text, cuda_available, describe_diff, snapshot_config
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")]
+
+
+@pytest.mark.parametrize("nx,ny,scheme,order,inner", [
+    (1, 3, "QUICK", 4, 4), (2, 2, "UDS", 2, 1), (3, 200, "QUICK", 2, 3), (49, 50, "QUICK", 4, 4),
+    (51, 50, "QUICK", 4, 4), (50, 90, "QUICK", 2, 2), (96, 96, "UDS", 2, 4), (130, 101, "QUICK", 4, 5),
+    (200, 199, "QUICK", 4, 4), (215, 215, "QUICK", 4, 4), (32, 1200, "QUICK", 4, 4), (250, 255, "UDS", 2, 4)])
+def test_small_grids_bit_for_bit(sgpu_mod, oracle_mod, nx, ny, scheme, order, inner):
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x=str(nx), N_cells_y=str(ny), Re="700", convection_scheme=scheme, diffusion_order=str(order),
+               momentum_solver="gs_multicolour", pressure_solver="gs_redblack", maxit="6", error_tolerance="0",
+               maxit_inner_u=str(inner), maxit_inner_v=str(inner))
+    p = sgpu_mod.params_from_config(config_text(cfg))
+    o = oracle_mod.Oracle(p)
+    _, _, olog = o.run(6)
+    with sgpu_mod.Solver(p) as g:
+        _, log = g.run(6)
+        assert bit_equal(log, olog), describe_diff(log, olog)
+        for f in (0, 1, 2, sgpu_mod.F_PC, sgpu_mod.CU[8], sgpu_mod.CV[8]):
+            a, b = g.download(f), o.get(f)
+            if f in (sgpu_mod.CU[8], sgpu_mod.CV[8]):  # AP: over the component's own cells
+                r = ((slice(p.H, p.H + nx), slice(p.H + 1, p.H + ny)) if f == sgpu_mod.CU[8]
+                     else (slice(p.H + 1, p.H + nx), slice(p.H + 1, p.H + ny + 1)))
+                a, b = a[r].copy(), b[r].copy()
+            assert bit_equal(a, b), f"field {f}: " + describe_diff(a, b)
