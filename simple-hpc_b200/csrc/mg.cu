@@ -7,8 +7,9 @@
 // norms (coarse_solve, :120-140), which runs inside one CTA so its data-dependent sweep count
 // needs no host round trip. Every kernel is a template on the element type: double gives the
 // reference's bits; float is the mixed-precision mode's V-cycle (sums and norms still in double).
-// The float V-cycle also has its own tail: the small levels held in shared memory
-// (k_mg_tail_smem). The coarsest solve has a kernel of its own, and a device function inside the
+// The small levels of the streaming V-cycle run in one kernel, the tail: in the shared memory of a
+// thread-block cluster (k_mg_tail_cluster) or of one CTA (k_mg_tail_smem), or on global memory in one
+// CTA (k_mg_tail). The coarsest solve has a kernel of its own, and a device function inside the
 // tails, with a cell pair per thread in registers (mg_coarse.cuh).
 #include "kernels.hpp"
 #include "mg_coarse.cuh"
@@ -26,19 +27,25 @@ constexpr int BX = 32, BY = 8;
 
 dim3 grid2(int nx, int ny) { return dim3((ny + BX - 1) / BX, (nx + BY - 1) / BY); }
 
-// mg_build: coarse links are the sums of the two fine links crossing each coarse face.
-template <class T> __global__ void k_mg_build(LevelViewT<T> F, LevelViewT<T> C) {
-    const int J = blockIdx.x * BX + threadIdx.x, I = blockIdx.y * BY + threadIdx.y;
-    if (I >= C.nx || J >= C.ny) return;
-    const int fs = F.stride;
-    const int f = 2 * I * fs + 2 * J, c = I * C.stride + J;
-    const Links<T> k00 = links(F, f), k01 = links(F, f + 1), k10 = links(F, f + fs), k11 = links(F, f + fs + 1);
+// Coarse cell c of mg_build from its four fine cells' links.
+template <class T>
+__device__ __forceinline__ void build_cell(const LevelViewT<T>& C, int c, Links<T> k00, Links<T> k01, Links<T> k10,
+                                           Links<T> k11) {
     const T ae = k01.e + k11.e;
     const T aw = k00.w + k10.w;
     const T an = k00.n + k01.n;
     const T as = k10.s + k11.s;
     set_links(C, c, ae, aw, an, as);
     C.AP[c] = ae + aw + an + as;
+}
+
+// mg_build: coarse links are the sums of the two fine links crossing each coarse face.
+template <class T> __global__ void k_mg_build(LevelViewT<T> F, LevelViewT<T> C) {
+    const int J = blockIdx.x * BX + threadIdx.x, I = blockIdx.y * BY + threadIdx.y;
+    if (I >= C.nx || J >= C.ny) return;
+    const int fs = F.stride;
+    const int f = 2 * I * fs + 2 * J, c = I * C.stride + J;
+    build_cell(C, c, links(F, f), links(F, f + 1), links(F, f + fs), links(F, f + fs + 1));
 }
 
 // One colour of smooth: colour (I + J) & 1, update x = b/AP; x += (E W S N)/AP.
@@ -177,6 +184,16 @@ template <class T> __device__ void cta_restrict(const LevelViewT<T>& F, const Le
     __syncthreads();
 }
 
+// mg_build (multigrid.cpp:232-261) inside one CTA.
+template <class T> __device__ void cta_build(const LevelViewT<T>& F, const LevelViewT<T>& C) {
+    const int n = C.nx * C.ny, fs = F.stride;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const int I = k / C.ny, J = k % C.ny, f = 2 * I * fs + 2 * J;
+        build_cell(C, I * C.stride + J, links(F, f), links(F, f + 1), links(F, f + fs), links(F, f + fs + 1));
+    }
+    __syncthreads();
+}
+
 // prolong (multigrid.cpp:106-116) inside one CTA.
 template <class T>
 __device__ void cta_prolong(const LevelViewT<T>& C, const LevelViewT<T>& F, double omega) {
@@ -219,46 +236,69 @@ __device__ void cta_coarse_solve(const LevelViewT<T>& L, double* rowbuf, double 
     if (threadIdx.x == 0 && sweeps_out) *sweeps_out = sweeps;
 }
 
-// A float level held in shared memory: (nx + 2) x (ny + 2) cells with the zero ring, row stride S,
-// interior cell (I, J) at index (I + 1) * S + J + 1; links {e, w, n, s}, AP, b and x per cell.
-struct SLevel {
+// A level held in shared memory: (nx + 2) x (ny + 2) cells with the zero ring, row stride S, interior
+// cell (I, J) at index (I + 1) * S + J + 1; links {e, w, n, s}, AP, b and x per cell.
+template <class T> struct alignas(16) Link4T {
+    T e, w, n, s;
+};
+template <class T> struct SLevel {
     int nx, ny, S;
-    float4* l4;
-    float *x, *b, *ap;
+    Link4T<T>* l4;
+    T *x, *b, *ap;
     __device__ int at(int I, int J) const { return (I + 1) * S + J + 1; }
+    __device__ T flow(int q) const {
+        const Link4T<T> a = l4[q];
+        return a.e * x[q + 1] + a.w * x[q - 1] + a.s * x[q + S] + a.n * x[q - S];
+    }
 };
 // Bytes of one SLevel block (links first, 16-byte aligned).
-[[maybe_unused]] __host__ __device__ inline int slevel_bytes(int nx, int ny) {
+template <class T> __host__ __device__ inline int slevel_bytes(int nx, int ny) {
     const int n2 = (nx + 2) * (ny + 2);
-    return ((n2 * 28) + 15) / 16 * 16;
+    return (n2 * 7 * static_cast<int>(sizeof(T)) + 15) / 16 * 16;
 }
-__device__ inline SLevel slevel_at(unsigned char* base, int nx, int ny) {
+template <class T> __device__ inline SLevel<T> slevel_at(unsigned char* base, int nx, int ny) {
     const int n2 = (nx + 2) * (ny + 2);
-    SLevel v;
+    SLevel<T> v;
     v.nx = nx;
     v.ny = ny;
     v.S = ny + 2;
-    v.l4 = reinterpret_cast<float4*>(base);
-    v.x = reinterpret_cast<float*>(base + 16 * n2);
+    v.l4 = reinterpret_cast<Link4T<T>*>(base);
+    v.x = reinterpret_cast<T*>(base) + 4 * n2;
     v.b = v.x + n2;
     v.ap = v.b + n2;
     return v;
 }
 
+// The block's threads over rows of `width` cells: a power of two of them per row, so that short rows
+// share a warp and no row index takes a division.
+struct RowWalk {
+    int r, dr, c, dc;
+    __device__ explicit RowWalk(int width) {
+        const int nt = static_cast<int>(blockDim.x), tid = static_cast<int>(threadIdx.x);
+        int sh = width > 1 ? 32 - __clz(width - 1) : 0;
+        while ((1 << sh) > nt) --sh;
+        dc = 1 << sh;
+        dr = nt >> sh;
+        c = tid & (dc - 1);
+        r = tid >> sh;
+        if (r >= dr) r = 1 << 29; // threads past the last whole row (a block that is no power of two)
+    }
+};
+
 // The coarsest solve on a shared level by the first coarse_threads() threads of the block: its scratch
 // is the level's own link array, which the solve has read into registers before it writes there (for
 // every level the links take more than the scratch).
-[[maybe_unused]] __device__ void s_coarse_solve(const SLevel& L, double tol, int* sweeps_out) {
+template <class T> __device__ void s_coarse_solve(const SLevel<T>& L, double tol, int* sweeps_out) {
     const CoarseCta team{coarse_threads(L.nx, L.ny)};
     if (static_cast<int>(threadIdx.x) < team.nt)
-        coarse_solve<float>(
-            team, L.nx, L.ny, 0, L.nx, 0, tol, coarse_smem<float>(L.l4, L.nx, L.nx, L.ny),
+        coarse_solve<T>(
+            team, L.nx, L.ny, 0, L.nx, 0, tol, coarse_smem<T>(L.l4, L.nx, L.nx, L.ny),
             [&](int I, int J) {
                 const int q = L.at(I, J);
-                const float4 a = L.l4[q];
-                return CoarseCell<float>{a.x, a.y, a.z, a.w, L.ap[q], L.b[q], L.x[q]};
+                const Link4T<T> a = L.l4[q];
+                return CoarseCell<T>{a.e, a.w, a.n, a.s, L.ap[q], L.b[q], L.x[q]};
             },
-            [&](int I, int J, float x, float b) {
+            [&](int I, int J, T x, T b) {
                 const int q = L.at(I, J);
                 L.x[q] = x;
                 L.b[q] = b;
@@ -267,36 +307,46 @@ __device__ inline SLevel slevel_at(unsigned char* base, int nx, int ny) {
     __syncthreads();
 }
 
-// Global level L into the shared level s (links, AP; b and x when `values`; zero elsewhere,
-// the ring included), by all threads of the block.
-__device__ void slevel_load(const LevelViewT<float>& L, const SLevel& s, bool values) {
-    const int n2 = (L.nx + 2) * s.S;
+// Rows [g0, g0 + s.nx) of the global level L into the shared band s, by all threads of the block:
+// links and AP with `links`, b and x (its ghost rows too) with `values`; zero elsewhere.
+template <class T> __device__ void slevel_load(const LevelViewT<T>& L, const SLevel<T>& s, int g0, bool link, bool values) {
+    const int n2 = (s.nx + 2) * s.S;
     for (int k = threadIdx.x; k < n2; k += blockDim.x) {
-        const int I = k / s.S - 1, J = k % s.S - 1;
-        const bool in = I >= 0 && I < L.nx && J >= 0 && J < L.ny;
-        const int q = I * L.stride + J;
-        float4 l = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (in) {
-            const Links<float> a = links(L, q);
-            l = make_float4(a.e, a.w, a.n, a.s);
+        const int I = k / s.S - 1, J = k % s.S - 1, g = g0 + I;
+        const bool cin = J >= 0 && J < L.ny, own = cin && I >= 0 && I < s.nx;
+        const int q = g * L.stride + J;
+        Link4T<T> l{T(0), T(0), T(0), T(0)};
+        if (own && link) {
+            const Links<T> a = links(L, q);
+            l = {a.e, a.w, a.n, a.s};
         }
         s.l4[k] = l;
-        s.ap[k] = in ? L.AP[q] : 0.0f;
-        s.b[k] = (in && values) ? L.b[q] : 0.0f;
-        s.x[k] = (in && values) ? L.x[q] : 0.0f;
+        s.ap[k] = own && link ? L.AP[q] : T(0);
+        s.b[k] = (own && values) ? L.b[q] : T(0);
+        s.x[k] = (values && cin && g >= 0 && g < L.nx) ? L.x[q] : T(0);
     }
 }
-// The interior x and b of the shared level back to L.
-__device__ void slevel_store(const LevelViewT<float>& L, const SLevel& s) {
-    const int n = L.nx * L.ny;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const int I = k / L.ny, J = k - I * L.ny;
-        L.x[I * L.stride + J] = s.x[s.at(I, J)];
-        L.b[I * L.stride + J] = s.b[s.at(I, J)];
-    }
+// The band's interior x back to rows g0 on of L.
+template <class T> __device__ void slevel_store_x(const LevelViewT<T>& L, const SLevel<T>& s, int g0) {
+    const RowWalk w(L.ny);
+    for (int I = w.r; I < s.nx; I += w.dr)
+        for (int J = w.c; J < L.ny; J += w.dc) L.x[(g0 + I) * L.stride + J] = s.x[s.at(I, J)];
 }
 
-// ---- the float tail with every level in shared memory ----
+// mg_build (multigrid.cpp:232-261) of the band F into rows c0 on of the coarse level C. No barrier.
+template <class T> __device__ void s_build(const SLevel<T>& F, const SLevel<T>& C, int c0) {
+    const RowWalk w(C.ny);
+    for (int I = w.r; I < F.nx / 2; I += w.dr)
+        for (int J = w.c; J < C.ny; J += w.dc) {
+            const int f = F.at(2 * I, 2 * J), c = C.at(c0 + I, J), S = F.S;
+            const Link4T<T> k00 = F.l4[f], k01 = F.l4[f + 1], k10 = F.l4[f + S], k11 = F.l4[f + S + 1];
+            const Link4T<T> k{k01.e + k11.e, k00.w + k10.w, k00.n + k01.n, k10.s + k11.s};
+            C.l4[c] = k;
+            C.ap[c] = k.e + k.w + k.n + k.s;
+        }
+}
+
+// ---- the tail with every level in the shared memory of one CTA ----
 
 // Byte offset of each tail level's SLevel block in dynamic shared memory, and the total.
 struct TailSmem {
@@ -304,96 +354,94 @@ struct TailSmem {
     int bytes;
 };
 
-// One colour of smooth on a shared level: warps take rows, lanes the colour's cells of a row.
-__device__ void s_smooth(const SLevel& L, int colour) {
-    const int w = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int nw = static_cast<int>(blockDim.x) >> 5, S = L.S;
-    for (int I = w; I < L.nx; I += nw)
-        for (int J = ((I + colour) & 1) + 2 * lane; J < L.ny; J += 64) {
+// One colour of smooth on a shared level.
+template <class T> __device__ void s_smooth(const SLevel<T>& L, int colour) {
+    const RowWalk w((L.ny + 1) / 2);
+    for (int I = w.r; I < L.nx; I += w.dr)
+        for (int J = ((I + colour) & 1) + 2 * w.c; J < L.ny; J += 2 * w.dc) {
             const int q = L.at(I, J);
-            const float4 a = L.l4[q];
-            L.x[q] = rb_value(L.b[q], a.x * L.x[q + 1] + a.y * L.x[q - 1] + a.w * L.x[q + S] + a.z * L.x[q - S],
-                              L.ap[q]);
+            L.x[q] = rb_value(L.b[q], L.flow(q), L.ap[q]);
         }
     __syncthreads();
 }
-// Residual of F (multigrid.cpp:84-85 form) restricted 2x2 into C.b (multigrid.cpp:90-103), C.x = 0.
-__device__ void s_residual_restrict(const SLevel& F, const SLevel& C) {
-    const int w = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int nw = static_cast<int>(blockDim.x) >> 5, S = F.S;
-    auto r = [&](int q) {
-        const float4 a = F.l4[q];
-        return F.b[q] - (F.ap[q] * F.x[q] - (a.x * F.x[q + 1] + a.y * F.x[q - 1] + a.w * F.x[q + S] + a.z * F.x[q - S]));
-    };
-    for (int I = w; I < C.nx; I += nw)
-        for (int J = lane; J < C.ny; J += 32) {
-            const int f = F.at(2 * I, 2 * J), c = C.at(I, J);
+// Residual of F (multigrid.cpp:84-85 form) restricted 2x2 (multigrid.cpp:90-103) into rows c0 on of C, C.x = 0.
+template <class T> __device__ void s_restrict_rows(const SLevel<T>& F, const SLevel<T>& C, int c0) {
+    const RowWalk w(C.ny);
+    const int S = F.S;
+    auto r = [&](int q) { return F.b[q] - (F.ap[q] * F.x[q] - F.flow(q)); };
+    for (int I = w.r; I < F.nx / 2; I += w.dr)
+        for (int J = w.c; J < C.ny; J += w.dc) {
+            const int f = F.at(2 * I, 2 * J), c = C.at(c0 + I, J);
             C.b[c] = r(f) + r(f + 1) + r(f + S) + r(f + S + 1);
-            C.x[c] = 0.0f;
+            C.x[c] = T(0);
         }
-    __syncthreads();
 }
 // prolong (multigrid.cpp:106-116): F.x += omega * C.x of the parent cell.
-__device__ void s_prolong(const SLevel& C, const SLevel& F, float om) {
-    const int w = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int nw = static_cast<int>(blockDim.x) >> 5;
-    for (int i = w; i < F.nx; i += nw)
-        for (int j = lane; j < F.ny; j += 32) F.x[F.at(i, j)] += om * C.x[C.at(i >> 1, j >> 1)];
+template <class T> __device__ void s_prolong(const SLevel<T>& C, const SLevel<T>& F, T om) {
+    const RowWalk w(F.ny);
+    for (int i = w.r; i < F.nx; i += w.dr)
+        for (int j = w.c; j < F.ny; j += w.dc) F.x[F.at(i, j)] += om * C.x[C.at(i >> 1, j >> 1)];
     __syncthreads();
 }
 
-// Levels [first, nl) of one float V-cycle (mg_vcycle, multigrid.cpp:299-323) in one CTA with every
-// level in shared memory: the links, AP, b and x of the first tail level are read once, the passes
-// run against shared memory with a block barrier between them, and x and b of every tail level are
-// written back at the end. Same passes and per-cell expressions as k_mg_tail.
+// Levels [first, nl) of one V-cycle (mg_vcycle, multigrid.cpp:299-323) in one CTA with every level in
+// shared memory: the links, AP, b and x of the first tail level are read once, the coarser operators
+// built from them (build) or read, the passes run against shared memory with a block barrier between
+// them, and x of the first level is written back. Same passes and per-cell expressions as k_mg_tail.
+template <class T>
 __global__ void __launch_bounds__(kCoarseThreads)
-    k_mg_tail_smem(MgLevelsT<float> lv, int first, int pre, int post, double omega, double tol, TailSmem ts,
+    k_mg_tail_smem(MgLevelsT<T> lv, int first, int pre, int post, double omega, double tol, TailSmem ts, int build,
                    int* sweeps_out) {
     extern __shared__ __align__(16) unsigned char tail_sm[];
     const int nl = lv.n;
-    auto sl = [&](int l) { return slevel_at(tail_sm + ts.off[l], lv.L[l].nx, lv.L[l].ny); };
-    for (int l = first; l < nl; ++l) slevel_load(lv.L[l], sl(l), l == first);
+    auto sl = [&](int l) { return slevel_at<T>(tail_sm + ts.off[l], lv.L[l].nx, lv.L[l].ny); };
+    for (int l = first; l < nl; ++l) slevel_load(lv.L[l], sl(l), 0, l == first || !build, l == first);
     __syncthreads();
     for (int l = first; l + 1 < nl; ++l) {
-        const SLevel L = sl(l);
+        const SLevel<T> L = sl(l);
         for (int s = 0; s < pre; ++s) {
             s_smooth(L, 0);
             s_smooth(L, 1);
         }
-        s_residual_restrict(L, sl(l + 1));
+        s_restrict_rows(L, sl(l + 1), 0);
+        if (build) s_build(L, sl(l + 1), 0);
+        __syncthreads();
     }
     s_coarse_solve(sl(nl - 1), tol, sweeps_out);
-    const float om = static_cast<float>(omega);
+    const T om = static_cast<T>(omega);
     for (int l = nl - 2; l >= first; --l) {
-        const SLevel L = sl(l);
+        const SLevel<T> L = sl(l);
         s_prolong(sl(l + 1), L, om);
         for (int s = 0; s < post; ++s) {
             s_smooth(L, 0);
             s_smooth(L, 1);
         }
     }
-    for (int l = first; l < nl; ++l) slevel_store(lv.L[l], sl(l));
+    slevel_store_x(lv.L[first], sl(first), 0);
 }
 
-#ifdef SGPU_FLOAT_UNIT
-// ---- the float tail on a thread-block cluster ----
+// ---- the tail on a thread-block cluster ----
 //
-// Levels [first, lg) of the float V-cycle are split by rows over the kClusterTail CTAs of one
-// cluster, each CTA's band of a level held in its shared memory as an SLevel whose ring rows are
-// ghost copies of the neighbouring bands' edge rows; levels [lg, nl) (at most kGatherCells cells
-// each) and the coarsest solve run on CTA 0 as in k_mg_tail_smem. The passes and per-cell
-// expressions are k_mg_tail_smem's, with a cluster barrier between passes instead of a block
-// barrier. Levels halve exactly (mg_level_dims halves only even sizes), and the bands of the
-// coarsest split level start at even rows, so every band of every split level starts at an even
-// row: a 2 x 2 restriction block and a prolongation parent lie in the CTA's own bands, and the
-// red-black colour of a cell is the parity of its local row plus column. A pass that updates a
-// band's first or last row also stores the value into the ghost row of the neighbouring band
-// (distributed shared memory). In a colour pass the neighbours read only the other colour's ghost
-// cells, and a prolongation reads no ghost cell, so the stores race with no read, and one cluster
-// barrier per pass publishes them.
-constexpr int kClusterTail = 16;        // CTAs per cluster (a non-portable size)
-constexpr int kGatherCells = 1024;      // levels of at most this many cells run on CTA 0
-constexpr int kClusterTailCells = 65536; // the cluster tail takes levels of at most this many cells
+// Levels [first, lg) of the V-cycle are split by rows over the kClusterTail CTAs of one cluster, each
+// CTA's band of a level held in its shared memory as an SLevel whose ring rows are ghost copies of the
+// neighbouring bands' edge rows; levels [lg, nl) (at most kGatherCells cells each) and the coarsest
+// solve run on CTA 0 as in k_mg_tail_smem. The passes and per-cell expressions are k_mg_tail_smem's,
+// with a cluster barrier between passes instead of a block barrier. Levels halve exactly
+// (mg_level_dims halves only even sizes), and the bands of the coarsest split level start at even rows,
+// so every band of every split level starts at an even row: a 2 x 2 restriction block, a coarse
+// operator's block and a prolongation parent lie in the CTA's own bands, and the red-black colour of a
+// cell is the parity of its local row plus column. A pass that updates a band's first or last row also
+// stores the value into the ghost row of the neighbouring band (distributed shared memory). In a
+// colour pass the neighbours read only the other colour's ghost cells, and a prolongation reads no
+// ghost cell, so the stores race with no read, and one cluster barrier per pass publishes them.
+// With `build` the coarse operators are formed here, beside the restriction of each level, from the
+// first level's links (mg_build's sums): no launch per level before the cycle.
+// It is bound by latency: about 0.6 us per pass, 77 us for the double tail from 128^2 against
+// 112 + 50 us for the single-CTA tail from 64^2 and the streamed level above it.
+constexpr int kClusterTail = 16;   // CTAs per cluster (a non-portable size)
+constexpr int kGatherCells = 1024; // levels of at most this many cells run on CTA 0
+// The cluster tail takes levels of at most this many cells (its shared memory: 7 values per cell).
+template <class T> constexpr int kClusterTailCells = sizeof(T) == 4 ? 65536 : 16384;
 
 struct ClusterTailPlan {
     int first, lg, nl;             // split levels [first, lg), gathered levels [lg, nl)
@@ -407,48 +455,29 @@ namespace cg = cooperative_groups;
 
 // One colour of smooth on a band; xup / xdn: the x arrays of the bands above / below (null at the
 // cluster's ends), mup: the rows of the band above (its bottom ghost row mirrors our row 0).
-__device__ void c_smooth(const SLevel& L, float* xup, int mup, float* xdn, int colour) {
-    const int w = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int nw = static_cast<int>(blockDim.x) >> 5, S = L.S;
-    for (int I = w; I < L.nx; I += nw)
-        for (int J = ((I + colour) & 1) + 2 * lane; J < L.ny; J += 64) {
+template <class T> __device__ void c_smooth(const SLevel<T>& L, T* xup, int mup, T* xdn, int colour) {
+    const RowWalk w((L.ny + 1) / 2);
+    const int S = L.S;
+    for (int I = w.r; I < L.nx; I += w.dr)
+        for (int J = ((I + colour) & 1) + 2 * w.c; J < L.ny; J += 2 * w.dc) {
             const int q = L.at(I, J);
-            const float4 a = L.l4[q];
-            const float v = rb_value(L.b[q], a.x * L.x[q + 1] + a.y * L.x[q - 1] + a.w * L.x[q + S] +
-                                                 a.z * L.x[q - S],
-                                     L.ap[q]);
+            const T v = rb_value(L.b[q], L.flow(q), L.ap[q]);
             L.x[q] = v;
             if (I == 0 && xup) xup[(mup + 1) * S + J + 1] = v;
             if (I == L.nx - 1 && xdn) xdn[J + 1] = v;
         }
     cg::this_cluster().sync();
 }
-// The residual of the band F restricted 2 x 2 into rows c0 + I of the coarse level C (a band of
-// this CTA, c0 = 0, or the gathered level on CTA 0), C.x = 0 there.
-__device__ void c_restrict(const SLevel& F, const SLevel& C, int c0) {
-    const int w = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int nw = static_cast<int>(blockDim.x) >> 5, S = F.S;
-    auto r = [&](int q) {
-        const float4 a = F.l4[q];
-        return F.b[q] - (F.ap[q] * F.x[q] - (a.x * F.x[q + 1] + a.y * F.x[q - 1] + a.w * F.x[q + S] + a.z * F.x[q - S]));
-    };
-    for (int I = w; I < F.nx / 2; I += nw)
-        for (int J = lane; J < C.ny; J += 32) {
-            const int f = F.at(2 * I, 2 * J), cq = C.at(c0 + I, J);
-            C.b[cq] = r(f) + r(f + 1) + r(f + S) + r(f + S + 1);
-            C.x[cq] = 0.0f;
-        }
-    cg::this_cluster().sync();
-}
 // prolong into the band F from rows c0 + I / 2 of the coarse level C (this CTA's band, c0 = 0, or
 // the gathered level on CTA 0), with the ghost stores of c_smooth.
-__device__ void c_prolong(const SLevel& C, int c0, const SLevel& F, float* xup, int mup, float* xdn, float om) {
-    const int w = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-    const int nw = static_cast<int>(blockDim.x) >> 5, S = F.S;
-    for (int I = w; I < F.nx; I += nw)
-        for (int J = lane; J < F.ny; J += 32) {
+template <class T>
+__device__ void c_prolong(const SLevel<T>& C, int c0, const SLevel<T>& F, T* xup, int mup, T* xdn, T om) {
+    const RowWalk w(F.ny);
+    const int S = F.S;
+    for (int I = w.r; I < F.nx; I += w.dr)
+        for (int J = w.c; J < F.ny; J += w.dc) {
             const int q = F.at(I, J);
-            const float v = F.x[q] + om * C.x[C.at(c0 + (I >> 1), J >> 1)];
+            const T v = F.x[q] + om * C.x[C.at(c0 + (I >> 1), J >> 1)];
             F.x[q] = v;
             if (I == 0 && xup) xup[(mup + 1) * S + J + 1] = v;
             if (I == F.nx - 1 && xdn) xdn[J + 1] = v;
@@ -456,8 +485,9 @@ __device__ void c_prolong(const SLevel& C, int c0, const SLevel& F, float* xup, 
     cg::this_cluster().sync();
 }
 
+template <class T>
 __global__ void __launch_bounds__(kCoarseThreads)
-    k_mg_tail_cluster(MgLevelsT<float> lv, ClusterTailPlan pl, int pre, int post, double omega, double tol,
+    k_mg_tail_cluster(MgLevelsT<T> lv, ClusterTailPlan pl, int pre, int post, double omega, double tol, int build,
                       int* sweeps_out) {
     extern __shared__ __align__(16) unsigned char tail_sm[];
     cg::cluster_group cl = cg::this_cluster();
@@ -467,67 +497,54 @@ __global__ void __launch_bounds__(kCoarseThreads)
     // this CTA's band of split level l (laid out for the level's largest band: the same offsets in
     // every CTA, so a neighbour's arrays are this CTA's mapped to its rank)
     auto band = [&](int l) {
-        SLevel s = slevel_at(tail_sm + pl.off[l], pl.rows[l], lv.L[l].ny);
+        SLevel<T> s = slevel_at<T>(tail_sm + pl.off[l], pl.rows[l], lv.L[l].ny);
         s.nx = start(l, rank + 1) - start(l, rank);
         return s;
     };
-    auto xup = [&](const SLevel& s) { return rank > 0 ? cl.map_shared_rank(s.x, rank - 1) : nullptr; };
-    auto xdn = [&](const SLevel& s) { return rank < R - 1 ? cl.map_shared_rank(s.x, rank + 1) : nullptr; };
+    auto xup = [&](const SLevel<T>& s) { return rank > 0 ? cl.map_shared_rank(s.x, rank - 1) : nullptr; };
+    auto xdn = [&](const SLevel<T>& s) { return rank < R - 1 ? cl.map_shared_rank(s.x, rank + 1) : nullptr; };
     auto mup = [&](int l) { return rank > 0 ? start(l, rank) - start(l, rank - 1) : 0; };
-    auto gathered = [&](int l) { return slevel_at(tail_sm + pl.off[l], lv.L[l].nx, lv.L[l].ny); };
+    auto gathered = [&](int l) { return slevel_at<T>(tail_sm + pl.off[l], lv.L[l].nx, lv.L[l].ny); };
     auto gathered0 = [&](int l) { // the gathered level l in CTA 0's shared memory
-        SLevel s = gathered(l);
+        SLevel<T> s = gathered(l);
         s.l4 = cl.map_shared_rank(s.l4, 0);
         s.x = cl.map_shared_rank(s.x, 0);
         s.b = cl.map_shared_rank(s.b, 0);
         s.ap = cl.map_shared_rank(s.ap, 0);
         return s;
     };
-    cl.sync(); // every CTA of the cluster runs before any touches another's shared memory
-    for (int l = first; l < lg; ++l) { // the bands, with their ghost rows of x
-        const LevelViewT<float>& L = lv.L[l];
-        const SLevel s = band(l);
-        const int g0 = start(l, rank), n2 = (s.nx + 2) * s.S;
-        for (int k = threadIdx.x; k < n2; k += blockDim.x) {
-            const int I = k / s.S - 1, J = k % s.S - 1, g = g0 + I;
-            const bool cin = J >= 0 && J < L.ny, own = cin && I >= 0 && I < s.nx;
-            const int q = g * L.stride + J;
-            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (own) {
-                const Links<float> k4 = links(L, q);
-                a = make_float4(k4.e, k4.w, k4.n, k4.s);
-            }
-            s.l4[k] = a;
-            s.ap[k] = own ? L.AP[q] : 0.0f;
-            s.b[k] = (own && l == first) ? L.b[q] : 0.0f;
-            s.x[k] = (l == first && cin && g >= 0 && g < L.nx) ? L.x[q] : 0.0f;
-        }
-    }
+    for (int l = first; l < lg; ++l) // the bands, with their ghost rows of x
+        slevel_load(lv.L[l], band(l), start(l, rank), l == first || !build, l == first);
     if (rank == 0)
-        for (int l = lg; l < nl; ++l) slevel_load(lv.L[l], gathered(l), false);
-    cl.sync();
-    const float om = static_cast<float>(omega);
+        for (int l = lg; l < nl; ++l) slevel_load(lv.L[l], gathered(l), 0, !build, false);
+    cl.sync(); // every CTA of the cluster has loaded before any touches another's shared memory
+    const T om = static_cast<T>(omega);
     for (int l = first; l < lg; ++l) {
-        const SLevel s = band(l);
+        const SLevel<T> s = band(l);
         for (int k = 0; k < pre; ++k) {
             c_smooth(s, xup(s), mup(l), xdn(s), 0);
             c_smooth(s, xup(s), mup(l), xdn(s), 1);
         }
-        if (l + 1 < lg) c_restrict(s, band(l + 1), 0);
-        else c_restrict(s, gathered0(lg), start(l, rank) / 2);
+        const SLevel<T> c = l + 1 < lg ? band(l + 1) : gathered0(lg);
+        const int c0 = l + 1 < lg ? 0 : start(l, rank) / 2;
+        s_restrict_rows(s, c, c0);
+        if (build) s_build(s, c, c0);
+        cl.sync();
     }
     if (rank == 0) { // the gathered levels and the coarsest solve, as k_mg_tail_smem
         for (int l = lg; l + 1 < nl; ++l) {
-            const SLevel L = gathered(l);
+            const SLevel<T> L = gathered(l);
             for (int k = 0; k < pre; ++k) {
                 s_smooth(L, 0);
                 s_smooth(L, 1);
             }
-            s_residual_restrict(L, gathered(l + 1));
+            s_restrict_rows(L, gathered(l + 1), 0);
+            if (build) s_build(L, gathered(l + 1), 0);
+            __syncthreads();
         }
         s_coarse_solve(gathered(nl - 1), tol, sweeps_out);
         for (int l = nl - 2; l >= lg; --l) {
-            const SLevel L = gathered(l);
+            const SLevel<T> L = gathered(l);
             s_prolong(gathered(l + 1), L, om);
             for (int k = 0; k < post; ++k) {
                 s_smooth(L, 0);
@@ -537,7 +554,7 @@ __global__ void __launch_bounds__(kCoarseThreads)
     }
     cl.sync();
     for (int l = lg - 1; l >= first; --l) {
-        const SLevel s = band(l);
+        const SLevel<T> s = band(l);
         if (l + 1 < lg) c_prolong(band(l + 1), 0, s, xup(s), mup(l), xdn(s), om);
         else c_prolong(gathered0(lg), start(l, rank) / 2, s, xup(s), mup(l), xdn(s), om);
         for (int k = 0; k < post; ++k) {
@@ -545,20 +562,8 @@ __global__ void __launch_bounds__(kCoarseThreads)
             c_smooth(s, xup(s), mup(l), xdn(s), 1);
         }
     }
-    for (int l = first; l < lg; ++l) { // the bands' x and b back
-        const LevelViewT<float>& L = lv.L[l];
-        const SLevel s = band(l);
-        const int g0 = start(l, rank), n = s.nx * L.ny;
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            const int I = k / L.ny, J = k - I * L.ny;
-            L.x[(g0 + I) * L.stride + J] = s.x[s.at(I, J)];
-            L.b[(g0 + I) * L.stride + J] = s.b[s.at(I, J)];
-        }
-    }
-    if (rank == 0)
-        for (int l = lg; l < nl; ++l) slevel_store(lv.L[l], gathered(l));
+    slevel_store_x(lv.L[first], band(first), start(first, rank));
 }
-#endif
 
 // A level in global memory as coarse_solve's cells.
 template <class T> __device__ CoarseCell<T> coarse_load(const LevelViewT<T>& L, int I, int J) {
@@ -600,10 +605,11 @@ __global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse(LevelViewT<T> L, d
 template <class T>
 __global__ void __launch_bounds__(kCoarseThreads)
     k_mg_tail(MgLevelsT<T> lv, int first, int pre, int post, double omega, double tol,
-              double* rowbuf, int* sweeps_out, int pairs) {
+              double* rowbuf, int* sweeps_out, int pairs, int build) {
     extern __shared__ __align__(16) unsigned char tail_dyn[];
     const int nl = lv.n;
     for (int l = first; l + 1 < nl; ++l) {
+        if (build) cta_build(lv.L[l], lv.L[l + 1]);
         for (int s = 0; s < pre; ++s) {
             cta_smooth_colour(lv.L[l], 0);
             cta_smooth_colour(lv.L[l], 1);
@@ -640,8 +646,8 @@ __global__ void __launch_bounds__(kCoarseThreads)
 
 } // namespace
 
-// The float tail runs with every level in shared memory when they fit (the 64^2-and-below levels
-// of a square grid take about 170 KB); otherwise, and for double, through global memory.
+// The tail runs with every level in shared memory when they fit (the 64^2-and-below float levels of a
+// square grid take about 170 KB, the 32^2-and-below double ones 100 KB); otherwise through global memory.
 constexpr int kTailSmemMax = 200 * 1024;
 // Shared memory of a pair solve: any level of 1024 threads per CTA takes less.
 constexpr int kCoarseSmemMax = 160 * 1024;
@@ -720,30 +726,30 @@ bool launch_coarse_pairs(const LevelViewT<T>& L, double tol, int* sweeps_out, cu
 
 template <class T>
 void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double omega, double tol,
-                    double* rowbuf, int* sweeps_out, cudaStream_t st) {
+                    double* rowbuf, int* sweeps_out, cudaStream_t st, bool build) {
     const LevelViewT<T>& Lc = lv.L[lv.n - 1];
     if (first == lv.n - 1 && launch_coarse_pairs(Lc, tol, sweeps_out, st)) return;
     // pair solve inside the tail: a thread of the block per pair
     const bool pairs = static_cast<long long>(Lc.nx) * coarse_hp(Lc.ny) <= kCoarseThreads;
-    if constexpr (sizeof(T) == 4) {
-        TailSmem ts{};
-        int bytes = 0;
-        for (int l = first; l < lv.n && l < 24; ++l) {
-            ts.off[l] = bytes;
-            bytes += slevel_bytes(lv.L[l].nx, lv.L[l].ny);
-        }
-        ts.bytes = bytes;
-        if (lv.n <= 24 && bytes <= kTailSmemMax && pairs) {
-            static PerDeviceOnce attr; // the attribute lives in each device's context
-            attr.get([] {
-                SGPU_CUDA(cudaFuncSetAttribute(k_mg_tail_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kTailSmemMax));
-                return 0;
-            });
-            k_mg_tail_smem<<<1, kCoarseThreads, bytes, st>>>(lv, first, pre, post, omega, tol, ts, sweeps_out);
-            SGPU_LAUNCH();
-            return;
-        }
+    TailSmem ts{};
+    long long bytes = 0;
+    for (int l = first; l < lv.n && l < 24 && bytes <= kTailSmemMax; ++l) {
+        ts.off[l] = static_cast<int>(bytes);
+        bytes += static_cast<long long>(lv.L[l].nx + 2) * (lv.L[l].ny + 2) * 7 * static_cast<int>(sizeof(T)) + 16;
+        bytes = bytes / 16 * 16;
+    }
+    if (lv.n <= 24 && bytes <= kTailSmemMax && pairs) {
+        static PerDeviceOnce attr; // the attribute lives in each device's context
+        attr.get([] {
+            SGPU_CUDA(cudaFuncSetAttribute(k_mg_tail_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kTailSmemMax));
+            return 0;
+        });
+        ts.bytes = static_cast<int>(bytes);
+        k_mg_tail_smem<T><<<1, kCoarseThreads, ts.bytes, st>>>(lv, first, pre, post, omega, tol, ts, build ? 1 : 0,
+                                                               sweeps_out);
+        SGPU_LAUNCH();
+        return;
     }
     static PerDeviceOnce attr;
     attr.get([] {
@@ -751,7 +757,8 @@ void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double
         return 0;
     });
     const int dyn = pairs ? coarse_smem_bytes<T>(Lc.nx, Lc.nx, Lc.ny) : 0;
-    k_mg_tail<T><<<1, kCoarseThreads, dyn, st>>>(lv, first, pre, post, omega, tol, rowbuf, sweeps_out, pairs ? 1 : 0);
+    k_mg_tail<T><<<1, kCoarseThreads, dyn, st>>>(lv, first, pre, post, omega, tol, rowbuf, sweeps_out, pairs ? 1 : 0,
+                                                 build ? 1 : 0);
     SGPU_LAUNCH();
 }
 template <class T> void launch_mg_build(const LevelViewT<T>& F, const LevelViewT<T>& C, cudaStream_t st) {
@@ -795,7 +802,6 @@ void launch_mg_sub_mean(const LevelView& L, double* x, const double* sum, cudaSt
 }
 #endif
 
-#ifdef SGPU_FLOAT_UNIT
 namespace {
 // Dynamic shared memory per CTA of the cluster tail (the 227 KB a CTA may have).
 constexpr int kClusterSmemMax = 227 * 1024;
@@ -803,7 +809,7 @@ constexpr int kClusterSmemMax = 227 * 1024;
 // The cluster tail's plan from level `first`; false where it does not apply: fewer than one split
 // level, a split level that does not halve exactly into the next, a coarsest split level of fewer
 // than 2 rows per CTA, or more shared memory per CTA than kClusterSmemMax.
-bool cluster_tail_plan(const MgLevelsT<float>& lv, int first, ClusterTailPlan& pl) {
+template <class T> bool cluster_tail_plan(const MgLevelsT<T>& lv, int first, ClusterTailPlan& pl) {
     const int nl = lv.n;
     if (nl > 24 || first < 0 || first >= nl - 1) return false;
     int lg = first;
@@ -819,17 +825,18 @@ bool cluster_tail_plan(const MgLevelsT<float>& lv, int first, ClusterTailPlan& p
     pl.nl = nl;
     for (int r = 0; r < kClusterTail; ++r) pl.band[r] = 2 * ((r * (nxc / 2)) / kClusterTail);
     pl.band[kClusterTail] = nxc;
+    if (lv.L[first].nx * lv.L[first].ny > kClusterTailCells<T>) return false;
     int bytes = 0;
     for (int l = first; l < lg; ++l) {
         int rows = 0;
         for (int r = 0; r < kClusterTail; ++r) rows = std::max(rows, (pl.band[r + 1] - pl.band[r]) << (Lc - l));
         pl.rows[l] = rows;
         pl.off[l] = bytes;
-        bytes += slevel_bytes(rows, lv.L[l].ny);
+        bytes += slevel_bytes<T>(rows, lv.L[l].ny);
     }
     for (int l = lg; l < nl; ++l) {
         pl.off[l] = bytes;
-        bytes += slevel_bytes(lv.L[l].nx, lv.L[l].ny);
+        bytes += slevel_bytes<T>(lv.L[l].nx, lv.L[l].ny);
     }
     pl.bytes = bytes;
     return bytes <= kClusterSmemMax;
@@ -837,17 +844,17 @@ bool cluster_tail_plan(const MgLevelsT<float>& lv, int first, ClusterTailPlan& p
 
 // Whether this device runs the cluster tail: its function attributes set (the dynamic shared memory
 // and the non-portable cluster size, once per device) and at least one such cluster resident.
-// SGPU_MG_CLUSTER=0 turns it off for the solvers created while it is set (their float tail then
-// runs as streamed levels and the single-CTA tail, as without a cluster).
-bool cluster_tail_available() {
+// SGPU_MG_CLUSTER=0 turns it off for the solvers created while it is set (their tail then runs as
+// streamed levels and the single-CTA tail, as without a cluster).
+template <class T> bool cluster_tail_available() {
     if (const char* e = std::getenv("SGPU_MG_CLUSTER"))
         if (std::atoi(e) == 0) return false;
     static PerDeviceOnce once;
     return once.get([] {
         // a device that refuses either attribute runs the kernels without a cluster
-        if (cudaFuncSetAttribute(k_mg_tail_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax) !=
+        if (cudaFuncSetAttribute(k_mg_tail_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax) !=
                 cudaSuccess ||
-            cudaFuncSetAttribute(k_mg_tail_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaFuncSetAttribute(k_mg_tail_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             (void)cudaGetLastError();
             return 0;
         }
@@ -863,7 +870,7 @@ bool cluster_tail_available() {
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_mg_tail_cluster, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&n, k_mg_tail_cluster<T>, &cfg) != cudaSuccess) {
             (void)cudaGetLastError(); // not supported here: the clear-up of the failed query
             return 0;
         }
@@ -872,18 +879,19 @@ bool cluster_tail_available() {
 }
 } // namespace
 
-int mg_cluster_tail_first(const MgLevelsT<float>& lv, int fallback) {
-    if (!cluster_tail_available()) return fallback;
+template <class T> int mg_cluster_tail_first(const MgLevelsT<T>& lv, int fallback) {
+    if (!cluster_tail_available<T>()) return fallback;
     int t = 0;
-    while (t < lv.n - 1 && lv.L[t].nx * lv.L[t].ny > kClusterTailCells) ++t;
+    while (t < lv.n - 1 && lv.L[t].nx * lv.L[t].ny > kClusterTailCells<T>) ++t;
     ClusterTailPlan pl{};
     for (; t < fallback; ++t)
         if (cluster_tail_plan(lv, t, pl)) return t;
     return fallback;
 }
 
-bool launch_mg_tail_cluster(const MgLevelsT<float>& lv, int first, int pre, int post, double omega, double tol,
-                            int* sweeps_out, cudaStream_t st) {
+template <class T>
+bool launch_mg_tail_cluster(const MgLevelsT<T>& lv, int first, int pre, int post, double omega, double tol,
+                            int* sweeps_out, cudaStream_t st, bool build) {
     ClusterTailPlan pl{};
     if (!cluster_tail_plan(lv, first, pl)) return false;
     cudaLaunchConfig_t cfg = {};
@@ -898,15 +906,17 @@ bool launch_mg_tail_cluster(const MgLevelsT<float>& lv, int first, int pre, int 
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    SGPU_CUDA(cudaLaunchKernelEx(&cfg, k_mg_tail_cluster, lv, pl, pre, post, omega, tol, sweeps_out));
+    SGPU_CUDA(cudaLaunchKernelEx(&cfg, k_mg_tail_cluster<T>, lv, pl, pre, post, omega, tol, build ? 1 : 0,
+                                 sweeps_out));
     SGPU_LAUNCH();
     return true;
 }
-#endif
-
 #define SGPU_MG_INST(T)                                                                            \
     template void launch_mg_tail<T>(const MgLevelsT<T>&, int, int, int, double, double, double*,   \
-                                    int*, cudaStream_t);                                           \
+                                    int*, cudaStream_t, bool);                                     \
+    template int mg_cluster_tail_first<T>(const MgLevelsT<T>&, int);                               \
+    template bool launch_mg_tail_cluster<T>(const MgLevelsT<T>&, int, int, int, double, double,    \
+                                            int*, cudaStream_t, bool);                             \
     template void launch_mg_build<T>(const LevelViewT<T>&, const LevelViewT<T>&, cudaStream_t);    \
     template void launch_mg_smooth_colour<T>(const LevelViewT<T>&, int, cudaStream_t);             \
     template void launch_mg_residual<T>(const LevelViewT<T>&, cudaStream_t);                       \

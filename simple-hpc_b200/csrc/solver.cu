@@ -101,13 +101,13 @@ struct Solver {
     double* coarse_rowbuf = nullptr;
     bool mg_fast = false;            // streaming level kernels (mg_fast.cu) + single-CTA tail
     int mg_tail = 0;                 // first level handled by the tail kernel
-    // first level of the float V-cycle's tail: the cluster tail's (mg.cu, k_mg_tail_cluster) where
-    // the device and the grid allow it, else mg_tail
-    int mg_tail32 = 0;
+    // first level of the float and of the double V-cycle's tail: the cluster tail's (mg.cu,
+    // k_mg_tail_cluster) where the device and the grid allow it, else mg_tail
+    int mg_tail32 = 0, mg_tail64 = 0;
     std::vector<double*> mg_x2;      // second iterate buffer per streamed level (interior (0,0))
     MgLevels mgl{};
-    // build: form the coarse operators inside the cycle (the streamed levels' down kernels, then the
-    // tail's levels) instead of before it.
+    // build: form the coarse operators inside the cycle (the streamed levels' down kernels, the tail)
+    // instead of before it.
     void mg_vcycle_fast(bool x_is_zero, bool build = false);
 
     // fused fast path (multicolour momentum): frozen velocity copy and the sweep ping-pong buffer
@@ -125,7 +125,7 @@ struct Solver {
         min_seg = 0;
         // A batch fills the GPU with many cavities' kernels, so SM time, not latency, bounds it: the
         // single-CTA tail (one SM) instead of the cluster tail (16 SMs for a shorter time).
-        mg_tail32 = mg_tail;
+        mg_tail32 = mg_tail64 = mg_tail;
         if (fast)
             seg_rows = mixed ? stream_seg_rows(dp, sms, corr_blocks_per_sm(dp.ncol), 0, corr_threads())
                              : stream_seg_rows(dp, sms, 2, 0);
@@ -464,8 +464,8 @@ struct Solver {
         launch_sum_partials(part, nparts, 2, nparts, res3 + 2, sums + 25, st);
         mark(SGPU_PH_SOLVE_P);
         // The coarse operators are built inside the V-cycle (fused_build: by the down kernel of the
-        // level above for the streamed levels, then the tail's levels), unless a warm start reads
-        // them before the first cycle.
+        // level above for the streamed levels, by the tail for its own), unless a warm start reads them
+        // before the first cycle.
         const bool fused_build = !net;
         if (!fused_build)
             for (std::size_t l = 1; l < lv32.size(); ++l) launch_mg_build<float>(lv32[l - 1], lv32[l], st);
@@ -494,14 +494,11 @@ struct Solver {
             for (int l = 0; l < mg_tail32; ++l)
                 launch_mg_down<float>(lv32[l], lv32[l + 1], mg32_x2[l], prm.mg_pre, x_zero || l > 0, sms,
                                       min_seg, st, fused_build);
-            if (fused_build)
-                for (std::size_t l = static_cast<std::size_t>(mg_tail32) + 1; l < lv32.size(); ++l)
-                    launch_mg_build<float>(lv32[l - 1], lv32[l], st);
             if (mg_tail32 == mg_tail ||
                 !launch_mg_tail_cluster(mgl32, mg_tail32, prm.mg_pre, prm.mg_post, prm.mg_omega, kCoarseTol32,
-                                        stats, st))
+                                        stats, st, fused_build))
                 launch_mg_tail<float>(mgl32, mg_tail32, prm.mg_pre, prm.mg_post, prm.mg_omega, kCoarseTol32,
-                                      coarse_rowbuf, stats, st);
+                                      coarse_rowbuf, stats, st, fused_build);
             for (int l = mg_tail32 - 1; l >= 0; --l)
                 launch_mg_up<float>(lv32[l + 1], lv32[l], mg32_x2[l], lv32[l].x, prm.mg_omega,
                                     prm.mg_post, sms, min_seg, st);
@@ -832,6 +829,7 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
         }
         mgl.n = nl;
         for (int l = 0; l < nl && l < 24; ++l) mgl.L[l] = lv[l];
+        mg_tail64 = mg_fast ? mg_cluster_tail_first(mgl, mg_tail) : mg_tail;
     }
 
     if (p.precision == SGPU_PREC_MIXED) {
@@ -1065,7 +1063,10 @@ template <class T> bool Solver::warm_start_on(std::vector<LevelViewT<T>>& L) {
 // mean of the solved p' there (both normalised as the network sees them).
 template <class T> void Solver::sample_pair(std::vector<LevelViewT<T>>& L, float* hin, float* htarget) {
     const int l = cnn_level(L);
-    for (int k = 0; k < l; ++k) launch_restrict_b(L[k], L[k + 1], st);
+    for (int k = 0; k < l; ++k) {
+        launch_mg_build(L[k], L[k + 1], st); // the tail keeps the operators of its levels to itself
+        launch_restrict_b(L[k], L[k + 1], st);
+    }
     launch_level_stats(L[l], cells, plane, st);
     launch_ordered_sum(cells, plane, L[l].ny, L[l].nx, L[l].ny, 2, sums + 30, ss, nullptr, st);
     const std::size_t n = static_cast<std::size_t>(L[l].nx) * L[l].ny;
@@ -1076,19 +1077,17 @@ template <class T> void Solver::sample_pair(std::vector<LevelViewT<T>>& L, float
     SGPU_CUDA(cudaStreamSynchronize(st));
 }
 
-// mg_vcycle with the streaming level kernels: levels [0, mg_tail) go down and up in one pass
-// each, the rest (and the coarse solve) in the single-CTA tail kernel.
+// mg_vcycle with the streaming level kernels: levels [0, mg_tail64) go down and up in one pass each, the
+// rest (and the coarse solve) in a tail kernel.
 void Solver::mg_vcycle_fast(bool x_is_zero, bool build) {
-    const int nl = static_cast<int>(lv.size());
-    for (int l = 0; l < mg_tail; ++l)
+    for (int l = 0; l < mg_tail64; ++l)
         launch_mg_down(lv[l], lv[l + 1], mg_x2[l], prm.mg_pre, x_is_zero || l > 0, sms, min_seg, st, build);
-    if (build)
-        for (int l = mg_tail + 1; l < nl; ++l) launch_mg_build(lv[l - 1], lv[l], st);
-    launch_mg_tail(mgl, mg_tail, prm.mg_pre, prm.mg_post, prm.mg_omega, kCoarseTol64, coarse_rowbuf,
-                   stats, st);
-    for (int l = mg_tail - 1; l >= 0; --l)
+    if (mg_tail64 == mg_tail || !launch_mg_tail_cluster(mgl, mg_tail64, prm.mg_pre, prm.mg_post, prm.mg_omega,
+                                                        kCoarseTol64, stats, st, build))
+        launch_mg_tail(mgl, mg_tail64, prm.mg_pre, prm.mg_post, prm.mg_omega, kCoarseTol64, coarse_rowbuf,
+                       stats, st, build);
+    for (int l = mg_tail64 - 1; l >= 0; --l)
         launch_mg_up(lv[l + 1], lv[l], mg_x2[l], lv[l].x, prm.mg_omega, prm.mg_post, sms, min_seg, st);
-    (void)nl;
 }
 
 void Solver::solve_p() {
