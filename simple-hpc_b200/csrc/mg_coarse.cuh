@@ -110,11 +110,7 @@ template <class T> struct CoarseCell {
 
 // The update value of a cell from its neighbour sum. Double: b / AP (t0, formed once) + nb / AP, the
 // two statements of multigrid.cpp:61-63; float: as rb_value.
-__device__ __forceinline__ double coarse_value(double t0, double, double nb, double ap) {
-    double t = t0;
-    t += nb / ap;
-    return t;
-}
+__device__ __forceinline__ double coarse_value(double t0, double, double nb, double ap) { return div_sum(t0, nb, ap); }
 __device__ __forceinline__ float coarse_value(float, float b, float nb, float ap) { return rb_value(b, nb, ap); }
 __device__ __forceinline__ double coarse_t0(double b, double ap) { return b / ap; }
 __device__ __forceinline__ float coarse_t0(float, float) { return 0.0f; }

@@ -206,11 +206,10 @@ __global__ void k_pc_redblack(DevParams p, PressurePtr w, Range r, int colour) {
     int i, j;
     if (!cell_of(r, i, j) || ((i + j) & 1) != colour) return;
     const std::size_t q = ix(p, i, j), ld = p.pitch;
-    double t = w.b[q] / w.APP[q];
-    t += (w.AEP[q] * w.pc[q + 1] + w.AWP[q] * w.pc[q - 1] + w.ASP[q] * w.pc[q + ld] +
-          w.ANP[q] * w.pc[q - ld]) /
-         w.APP[q];
-    w.pc[q] = t;
+    w.pc[q] = rb_value(w.b[q],
+                       w.AEP[q] * w.pc[q + 1] + w.AWP[q] * w.pc[q - 1] + w.ASP[q] * w.pc[q + ld] +
+                           w.ANP[q] * w.pc[q - ld],
+                       w.APP[q]);
 }
 
 // One damped Jacobi pass of solve_pc_jacobi (pressure.cpp:77-112), weight 0.8.
