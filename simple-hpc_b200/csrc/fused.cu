@@ -13,14 +13,19 @@
 //    of each cell relative to its neighbours is exactly the reference's colour order. Rows stream
 //    through a shared-memory ring filled by cp.async; halo cells are updated redundantly and only
 //    the owned block is written, to a second buffer.
+//  * k_mom_prep_rec and k_mom_rec_stream are the same pair with the coefficients stored instead, once per
+//    component, in records laid out by sweep step: the sweep reads them (80 B/cell) and is left with a
+//    third of the instructions.
 //  * k_mom_cluster does both for a small grid, in the shared memory of one thread-block cluster.
 // Pressure assembly (assemble_p, pressure.cpp:14-54) is one kernel with the wall zeros folded in.
 #include "kernels.hpp"
+#include "bulk.cuh"
 #include "stencil.cuh"
 
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdlib>
 #include <climits>
 
@@ -83,15 +88,6 @@ constexpr int kPrefetch = 8; // rows the cp.async ring runs ahead of the rows be
 #define SGPU_STREAM_PF 0
 #endif
 constexpr int kStreamPF = SGPU_STREAM_PF; // input staging of k_mom_stream (see the kernel)
-
-__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // The 9 global inputs of one cell's coefficient recomputation and pressure term, read through
 // per-thread column pointers (xF, oth, pf already offset by the thread's column) at row offset o.
@@ -259,7 +255,7 @@ __global__ void __launch_bounds__(NT, PF == 0 ? 2 : 3)
 
     int next = L0;
     auto issue = [&]() {
-        if (next < L1 && col_in) cp_async8(ringc + (next & (kRing - 1)) * NT, xinc + next * ld);
+        if (next < L1 && col_in) cp_async(ringc + (next & (kRing - 1)) * NT, xinc + next * ld);
         cp_async_commit();
         ++next;
     };
@@ -411,6 +407,249 @@ __global__ void __launch_bounds__(NT, PF == 0 ? 2 : 3)
             c0 = cn;
         }
     }
+    cp_async_wait<0>();
+}
+
+// ---- stored coefficients ----
+//
+// The recomputing sweep is bound by instruction issue (about 400 a cell, half of the slots busy, DRAM at
+// 17%), and its CTAs' halo and skew rows cost as much as their own. Records cost 72 B/cell once per
+// component and 56 B/cell more per sweep, but a third of the instructions, and up to about 1024^2 they
+// stay in L2. Measured, prep and four sweeps of one component: 178 us at 1024^2 and 1570 us at 4096^2,
+// against 206 and 1810 us (a sweep: 37 and 262 us against 47 and 390; the prep, bound by the latency of
+// its loads, 31 and 520 us against 18 and 260).
+
+constexpr int kRecTileRows = 16; // rows of a prep block's tile: 40 KB of records in shared memory
+
+// Prep over the update range: |R|, AP and the records. A block of 32 x 8 threads stages the records of a
+// tile of 32 columns x kRecTileRows rows in shared memory and then writes whole step rows (the cells of
+// one step row lie on up to five field rows; a step row shared with the neighbouring tile is written in
+// part by each). At 4096^2: 0.52 ms; a tile of 16 x 32 0.55, 80 registers and three CTAs an SM 0.55, 48 and
+// five 0.58.
+template <int NCOL, bool V>
+__global__ void __launch_bounds__(256, 4)
+    k_mom_prep_rec(DevParams p, const double* __restrict__ x, const double* __restrict__ oth,
+                   const double* __restrict__ pf, double* __restrict__ AP, double* __restrict__ cells, MomRec64 rec,
+                   Range ur) {
+    constexpr int NK = NCOL == 5 ? 5 : 3;
+    __shared__ double2 s[NK][kRecTileRows][32];
+    const int lane = static_cast<int>(threadIdx.x), wy = static_cast<int>(threadIdx.y);
+    const int j = ur.j0 + static_cast<int>(blockIdx.x) * 32 + lane;
+    const int ib = ur.i0 + static_cast<int>(blockIdx.y) * kRecTileRows;
+    if (j <= ur.j1) {
+#pragma unroll 1
+        for (int ti = wy; ti < kRecTileRows; ti += 8) {
+            const int i = ib + ti;
+            if (i > ur.i1) break;
+            const std::size_t q = ix(p, i, j), ld = p.pitch;
+            const Coef9 c = V ? coef_v(p, oth, x, i, j) : coef_u(p, x, oth, i, j);
+            const double nb = (c.AE * x[q + 1] + c.AW * x[q - 1] + c.AN * x[q - ld] + c.AS * x[q + ld]) +
+                              (c.AEE * x[q + 2] + c.AWW * x[q - 2] + c.ANN * x[q - 2 * ld] + c.ASS * x[q + 2 * ld]);
+            const double pt = V ? (pf[q] - pf[q - ld]) * p.dx : (pf[q] - pf[q + 1]) * p.dy;
+            cells[static_cast<std::size_t>(i - ur.i0) * ur.cols() + (j - ur.j0)] = fabs(nb + pt - c.AP * x[q]);
+            AP[q] = c.AP;
+            s[0][ti][lane] = make_double2(c.AE, c.AW);
+            s[1][ti][lane] = make_double2(c.AN, c.AS);
+            if (NCOL == 5) {
+                s[2][ti][lane] = make_double2(c.AEE, c.AWW);
+                s[NK - 2][ti][lane] = make_double2(c.ANN, c.ASS);
+            }
+            s[NK - 1][ti][lane] = make_double2(c.AP, pt);
+        }
+    }
+    __syncthreads();
+    if (j > ur.j1) return;
+    const int nsteps = kRecTileRows + 2 * (NCOL - 1);
+    for (int k = wy; k < nsteps; k += 8) {
+        const int st = ib + k;
+        const int c = NCOL == 5 ? (2 * st + j) % 5 : (st + j) & 1; // the colour of step st in column j
+        const int ti = k - 2 * c;
+        if (ti < 0 || ti >= kRecTileRows || ib + ti > ur.i1) continue;
+        const std::size_t q = static_cast<std::size_t>(st) * p.pitch + j;
+        rec.r[0][q] = s[0][ti][lane];
+        rec.r[1][q] = s[1][ti][lane];
+        if (NCOL == 5) {
+            rec.r[2][q] = s[2][ti][lane];
+            rec.r[3][q] = s[NK - 2][ti][lane];
+        }
+        rec.r[4][q] = s[NK - 1][ti][lane];
+    }
+}
+
+// Threads of the record sweep's CTAs, and the resident CTAs its registers are bounded for: the x ring and
+// two record slot sets of 224 columns take 98 KB, so two CTAs fit an SM.
+constexpr int kMomRecNT = 224, kMomRecMinb = 2;
+constexpr int kMomRecRing = 16; // x rows: a super-step reads down to 2 NCOL behind it, 6 rows ahead are issued
+constexpr int kMomRecAhead = 2; // record slot sets (super-steps in flight)
+
+template <int NCOL, int NT> struct MomRecSmem {
+    static constexpr int SPB = NCOL == 5 ? 2 : 1;
+    static constexpr int NK = NCOL == 5 ? 5 : 3;
+    static constexpr int slots = kMomRecAhead * SPB;
+    static constexpr int ring = kMomRecRing * NT * 8;
+    static constexpr int bytes = ring + NK * slots * NT * 16;
+    static constexpr unsigned row_bytes = NK * NT * 16; // bytes one step row of records brings in
+};
+
+// One multicolour sweep xin -> xout from the records: the schedule of k_mom_stream (cell (r, j) of colour
+// c at step r + 2c, SPB steps per barrier, strip halo of 2 per colour). The records of one step for the
+// CTA's columns are NK contiguous row segments; thread 0 fetches a super-step's with bulk copies into one
+// of kMomRecAhead slot sets, completing on its `full` mbarrier, and refills a set once every thread has
+// arrived on its `empty` mbarrier. x rows are per-thread cp.async copies, one group per super-step. Waits
+// are bounded; a give-up sets *err, the next barrier stops the CTA, no further copy is issued, and thread
+// 0 waits (bounded) for its copies in flight before it exits.
+template <int NCOL, bool V, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
+    k_mom_rec_stream(DevParams p, const double* __restrict__ xin, double* __restrict__ xout, MomRec64 rec, int seg_rows,
+                     unsigned* err) {
+    using S = MomRecSmem<NCOL, NT>;
+    constexpr int SPB = S::SPB, NK = S::NK;
+    constexpr int HC = 2 * NCOL;
+    constexpr int W = NT - 2 * HC;
+    constexpr int D = kMomRecAhead;
+    constexpr int E0 = SPB * D + 2; // x rows issued before the first super-step
+    constexpr int MASK = kMomRecRing - 1;
+    static_assert(D == 2, "the step loop is unrolled over the two record slot sets");
+    extern __shared__ __align__(16) unsigned char mr_mem[];
+    double* ring_mem = reinterpret_cast<double*>(mr_mem);
+    double2* s_rec = reinterpret_cast<double2*>(mr_mem + S::ring); // [array][slot][column]
+    __shared__ int s_rmin[NCOL], s_rmax[NCOL];
+    __shared__ __align__(8) unsigned long long full[D], empty[D];
+    const int tid = threadIdx.x;
+    const int j0 = blockIdx.x * W;
+    const int C0 = j0 - HC, C1 = j0 + W + HC;
+    const int col = C0 + tid;
+    const int R0 = blockIdx.y * seg_rows;
+    const int R1 = min(R0 + seg_rows, p.nrows);
+    const int L0 = max(R0 - HC, 0), L1 = min(R1 + HC, p.nrows);
+    const int ld = p.pitch, H = p.H;
+    const bool col_in = col >= 0 && col < p.ncols;
+    const bool col_out = col_in && col >= j0 && col < j0 + W;
+    if (tid < NCOL) { // the rows a cell of colour tid may be updated at (k_mom_stream)
+        int lo = V ? H + 1 : H, hi = p.NX + H - 1;
+        if (L0 > 0) lo = max(lo, L0 + 2 + 2 * tid);
+        if (L1 < p.nrows) hi = min(hi, L1 - 3 - 2 * tid);
+        s_rmin[tid] = lo;
+        s_rmax[tid] = hi;
+    }
+    if (tid == 0) {
+        for (int d = 0; d < D; ++d) {
+            mbar_init(&full[d], 1);
+            mbar_init(&empty[d], NT);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    unsigned colmask = 0;
+    {
+        const int ju0 = H + 1, ju1 = V ? p.NY + H : p.NY + H - 1;
+#pragma unroll
+        for (int c = 0; c < NCOL; ++c) {
+            bool ok = col >= ju0 && col <= ju1;
+            if (C0 > 0) ok = ok && col >= C0 + 2 + 2 * c;
+            if (C1 < p.ncols) ok = ok && col <= C1 - 3 - 2 * c;
+            colmask |= (ok ? 1u : 0u) << c;
+        }
+    }
+    const double relax = V ? p.av : p.au;
+    const double omr = 1 - relax;
+    double* ringc = ring_mem + tid;
+    int next = L0;
+    const double* xo = xin + col + static_cast<std::ptrdiff_t>(L0) * ld; // the next row to issue
+    double* wo = xout + col + static_cast<std::ptrdiff_t>(L0 - 2 * NCOL + 1 - (SPB - 1)) * ld; // ... to write
+    auto issue_row = [&]() {
+        if (next < L1 && col_in) cp_async(ringc + (next & MASK) * NT, xo);
+        ++next;
+        xo += ld;
+    };
+    auto step_cell = [&](int c, int t, int& r) -> bool {
+        r = t - 2 * c;
+        return ((colmask >> c) & 1u) && r >= s_rmin[c] && r <= s_rmax[c];
+    };
+    auto next_colour = [&](int c, int steps) { return NCOL == 5 ? (c + 2 * steps) % 5 : (c + steps) & 1; };
+    const int rec_rows = p.nrows + kRecExtraRows;
+    unsigned inflight = 0, inflight_parity = 0; // thread 0: the slot sets whose copies it has not seen land
+    auto fill = [&](int slot, int t, unsigned parity) {
+        inflight |= 1u << slot;
+        inflight_parity = (inflight_parity & ~(1u << slot)) | (parity << slot);
+        unsigned bytes = 0;
+#pragma unroll
+        for (int s = 0; s < SPB; ++s)
+            if (t + s < rec_rows) bytes += S::row_bytes;
+        mbar_arrive_expect(&full[slot], bytes);
+#pragma unroll
+        for (int s = 0; s < SPB; ++s) {
+            if (t + s >= rec_rows) continue;
+            const std::ptrdiff_t o = static_cast<std::ptrdiff_t>(t + s) * ld + C0;
+#pragma unroll
+            for (int k = 0; k < NK; ++k)
+                bulk_load(s_rec + (k * S::slots + slot * SPB + s) * NT, rec.r[NK == 5 ? k : (k == 2 ? 4 : k)] + o,
+                          NT * 16, &full[slot]);
+        }
+    };
+    auto update = [&](int r, int q) {
+        double* rc = ringc + (r & MASK) * NT;
+        const double2 ew = s_rec[q], ns = s_rec[S::slots * NT + q], d = s_rec[(NK - 1) * S::slots * NT + q];
+        const double xn = ringc[((r - 1) & MASK) * NT], xs = ringc[((r + 1) & MASK) * NT];
+        double nb = ew.x * rc[1] + ew.y * rc[-1] + ns.x * xn + ns.y * xs;
+        if (NCOL == 5) {
+            const double2 fe = s_rec[2 * S::slots * NT + q], fn = s_rec[(NK - 2) * S::slots * NT + q];
+            const double xnn = ringc[((r - 2) & MASK) * NT], xss = ringc[((r + 2) & MASK) * NT];
+            nb = nb + (fe.x * rc[2] + fe.y * rc[-2] + fn.x * xnn + fn.y * xss);
+        }
+        rc[0] = relax * (nb + d.y) / d.x + omr * rc[0];
+    };
+
+    __syncthreads(); // s_rmin / s_rmax and the initialised mbarriers
+    const int c_start = NCOL == 5 ? (2 * L0 + col + 1000) % 5 : (L0 + col + 1000) & 1;
+    const int t_last = R1 + 2 * NCOL - 2 + (SPB - 1);
+    for (int i = 0; i < E0; ++i) issue_row();
+    cp_async_commit();
+    cp_async_commit();
+    if (tid == 0) {
+        fill(0, L0, 0u);
+        if (L0 + SPB <= t_last) fill(1, L0 + SPB, 0u);
+    }
+    int c_cur = c_start;
+    bool gave_up = false;
+    auto super_step = [&](int t, int slot, unsigned parity) -> bool {
+        cp_async_wait<D - 1>(); // this thread's x rows for this super-step
+        if (mbar_wait(&full[slot], parity, err)) {
+            if (tid == 0) inflight &= ~(1u << slot);
+        } else {
+            gave_up = true;
+        }
+        if (__syncthreads_or(gave_up ? 1 : 0)) return false; // ... and everyone's
+#pragma unroll
+        for (int s = 0; s < SPB; ++s) {
+            int r;
+            if (step_cell(next_colour(c_cur, s), t + s, r)) update(r, (slot * SPB + s) * NT + tid);
+        }
+        mbar_arrive(&empty[slot]);
+#pragma unroll
+        for (int s = 0; s < SPB; ++s) {
+            const int rw = t - 2 * NCOL + 1 - (SPB - 1) + s;
+            if (rw >= R0 && rw < R1 && col_out) wo[s * ld] = ringc[(rw & MASK) * NT];
+        }
+        wo += SPB * ld;
+#pragma unroll
+        for (int s = 0; s < SPB; ++s) issue_row();
+        cp_async_commit();
+        c_cur = next_colour(c_cur, SPB);
+        if (tid == 0 && t + SPB * D <= t_last) {
+            if (mbar_wait(&empty[slot], parity, err)) fill(slot, t + SPB * D, parity ^ 1u);
+            else gave_up = true; // not refilled: the next super-step's barrier stops the CTA
+        }
+        return true;
+    };
+    unsigned parity = 0;
+    for (int t = L0; t <= t_last; t += 2 * SPB) {
+        if (!super_step(t, 0, parity)) break;
+        if (t + SPB <= t_last && !super_step(t + SPB, 1, parity)) break;
+        parity ^= 1u;
+    }
+    if (tid == 0) // after a give-up only
+        for (int sl = 0; sl < D; ++sl)
+            if ((inflight >> sl) & 1u) mbar_wait(&full[sl], (inflight_parity >> sl) & 1u, err);
     cp_async_wait<0>();
 }
 
@@ -700,6 +939,27 @@ void launch_mom_cluster_t(const DevParams& p, double* x, const double* oth, cons
     SGPU_LAUNCH();
 }
 
+template <int NCOL, bool V>
+void launch_rec_stream(const DevParams& p, const double* xin, double* xout, MomRec64 rec, int seg_rows, unsigned* err,
+                       cudaStream_t st) {
+    // A bulk copy starts at record (t * pitch + first column), 16 bytes each: aligned when the arrays are.
+    for (int k = 0; k < 5; ++k)
+        if (mom_rec_used(NCOL, k) && (!rec.r[k] || (reinterpret_cast<std::uintptr_t>(rec.r[k]) & 15u)))
+            throw Error(SGPU_E_INVALID, "momentum sweep: records missing or not aligned for bulk copies");
+    constexpr int NT = kMomRecNT, W = NT - 4 * NCOL;
+    static_assert(2 * NCOL <= kRecFrontCols && NT <= kRecBackCols, "copy windows must stay in the margins");
+    using S = MomRecSmem<NCOL, NT>;
+    static PerDeviceOnce attr;
+    attr.get([] {
+        SGPU_CUDA(cudaFuncSetAttribute(k_mom_rec_stream<NCOL, V, NT, kMomRecMinb>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, S::bytes));
+        return 0;
+    });
+    const dim3 grid((p.ncols + W - 1) / W, (p.nrows + seg_rows - 1) / seg_rows);
+    k_mom_rec_stream<NCOL, V, NT, kMomRecMinb><<<grid, NT, S::bytes, st>>>(p, xin, xout, rec, seg_rows, err);
+    SGPU_LAUNCH();
+}
+
 } // namespace
 
 // Rows per CTA segment of the streaming sweep: enough segments to fill the GPU with one wave of
@@ -757,6 +1017,48 @@ void launch_mom_sweep(const DevParams& p, bool v_component, const double* xin, d
                       cudaStream_t st) {
     if (v_component) launch_stream_v<true, kStreamPF>(p, xin, xout, xF, oth, pf, seg_rows, st);
     else launch_stream_v<false, kStreamPF>(p, xin, xout, xF, oth, pf, seg_rows, st);
+}
+
+void launch_mom_prep_rec(const DevParams& p, bool v_component, const double* x, const double* oth, const double* pf,
+                         double* AP, double* cells, MomRec64 rec, cudaStream_t st) {
+    Range ur, cr;
+    if (v_component) prep_ranges<true>(p, ur, cr);
+    else prep_ranges<false>(p, ur, cr);
+    if (ur.rows() <= 0 || ur.cols() <= 0) return;
+    const dim3 grid((ur.cols() + 31) / 32, (ur.rows() + kRecTileRows - 1) / kRecTileRows), block(32, 8);
+    if (p.ncol == 5) {
+        if (v_component) k_mom_prep_rec<5, true><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
+        else k_mom_prep_rec<5, false><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
+    } else {
+        if (v_component) k_mom_prep_rec<2, true><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
+        else k_mom_prep_rec<2, false><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
+    }
+    SGPU_LAUNCH();
+}
+
+void launch_mom_sweep_rec(const DevParams& p, bool v_component, const double* xin, double* xout, MomRec64 rec,
+                          int seg_rows, unsigned* err, cudaStream_t st) {
+    if (p.ncol == 5) {
+        if (v_component) launch_rec_stream<5, true>(p, xin, xout, rec, seg_rows, err, st);
+        else launch_rec_stream<5, false>(p, xin, xout, rec, seg_rows, err, st);
+    } else {
+        if (v_component) launch_rec_stream<2, true>(p, xin, xout, rec, seg_rows, err, st);
+        else launch_rec_stream<2, false>(p, xin, xout, rec, seg_rows, err, st);
+    }
+}
+
+int mom_rec_threads() { return kMomRecNT; }
+int mom_rec_blocks_per_sm(int ncol) {
+    static PerDeviceOnce five, two;
+    auto resident = [](auto kernel, int smem) {
+        int n = 0;
+        SGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        SGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kMomRecNT, smem));
+        return std::max(n, 1);
+    };
+    if (ncol == 5)
+        return five.get([&] { return resident(k_mom_rec_stream<5, false, kMomRecNT, kMomRecMinb>, MomRecSmem<5, kMomRecNT>::bytes); });
+    return two.get([&] { return resident(k_mom_rec_stream<2, false, kMomRecNT, kMomRecMinb>, MomRecSmem<2, kMomRecNT>::bytes); });
 }
 
 void launch_assemble_p_fused(const DevParams& p, const double* APU, const double* APV,

@@ -246,6 +246,24 @@ void launch_mom_prep(const DevParams& p, bool v_component, const double* x, cons
 bool mom_cluster_fits(const DevParams& p, bool v_component);
 void launch_mom_cluster(const DevParams& p, bool v_component, double* x, const double* oth, const double* pf,
                         double* AP, double* cells, int nsweeps, cudaStream_t st);
+// Per-cell FP64 momentum records, by sweep step as MomRec32: {AE AW}, {AN AS}, {AEE AWW}, {ANN ASS} and
+// {AP, pressure term}; 80 bytes per cell, 48 with two colours, whose far links are not stored. Null: the
+// sweeps recompute the coefficients (launch_mom_prep, launch_mom_sweep).
+struct MomRec64 {
+    double2* r[5];
+};
+// Arrays of a MomRec64 that a colour count uses, in its order.
+inline bool mom_rec_used(int ncol, int k) { return ncol == 5 || (k != 2 && k != 3); }
+// Momentum prep with records: |R| into cells, AP over the update range, the records.
+void launch_mom_prep_rec(const DevParams& p, bool v_component, const double* x, const double* oth, const double* pf,
+                         double* AP, double* cells, MomRec64 rec, cudaStream_t st);
+// One whole multicolour sweep xin -> xout from the records (every cell of xout written). *err gets a bit
+// if a bounded wait for the record copies gave up.
+void launch_mom_sweep_rec(const DevParams& p, bool v_component, const double* xin, double* xout, MomRec64 rec,
+                          int seg_rows, unsigned* err, cudaStream_t st);
+// Resident CTAs per SM of that sweep and its threads per CTA (for stream_seg_rows).
+int mom_rec_blocks_per_sm(int ncol);
+int mom_rec_threads();
 // One whole multicolour sweep xin -> xout (every cell of xout written).
 void launch_mom_sweep(const DevParams& p, bool v_component, const double* xin, double* xout,
                       const double* xF, const double* oth, const double* pf, int seg_rows,

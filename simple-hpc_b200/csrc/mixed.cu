@@ -19,6 +19,7 @@
 // p' vanish too, whatever their precision.
 #include "kernels.hpp"
 #include "blocksum.cuh"
+#include "bulk.cuh"
 #include "stencil.cuh"
 
 #include <cooperative_groups.h>
@@ -36,20 +37,6 @@ __device__ __forceinline__ std::size_t ix(const DevParams& p, int i, int j) {
 }
 
 // The correction sweep (k_corr_stream and its launchers) is built in the FP32 unit only.
-#ifdef SGPU_FLOAT_UNIT
-template <class T> __device__ __forceinline__ void cp_async(T* smem, const T* gmem) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    if (sizeof(T) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-#endif
 
 // The tile of one prep block: 32 columns x kTileRows rows, 32 x 8 threads, kTileRows / 8 cells per
 // thread. The block's partial sum (a block tree's tail: one thread adding the warps' sums) is paid
@@ -145,43 +132,6 @@ __global__ void __launch_bounds__(256, 4)
 // own columns, so a slot is refilled as soon as its owner has written the row out.
 constexpr int kRing = 16;
 constexpr int kRecAhead = 2; // record slots: super-steps whose records are in flight
-constexpr int kSpinLimit = 1 << 20; // bounded mbarrier waits (a give-up is reported, never a hang)
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(b)) : "memory");
-}
-// Arrive (count one) and expect `bytes` of bulk copies to complete on b.
-__device__ __forceinline__ void mbar_arrive_expect(unsigned long long* b, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(b)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned long long* b, unsigned parity) {
-    unsigned done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 " selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done)
-                 : "r"(smem_u32(b)), "r"(parity)
-                 : "memory");
-    return done != 0;
-}
-// Wait for phase `parity` of b to complete, at most kSpinLimit polls. Returns false on a give-up,
-// which also sets *err.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity, unsigned* err,
-                                          int limit = kSpinLimit) {
-    for (int it = 0; !mbar_test(b, parity); ++it)
-        if (it >= limit) {
-            atomicOr(err, 1u);
-            return false;
-        }
-    return true;
-}
-
 // The give-up path of mbar_wait, exercised on purpose: one warp waits, at most `polls` polls, for a
 // phase of an mbarrier that nothing ever arrives on, so the wait must end by giving up and setting
 // *err. No copy is in flight and nothing else waits on this warp: the kernel returns normally.
@@ -194,15 +144,6 @@ __global__ void k_wait_selftest(int polls, unsigned* err) {
     __syncthreads();
     mbar_wait(&bar, 0, err, polls);
 }
-// One bulk copy (TMA, no tensor map) of `bytes` from global to this CTA's shared memory, completing
-// on mbarrier b. Both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* b) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(b))
-                 : "memory");
-}
-
 // Shared memory of k_corr_stream: the e ring (kRing rows of NT floats), then kRecAhead x SPB record
 // slots, each one step row of NT cells in three arrays (near links, far links for five colours,
 // {1/AP, R}).
@@ -845,7 +786,6 @@ void launch_corr_m(const DevParams& p, const float* ein, float* eout, MomRec32 r
                    int seg_rows, double* xfinal, unsigned* err, cudaStream_t st) {
     launch_corr<NCOL, V, kCorrNT, kCorrMinb>(p, ein, eout, rec, e_zero, seg_rows, xfinal, err, st);
 }
-
 
 // The cluster sweep's plan: bands of at least kCorrGhost rows, the shared memory of the largest
 // within a CTA's 227 KB; false where the component does not fit.

@@ -12,6 +12,7 @@
 #include "cnn.hpp"
 #include "kernels.hpp"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -126,9 +127,7 @@ struct Solver {
         // A batch fills the GPU with many cavities' kernels, so SM time, not latency, bounds it: the
         // single-CTA tail (one SM) instead of the cluster tail (16 SMs for a shorter time).
         mg_tail32 = mg_tail64 = mg_tail;
-        if (fast)
-            seg_rows = mixed ? stream_seg_rows(dp, sms, corr_blocks_per_sm(dp.ncol), 0, corr_threads())
-                             : stream_seg_rows(dp, sms, 2, 0);
+        if (fast) set_seg_rows(0);
     }
 
     int ncol = 5;
@@ -175,6 +174,22 @@ struct Solver {
                                     sizeof(double) * g.ncols, g.nrows, cudaMemcpyDeviceToHost, st));
         SGPU_CUDA(cudaStreamSynchronize(st));
     }
+    bool is_coef(int id) const {
+        return (id >= SGPU_F_CU_AE && id < SGPU_F_CU_AP) || (id >= SGPU_F_CV_AE && id < SGPU_F_CV_AP);
+    }
+    // Copies field id to the host; false for an unknown id. A coefficient array that nothing has written
+    // yet is zero.
+    bool fetch_field(int id, double* host) {
+        if (is_coef(id) && !coefs()) {
+            std::memset(host, 0, sizeof(double) * static_cast<std::size_t>(g.nrows) * g.ncols);
+            return true;
+        }
+        double* f = field_ptr(id);
+        if (!f) return false;
+        form_p_links_if_stale(id);
+        download(f, host);
+        return true;
+    }
     double* field_ptr(int id) {
         if (id == SGPU_F_U) return u;
         if (id == SGPU_F_V) return v;
@@ -199,16 +214,24 @@ struct Solver {
     }
 
     // ---- phases (enqueue only) ----
-    void assemble_u() { launch_assemble_u(dp, u, v, cu, st); }
+    void assemble_u() {
+        need_coefs();
+        launch_assemble_u(dp, u, v, cu, st);
+    }
     void bc_u() { launch_bc_u(dp, u, st); }
     void residual_u(double* out) {
+        need_coefs();
         launch_residual_u_cells(dp, cu, u, pf, cells, st);
         launch_ordered_sum(cells, 0, prm.NY - 1, prm.NX, prm.NY - 1, 1, out, ss, nullptr, st);
     }
     void sweep_u(int n);
-    void assemble_v() { launch_assemble_v(dp, u, v, cv, st); }
+    void assemble_v() {
+        need_coefs();
+        launch_assemble_v(dp, u, v, cv, st);
+    }
     void bc_v() { launch_bc_v(dp, v, st); }
     void residual_v(double* out) {
+        need_coefs();
         launch_residual_v_cells(dp, cv, v, pf, cells, st);
         launch_ordered_sum(cells, 0, prm.NY, prm.NX - 1, prm.NY, 1, out, ss, nullptr, st);
     }
@@ -256,7 +279,8 @@ struct Solver {
             return;
         }
         mark(vcomp ? SGPU_PH_ASSEMBLE_V : SGPU_PH_ASSEMBLE_U);
-        launch_mom_prep(dp, vcomp, x, oth, pf, xF, AP, cplane, st);
+        if (rec64.r[0]) launch_mom_prep_rec(dp, vcomp, x, oth, pf, AP, cplane, rec64, st);
+        else launch_mom_prep(dp, vcomp, x, oth, pf, xF, AP, cplane, st);
         mark(vcomp ? SGPU_PH_RESIDUAL_V : SGPU_PH_RESIDUAL_U);
         if (!deferred) momentum_sum(vcomp, res, cplane, false);
         mark(vcomp ? SGPU_PH_SWEEP_V : SGPU_PH_SWEEP_U);
@@ -264,12 +288,81 @@ struct Solver {
         double* out = tmp;
         sweep_mark(vcomp, 0, n);
         for (int k = 0; k < n; ++k) {
-            launch_mom_sweep(dp, vcomp, in, out, xF, oth, pf, seg_rows, st);
+            if (rec64.r[0]) launch_mom_sweep_rec(dp, vcomp, in, out, rec64, seg_rows, corr_err, st);
+            else launch_mom_sweep(dp, vcomp, in, out, xF, oth, pf, seg_rows, st);
             std::swap(in, out);
         }
         sweep_mark(vcomp, 1, n);
         if (in != x) launch_copy(in, x, g.elems(), st);
         if (deferred) momentum_sum(vcomp, res, cplane, true); // beside the next prep / assemble_p
+    }
+
+    // FP64 momentum records (fused.cu): stored coefficients for the sweeps of grids that do not fit a
+    // cluster. Where the device has no memory for them (or SGPU_MOM_RECORDS=0) the sweeps recompute the
+    // coefficients: the same bits.
+    MomRec64 rec64{};
+    void alloc_records() {
+        if (!fast || mixed || (mom_cluster_fits(dp, false) && mom_cluster_fits(dp, true))) return;
+        if (const char* e = std::getenv("SGPU_MOM_RECORDS"))
+            if (std::atoi(e) == 0) return;
+        const std::size_t n =
+            g.elems() + static_cast<std::size_t>(kRecExtraRows) * g.pitch + kRecFrontCols + kRecBackCols;
+        try {
+            for (int k = 0; k < 5; ++k)
+                if (mom_rec_used(ncol, k)) rec64.r[k] = dalloc<double2>(n) + kRecFrontCols;
+            corr_err = dalloc<unsigned>(1);
+        } catch (const Error& e) {
+            if (e.code != SGPU_E_NOMEM) throw;
+            free_records();
+        }
+        if (rec64.r[0]) set_seg_rows(min_seg);
+    }
+    void free_records() {
+        (void)cudaGetLastError();
+        for (double2*& r : rec64.r) {
+            if (r) dfree(r - kRecFrontCols);
+            r = nullptr;
+        }
+    }
+    void dfree(void* q) {
+        const auto it = std::find(allocs.begin(), allocs.end(), q);
+        if (it == allocs.end()) return;
+        allocs.erase(it);
+        cudaFree(q);
+    }
+    void set_seg_rows(int min_rows) {
+        if (mixed) seg_rows = stream_seg_rows(dp, sms, corr_blocks_per_sm(dp.ncol), min_rows, corr_threads());
+        else if (rec64.r[0]) seg_rows = stream_seg_rows(dp, sms, mom_rec_blocks_per_sm(dp.ncol), min_rows, mom_rec_threads());
+        else seg_rows = stream_seg_rows(dp, sms, 2, min_rows);
+    }
+
+    // The coefficient arrays but AP belong to the per-phase entry points: allocated when one of those (or
+    // an upload) first needs them; the fast and mixed iterations never do. If the memory they need is
+    // what the records hold, the records go.
+    bool coefs() const { return cu.a[0] != nullptr; }
+    void need_coefs() {
+        if (coefs()) return;
+        for (int attempt = 0;; ++attempt) {
+            double* got[16] = {};
+            try {
+                for (double*& q : got) q = field();
+                for (int k = 0; k < 8; ++k) {
+                    cu.a[k] = got[k];
+                    cv.a[k] = got[8 + k];
+                }
+                return;
+            } catch (const Error& e) {
+                (void)cudaGetLastError();
+                for (double* q : got)
+                    if (q) dfree(q);
+                if (e.code != SGPU_E_NOMEM || attempt || !rec64.r[0]) throw;
+                sync();
+                destroy_iter_graph(run_graph); // it holds the records
+                run_graph = nullptr;
+                free_records();
+                set_seg_rows(min_seg);
+            }
+        }
     }
 
     // res_u / res_v: the ordered sum of |R| over the residual range. The sums feed only the stopping
@@ -401,8 +494,8 @@ struct Solver {
         p_links_stale = false;
     }
     MomRec32 rec32{};                 // per-cell FP32 records: coefficients, 1/AP, R
-    unsigned* corr_err = nullptr;     // device word: a correction sweep's bounded wait gave up
-    // Raises SGPU_E_TIMEOUT if a correction sweep since the last check gave up waiting for its
+    unsigned* corr_err = nullptr;     // device word: a record sweep's bounded wait gave up
+    // Raises SGPU_E_TIMEOUT if a record sweep since the last check gave up waiting for its
     // record copies (its results are then not to be trusted); clears the word.
     void check_pipeline() {
         if (net) net->check_error(st);
@@ -412,7 +505,7 @@ struct Solver {
         sync();
         if (h) {
             SGPU_CUDA(cudaMemsetAsync(corr_err, 0, sizeof h, st));
-            throw Error(SGPU_E_TIMEOUT, "correction sweep: a bounded wait for its record copies ran out");
+            throw Error(SGPU_E_TIMEOUT, "momentum sweep: a bounded wait for its record copies ran out");
         }
     }
     // FP64 defect correction of the p' solve in tolerance mode: the FP64 iterate ping-pongs between
@@ -715,8 +808,9 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
     u = field();
     v = field();
     pf = field();
-    for (int k = 0; k < 9; ++k) cu.a[k] = field();
-    for (int k = 0; k < 9; ++k) cv.a[k] = field();
+    cu.a[8] = field();
+    cv.a[8] = field();
+    if (p.momentum_solver != SGPU_MOM_GS_MULTICOLOUR) need_coefs();
     w.AEP = field();
     w.AWP = field();
     w.ANP = field();
@@ -840,7 +934,7 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
                         "mg and 1 <= mg_pre <= 4, 0 <= mg_post <= 4");
         mixed = true;
         init_mixed_kernels();
-        seg_rows = stream_seg_rows(dp, sms, corr_blocks_per_sm(dp.ncol), min_seg, corr_threads());
+        set_seg_rows(min_seg);
         const std::size_t nrec =
             g.elems() + static_cast<std::size_t>(kRecExtraRows) * g.pitch + kRecFrontCols + kRecBackCols;
         rec32.near_links = dalloc<float4>(nrec) + kRecFrontCols;
@@ -883,6 +977,7 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
         net = own_net.get();
     }
 
+    alloc_records(); // last: everything a solve cannot do without has its memory
     if (hu) upload(u, hu);
     if (hv) upload(v, hv);
     if (hp) upload(pf, hp);
@@ -911,6 +1006,7 @@ Solver::~Solver() {
 // sweep_u_batch (momentum_u.cpp:162-171).
 void Solver::sweep_u(int n) {
     if (n <= 0) return;
+    need_coefs();
     if (prm.momentum_solver == SGPU_MOM_JACOBI) {
         launch_copy(u, scratch, g.elems(), st);
         for (int k = 0; k < n; ++k) {
@@ -926,6 +1022,7 @@ void Solver::sweep_u(int n) {
 // sweep_v_batch (momentum_v.cpp:164-173).
 void Solver::sweep_v(int n) {
     if (n <= 0) return;
+    need_coefs();
     if (prm.momentum_solver == SGPU_MOM_JACOBI) {
         launch_copy(v, scratch, g.elems(), st);
         for (int k = 0; k < n; ++k) {
@@ -1678,10 +1775,8 @@ int sgpu_download(sgpu_handle* h, int id, double* host) {
     SGPU_NEED_HANDLE(h);
     if (!host) return sgpu::fail(SGPU_E_INVALID, "sgpu_download: null buffer");
     return guarded([&] {
-        double* f = h->s->field_ptr(id);
-        if (!f) throw sgpu::Error(SGPU_E_INVALID, "sgpu_download: unknown field id " + std::to_string(id));
-        h->s->form_p_links_if_stale(id);
-        h->s->download(f, host);
+        if (!h->s->fetch_field(id, host))
+            throw sgpu::Error(SGPU_E_INVALID, "sgpu_download: unknown field id " + std::to_string(id));
     });
 }
 
@@ -1689,6 +1784,7 @@ int sgpu_upload(sgpu_handle* h, int id, const double* host) {
     SGPU_NEED_HANDLE(h);
     if (!host) return sgpu::fail(SGPU_E_INVALID, "sgpu_upload: null buffer");
     return guarded([&] {
+        if (h->s->is_coef(id)) h->s->need_coefs();
         double* f = h->s->field_ptr(id);
         if (!f) throw sgpu::Error(SGPU_E_INVALID, "sgpu_upload: unknown field id " + std::to_string(id));
         h->s->upload(f, host);
@@ -2077,8 +2173,13 @@ int sgpu_batch_autotune(sgpu_batch* b, int* chosen) {
                     if (sv.mixed)
                         sgpu::launch_corr_sweep(sv.dp, false, sv.e32[0], sv.e32[1], sv.rec32, true, seg,
                                                 sv.corr_err, sv.st);
+                    else if (sv.rec64.r[0])
+                        sgpu::launch_mom_sweep_rec(sv.dp, false, sv.u, sv.tmp, sv.rec64, seg, sv.corr_err, sv.st);
                     else sgpu::launch_mom_sweep(sv.dp, false, sv.u, sv.tmp, sv.xF, sv.v, sv.pf, seg, sv.st);
                 };
+                // real records to time the sweep on (AP into scratch: xF has no other use with records)
+                if (sv.rec64.r[0])
+                    sgpu::launch_mom_prep_rec(sv.dp, false, sv.u, sv.v, sv.pf, sv.xF, sv.cells, sv.rec64, sv.st);
                 int pick = heur;
                 float tbest = 1e30f;
                 for (int seg : cand) {
@@ -2191,10 +2292,8 @@ int sgpu_batch_download(sgpu_batch* b, int index, int field_id, double* host) {
     return guarded([&] {
         SGPU_CUDA(cudaStreamSynchronize(b->st));
         sgpu::Solver& sv = *b->s[index];
-        double* f = sv.field_ptr(field_id);
-        if (!f) throw sgpu::Error(SGPU_E_INVALID, "sgpu_batch_download: unknown field id " + std::to_string(field_id));
-        sv.form_p_links_if_stale(field_id);
-        sv.download(f, host);
+        if (!sv.fetch_field(field_id, host))
+            throw sgpu::Error(SGPU_E_INVALID, "sgpu_batch_download: unknown field id " + std::to_string(field_id));
     });
 }
 

@@ -32,3 +32,40 @@ def test_small_grids_bit_for_bit(sgpu_mod, oracle_mod, nx, ny, scheme, order, in
                      else (slice(p.H + 1, p.H + nx), slice(p.H + 1, p.H + ny + 1)))
                 a, b = a[r].copy(), b[r].copy()
             assert bit_equal(a, b), f"field {f}: " + describe_diff(a, b)
+
+
+@pytest.mark.parametrize("nx,ny,scheme,order", [(300, 520, "QUICK", 4), (530, 120, "QUICK", 2), (260, 300, "UDS", 2),
+                                                (420, 210, "UDS", 4)])
+def test_stored_and_recomputed_coefficients_same_bits(sgpu_mod, monkeypatch, nx, ny, scheme, order):
+    """Grids past the cluster: sweeps from stored coefficients and sweeps that recompute them (a device
+    without memory for the records), over several strips and segments and an odd sweep count."""
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x=str(nx), N_cells_y=str(ny), Re="700", convection_scheme=scheme, diffusion_order=str(order),
+               momentum_solver="gs_multicolour", pressure_solver="mg", maxit="5", error_tolerance="0",
+               maxit_inner_u="3", maxit_inner_v="4")
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("SGPU_MOM_RECORDS", on)
+        with sgpu_mod.Solver(sgpu_mod.params_from_config(config_text(cfg))) as g:
+            _, log = g.run(5)
+            out.append([log] + [g.download(f) for f in (0, 1, 2, sgpu_mod.F_PC)])
+    for a, b in zip(*out):
+        assert bit_equal(a, b), describe_diff(a, b)
+
+
+def test_coefficient_arrays_appear_with_the_per_phase_calls(sgpu_mod, oracle_mod):
+    """The coefficient arrays are allocated when a per-phase call needs them: zero before, the oracle's after,
+    and an iteration in between changes nothing about that."""
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x="250", N_cells_y="240", momentum_solver="gs_multicolour", pressure_solver="mg", maxit="2")
+    p = sgpu_mod.params_from_config(config_text(cfg))
+    o = oracle_mod.Oracle(p)
+    with sgpu_mod.Solver(p) as g:
+        g.run(2)
+        o.run(2)
+        assert not g.download(sgpu_mod.CU[0]).any() and not g.download(sgpu_mod.CV[7]).any()
+        g.assemble_u()
+        o.assemble_u()
+        for f in sgpu_mod.CU:
+            a, b = (x[p.H:p.H + 250, p.H:p.H + 241].copy() for x in (g.download(f), o.get(f)))
+            assert bit_equal(a, b), f"field {f}: " + describe_diff(a, b)
