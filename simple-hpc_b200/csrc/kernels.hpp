@@ -162,6 +162,11 @@ void launch_cg_dq(const DevParams& p, PressurePtr w, CgPtr cg, const CgScalars* 
 void launch_cg_update(const DevParams& p, PressurePtr w, CgPtr cg, const CgScalars* sc,
                       double* cells, std::size_t plane, cudaStream_t st);
 void launch_cg_dir(const DevParams& p, CgPtr cg, const CgScalars* sc, cudaStream_t st);
+// The whole solve (p' zero on entry, its mean removed on return) in one cooperative kernel; false, and
+// nothing is launched, where the grid does not fit one CTA per SM. sums: 12 NX words of scratch; *err gets
+// a bit if a bounded wait gave up.
+bool launch_cg_solve(const DevParams& p, PressurePtr w, CgPtr cg, CgScalars* sc, unsigned long long* sums, unsigned* err,
+                     int sms, cudaStream_t st);
 
 // ---- mixed precision (mixed.cu) ----
 void init_mixed_kernels();

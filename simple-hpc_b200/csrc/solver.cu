@@ -88,6 +88,8 @@ struct Solver {
     double* scratch = nullptr; // Jacobi previous iterate (u, v and p')
     CgPtr cg{};
     CgScalars* cgs = nullptr;
+    unsigned long long* cg_sums = nullptr; // the one-kernel solve's row sums
+    unsigned* cg_err = nullptr;            // device word: a wait of that kernel gave up
     double* cells = nullptr; // 4 planes of NX x NY per-cell values for the ordered sums
     std::size_t plane = 0;
     double* sums = nullptr;  // 32 device doubles: results of ordered sums
@@ -499,6 +501,15 @@ struct Solver {
     // record copies (its results are then not to be trusted); clears the word.
     void check_pipeline() {
         if (net) net->check_error(st);
+        if (cg_err) {
+            unsigned h = 0;
+            SGPU_CUDA(cudaMemcpyAsync(&h, cg_err, sizeof h, cudaMemcpyDeviceToHost, st));
+            sync();
+            if (h) {
+                SGPU_CUDA(cudaMemsetAsync(cg_err, 0, sizeof h, st));
+                throw Error(SGPU_E_TIMEOUT, "conjugate gradients: a bounded wait for the other blocks' sums ran out");
+            }
+        }
         if (!corr_err) return;
         unsigned h = 0;
         SGPU_CUDA(cudaMemcpyAsync(&h, corr_err, sizeof h, cudaMemcpyDeviceToHost, st));
@@ -821,12 +832,14 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
     if (p.momentum_solver == SGPU_MOM_JACOBI || p.pressure_solver == SGPU_P_JACOBI)
         scratch = field();
     fast = p.momentum_solver == SGPU_MOM_GS_MULTICOLOUR;
-    if (fast) {
-        xF = field();
-        tmp = field();
+    {
         int dev = 0;
         SGPU_CUDA(cudaGetDevice(&dev));
         SGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    }
+    if (fast) {
+        xF = field();
+        tmp = field();
         seg_rows = stream_seg_rows(dp, sms, 2, min_seg);
         if (const char* e = std::getenv("SGPU_SIDE_SUMS")) side_sums = std::atoi(e) != 0;
         ss_side.max_rows = p.nrows;
@@ -848,6 +861,8 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
         cg.d = field();
         cg.q = field();
         cgs = dalloc<CgScalars>(1);
+        cg_sums = dalloc<unsigned long long>(12 * static_cast<std::size_t>(p.NX));
+        cg_err = dalloc<unsigned>(1);
         CgScalars init{};
         init.n = static_cast<double>(p.NX) * p.NY;
         init.tol = p.pressure_tolerance;
@@ -1056,6 +1071,10 @@ void Solver::solve_jacobi() {
 // solve_pc_cg (pressure.cpp:208-317) with device-resident scalars.
 void Solver::solve_cg() {
     SGPU_CUDA(cudaMemsetAsync(w.pc, 0, g.bytes(), st));
+    if (launch_cg_solve(dp, w, cg, cgs, cg_sums, cg_err, sms, st)) {
+        cg_stats_pending = true;
+        return;
+    }
     const double* b0 = at(w.b, prm.H, prm.H + 1);
     launch_ordered_sum(b0, 0, g.pitch, prm.NX, prm.NY, 1, sums, ss, nullptr, st);
     launch_cg_scalars(0, cgs, sums, st);
