@@ -168,7 +168,17 @@ void launch_cg_dir(const DevParams& p, CgPtr cg, const CgScalars* sc, cudaStream
 bool launch_cg_solve(const DevParams& p, PressurePtr w, CgPtr cg, CgScalars* sc, unsigned long long* sums, unsigned* err,
                      int sms, cudaStream_t st);
 
+// State of a tolerance-driven V-cycle loop that runs inside a graph (mg_mode = tolerance): the cycles of the
+// current p' solve, ||b||^2 and the relative residual after the last one.
+struct TolState {
+    double bb, rel;
+    int cycles;
+};
+
 // ---- mixed precision (mixed.cu) ----
+// With `state` (a captured loop) launch_dc_update takes pnew on even cycles (from 0) and swaps the two on odd
+// ones, and launch_correct_dc reads pc64 after an odd number of cycles (or none) and pc64b after an even one;
+// launch_dc_zero_if gives p' = 0 where the loop ran no cycle.
 void init_mixed_kernels();
 // Resident CTAs per SM of the FP32 correction sweep (its register and shared-memory footprint).
 int corr_blocks_per_sm(int ncol);
@@ -223,9 +233,11 @@ int launch_dc_rhs0(const DevParams& p, const double* bfield, const double* sum_b
                    double* part, cudaStream_t st);
 int launch_dc_update(const DevParams& p, const double* APU, const double* APV, const double* bfield,
                      const double* sum_b, const LevelView32& L0, const double* pold, double* pnew, bool first,
-                     double* part, cudaStream_t st);
+                     double* part, cudaStream_t st, const TolState* state = nullptr);
 void launch_correct_dc(const DevParams& p, const double* pc64, const double* sum_pc, const double* APU,
-                       const double* APV, double* u, double* v, double* pf, cudaStream_t st);
+                       const double* APV, double* u, double* v, double* pf, cudaStream_t st,
+                       const double* pc64b = nullptr, const TolState* state = nullptr);
+void launch_dc_zero_if(const TolState* state, double* pc64, std::size_t n, double* sum_pc, cudaStream_t st);
 void launch_pc_from64(const DevParams& p, const double* src, const double* sum_pc, double* dst, cudaStream_t st);
 void launch_b_to_f32(const DevParams& p, const double* bfield, const double* sum_b,
                      const LevelView32& L0, cudaStream_t st);

@@ -677,8 +677,17 @@ __global__ void __launch_bounds__(256)
     k_dc_update(DevParams p, const double* __restrict__ APU, const double* __restrict__ APV,
                 const double* __restrict__ bfield, const double* __restrict__ sum_b,
                 const float* __restrict__ e, int lde, const double* __restrict__ pold,
-                double* __restrict__ pnew, int first, LevelView32 L0, double* __restrict__ part) {
+                double* __restrict__ pnew, int first, const TolState* __restrict__ state, LevelView32 L0,
+                double* __restrict__ part) {
     __shared__ double s_rr[8], s_ps[8];
+    if (state) { // a cycle of a captured loop: which array is which, and whether it is the first, from the device
+        first = state->cycles == 0;
+        if (state->cycles & 1) {
+            const double* t = pold;
+            pold = pnew;
+            pnew = const_cast<double*>(t);
+        }
+    }
     const int J = static_cast<int>(blockIdx.x * 32 + threadIdx.x);
     const int I0 = static_cast<int>(blockIdx.y * kTileRows + threadIdx.y);
     const double m = *sum_b / (static_cast<double>(p.NX) * p.NY);
@@ -725,9 +734,12 @@ __global__ void __launch_bounds__(256)
 }
 
 // correct (pressure.cpp:136-157) in FP64 from the FP64 p' of the defect correction minus its mean.
-__global__ void k_correct_dc(DevParams p, const double* __restrict__ pc64, const double* __restrict__ sum_pc,
+// state (not null): pc64 after an odd number of cycles (or none), pc64b after an even one.
+__global__ void k_correct_dc(DevParams p, const double* __restrict__ pc64, const double* __restrict__ pc64b,
+                             const TolState* __restrict__ state, const double* __restrict__ sum_pc,
                              const double* __restrict__ APU, const double* __restrict__ APV, double* u,
                              double* v, double* pf) {
+    if (state && state->cycles > 0 && !(state->cycles & 1)) pc64 = pc64b;
     const int J = static_cast<int>(blockIdx.x * 32 + threadIdx.x);
     const int I = static_cast<int>(blockIdx.y * 8 + threadIdx.y);
     if (I >= p.NX || J >= p.NY) return;
@@ -738,6 +750,15 @@ __global__ void k_correct_dc(DevParams p, const double* __restrict__ pc64, const
     if (j <= p.NY + H - 1) u[q] += p.dy * (pc - (pc64[q + 1] - m)) / APU[q];
     if (i >= H + 1) v[q] += p.dx * (pc - (pc64[q - p.pitch] - m)) / APV[q];
     pf[q] += p.ap * pc;
+}
+
+// p' = 0 and its sum where the loop ran no cycle (b equal to its mean).
+__global__ void k_dc_zero_if(const TolState* __restrict__ state, double* __restrict__ pc64, std::size_t n, double* sum_pc) {
+    if (state->cycles > 0) return;
+    for (std::size_t k = blockIdx.x * static_cast<std::size_t>(blockDim.x) + threadIdx.x; k < n;
+         k += static_cast<std::size_t>(gridDim.x) * blockDim.x)
+        pc64[k] = 0.0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *sum_pc = 0.0;
 }
 
 // The p' field a download shows: the FP64 iterate minus its mean (src may equal dst).
@@ -923,18 +944,24 @@ int launch_dc_rhs0(const DevParams& p, const double* bfield, const double* sum_b
 
 int launch_dc_update(const DevParams& p, const double* APU, const double* APV, const double* bfield,
                      const double* sum_b, const LevelView32& L0, const double* pold, double* pnew, bool first,
-                     double* part, cudaStream_t st) {
+                     double* part, cudaStream_t st, const TolState* state) {
     const dim3 grid((p.NY + 31) / 32, (p.NX + kTileRows - 1) / kTileRows);
     k_dc_update<<<grid, dim3(32, 8), 0, st>>>(p, APU, APV, bfield, sum_b, L0.x, L0.stride, pold, pnew,
-                                               first ? 1 : 0, L0, part);
+                                               first ? 1 : 0, state, L0, part);
     SGPU_LAUNCH();
     return static_cast<int>(grid.x * grid.y);
 }
 
 void launch_correct_dc(const DevParams& p, const double* pc64, const double* sum_pc, const double* APU,
-                       const double* APV, double* u, double* v, double* pf, cudaStream_t st) {
+                       const double* APV, double* u, double* v, double* pf, cudaStream_t st, const double* pc64b,
+                       const TolState* state) {
     const dim3 grid((p.NY + 31) / 32, (p.NX + 7) / 8);
-    k_correct_dc<<<grid, dim3(32, 8), 0, st>>>(p, pc64, sum_pc, APU, APV, u, v, pf);
+    k_correct_dc<<<grid, dim3(32, 8), 0, st>>>(p, pc64, pc64b, state, sum_pc, APU, APV, u, v, pf);
+    SGPU_LAUNCH();
+}
+
+void launch_dc_zero_if(const TolState* state, double* pc64, std::size_t n, double* sum_pc, cudaStream_t st) {
+    k_dc_zero_if<<<296, 256, 0, st>>>(state, pc64, n, sum_pc);
     SGPU_LAUNCH();
 }
 

@@ -74,6 +74,22 @@ static void diffusive_host(const sgpu_params_t& p, bool band_or_order2, double o
 struct IterGraph;
 void destroy_iter_graph(IterGraph* g);
 
+// The stopping test of the tolerance-driven V-cycles (mg_mode = tolerance) as the condition of a WHILE node,
+// with the host loop's arithmetic (Solver::run_cycles, run_cycles_dc): begin with ||b||^2, then one step per
+// cycle with ||r||^2.
+__global__ void k_tol_begin(TolState* t, const double* bb, int maxc, cudaGraphConditionalHandle h) {
+    t->bb = *bb;
+    t->cycles = 0;
+    t->rel = *bb > 0.0 ? 1.0 : 0.0;
+    cudaGraphSetConditional(h, *bb > 0.0 && maxc > 0 ? 1u : 0u);
+}
+__global__ void k_tol_step(TolState* t, const double* rr, double tol, int maxc, cudaGraphConditionalHandle h) {
+    const double nb = sqrt(t->bb), nr = sqrt(*rr);
+    t->rel = nr / nb;
+    const int c = ++t->cycles;
+    cudaGraphSetConditional(h, !(nr <= tol * nb) && c < maxc ? 1u : 0u);
+}
+
 struct Solver {
     sgpu_params_t prm{};
     DevParams dp{};
@@ -473,6 +489,7 @@ struct Solver {
 
     void iteration_enqueue(double* res3) {
         ev_n = 0;
+        tol_stats = false;
         if (mixed) mixed_iteration_enqueue(res3);
         else if (fast) fast_iteration_enqueue(res3);
         else outer_iteration_enqueue(res3);
@@ -485,6 +502,7 @@ struct Solver {
     bool p_links_stale = false;
     bool pc_stale = false; // the mixed iteration keeps p' in FP32; the FP64 field is formed on download
     void form_p_links_if_stale(int id) {
+        if (id == SGPU_F_PC) fetch_tol();
         if (pc_stale && id == SGPU_F_PC) { // p' of the last mixed iteration, kept in FP32 (or FP64)
             if (pc_dc_src) launch_pc_from64(dp, pc_dc_src, sums + 26, w.pc, st);
             else launch_pc_from32(dp, lv32[0], sums + 26, w.pc, st);
@@ -577,10 +595,7 @@ struct Solver {
         pc_dc_src = nullptr;
         int nbb = 0;
         if (dc_mode) {
-            if (!dc[0]) {
-                dc[0] = field();
-                dc[1] = field();
-            }
+            need_dc();
             nbb = launch_dc_rhs0(dp, w.b, sums + 25, lv32[0], part, st);
         } else {
             launch_b_to_f32(dp, w.b, sums + 25, lv32[0], st);
@@ -607,7 +622,18 @@ struct Solver {
                 launch_mg_up<float>(lv32[l + 1], lv32[l], mg32_x2[l], lv32[l].x, prm.mg_omega,
                                     prm.mg_post, sms, min_seg, st);
         };
-        if (dc_mode) {
+        if (dc_mode && capturing) {
+            launch_sum_partials(part, nbb, 1, 0, sums + 28, nullptr, st);
+            capture_while(sums + 28, sums + 29, [&] {
+                if (mg_tail32 == 0) launch_zero_x(L0, st);
+                vcycle32(true);
+                const int nb = launch_dc_update(dp, cu.a[8], cv.a[8], w.b, sums + 25, L0, dc[1], dc[0], true, part, st, tol);
+                launch_sum_partials(part, nb, 2, nb, sums + 29, sums + 26, st);
+            });
+            launch_dc_zero_if(tol, dc[0], g.elems(), sums + 26, st);
+            mark(SGPU_PH_CORRECT);
+            launch_correct_dc(dp, dc[0], sums + 26, cu.a[8], cv.a[8], u, v, pf, st, dc[1], tol);
+        } else if (dc_mode) {
             last_vcycles = run_cycles_dc(L0, guess, nbb, vcycle32); // p' in FP64, its sum in sums[26]
             mark(SGPU_PH_CORRECT);
             launch_correct_dc(dp, pc_dc_src, sums + 26, cu.a[8], cv.a[8], u, v, pf, st);
@@ -669,6 +695,75 @@ struct Solver {
         return run;
     }
 
+    // ---- the tolerance-driven cycles inside a graph ----
+    // While an iteration is captured, its V-cycle loop becomes a WHILE node: no host round trip per cycle.
+    bool capturing = false;
+    TolState* tol = nullptr;   // device; its cycles and residual are the last solve's while tol_stats
+    bool tol_stats = false;
+    // What a capture may not allocate.
+    void before_capture() {
+        if (prm.pressure_solver != SGPU_P_MG || prm.mg_mode != SGPU_MG_TOLERANCE) return;
+        if (!tol) tol = dalloc<TolState>(1);
+        if (mixed) need_dc();
+        sync();
+    }
+    void need_dc() {
+        for (double*& d : dc)
+            if (!d) d = field();
+    }
+    template <class F> void capture_while(const double* bb, const double* rr, F&& cycle) {
+        cudaStreamCaptureStatus status{};
+        unsigned long long id = 0;
+        cudaGraph_t graph = nullptr;
+        SGPU_CUDA(cudaStreamGetCaptureInfo_v2(st, &status, &id, &graph, nullptr, nullptr));
+        cudaGraphNodeParams wp{};
+        wp.type = cudaGraphNodeTypeConditional;
+        wp.conditional.type = cudaGraphCondTypeWhile;
+        wp.conditional.size = 1;
+        SGPU_CUDA(cudaGraphConditionalHandleCreate(&wp.conditional.handle, graph, 0, 0));
+        const cudaGraphConditionalHandle h = wp.conditional.handle;
+        k_tol_begin<<<1, 1, 0, st>>>(tol, bb, prm.pressure_maxit, h);
+        SGPU_LAUNCH();
+        const cudaGraphNode_t* deps = nullptr;
+        std::size_t ndeps = 0;
+        SGPU_CUDA(cudaStreamGetCaptureInfo_v2(st, &status, &id, &graph, &deps, &ndeps));
+        cudaGraphNode_t node;
+        SGPU_CUDA(cudaGraphAddNode(&node, graph, deps, ndeps, &wp));
+        SGPU_CUDA(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
+        // the body is captured on a stream of its own; the launchers take the member
+        cudaStream_t outer = st, inner = nullptr;
+        SGPU_CUDA(cudaStreamCreateWithFlags(&inner, cudaStreamNonBlocking));
+        cudaGraph_t got = nullptr;
+        try {
+            SGPU_CUDA(cudaStreamBeginCaptureToGraph(inner, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                    cudaStreamCaptureModeRelaxed));
+            st = inner;
+            cycle();
+            k_tol_step<<<1, 1, 0, st>>>(tol, rr, prm.pressure_tolerance, prm.pressure_maxit, h);
+            SGPU_LAUNCH();
+            st = outer;
+            SGPU_CUDA(cudaStreamEndCapture(inner, &got));
+        } catch (...) {
+            st = outer;
+            (void)cudaStreamEndCapture(inner, &got);
+            cudaStreamDestroy(inner);
+            throw;
+        }
+        cudaStreamDestroy(inner);
+    }
+    // The last p' solve of a graph's tolerance loop, for the statistics and the p' field of a download.
+    void fetch_tol() {
+        if (!tol_stats) return;
+        tol_stats = false;
+        TolState h{};
+        SGPU_CUDA(cudaMemcpyAsync(&h, tol, sizeof h, cudaMemcpyDeviceToHost, st));
+        sync();
+        last_vcycles = h.cycles;
+        last_rel = h.rel;
+        last_rel_initial = 1.0;
+        if (mixed) pc_dc_src = dc[h.cycles > 0 && !(h.cycles & 1) ? 1 : 0];
+    }
+
     // V-cycles on level 0 (iterate L0.x, right-hand side L0.b). mg_mode = fixed: mg_cycles cycles
     // (the reference, multigrid.cpp:349-354). mg_mode = tolerance: cycles until the FP64 norm
     // ||b - A x|| <= pressure_tolerance ||b||, at most pressure_maxit; each norm is an ordered sum
@@ -688,6 +783,16 @@ struct Solver {
             launch_ordered_sum(cells, 0, L0.ny, nr, L0.ny, 1, slot, ss, nullptr, st);
             return fetch(slot);
         };
+        if (tol_mode && capturing) { // from zero (a warm start is never captured): x is the cleared array
+            launch_mg_b_sq(L0, cells, st);
+            launch_ordered_sum(cells, 0, L0.ny, nr, L0.ny, 1, sums + 28, ss, nullptr, st);
+            capture_while(sums + 28, sums + 29, [&] {
+                vcycle(false);
+                launch_mg_residual_sq(L0, cells, st);
+                launch_ordered_sum(cells, 0, L0.ny, nr, L0.ny, 1, sums + 29, ss, nullptr, st);
+            });
+            return 0;
+        }
         if (!tol_mode && !judge) { // the reference's fixed cycle count from zero
             for (int c = 0; c < prm.mg_cycles; ++c) vcycle(c == 0);
             return prm.mg_cycles;
@@ -1334,6 +1439,7 @@ struct IterGraph {
         std::vector<double> tol(n);
         std::vector<int> runmax(n);
         for (int c = 0; c < n; ++c) {
+            sv[c]->before_capture();
             sv[c]->sync();
             res[c] = sv[c]->res_dev;
             tol[c] = sv[c]->prm.error_tolerance;
@@ -1399,11 +1505,14 @@ struct IterGraph {
                 SGPU_CUDA(cudaStreamBeginCaptureToGraph(s.st, ib, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
                 try {
                     const long long before = g_launches.load();
+                    s.capturing = true;
                     s.iteration_enqueue(s.res_dev);
+                    s.capturing = false;
                     const long long captured = g_launches.load() - before;
                     kernels_per_iteration += captured;
                     count_launches(-captured); // captured, not run: counted when the graph runs
                 } catch (...) {
+                    s.capturing = false;
                     cudaGraph_t tmp = nullptr;
                     cudaStreamEndCapture(s.st, &tmp);
                     throw;
@@ -1632,10 +1741,10 @@ int sgpu_outer_iteration(sgpu_handle* h, double res[3], double* phase_seconds) {
 
 // sgpu_run without per-iteration host round trips: the iterations run inside one graph launch per
 // print interval (sgpu::IterGraph), the stopping rule and the residual log on the device. Used when
-// every outer iteration is a fixed sequence of launches (no CG, no tolerance-driven multigrid, no
-// warm start) and the per-phase timers are off.
+// every outer iteration is a sequence of launches that the device can decide (no CG, no warm start) and
+// the per-phase timers are off; tolerance-driven multigrid loops inside it (Solver::capture_while).
 static bool graphable(const sgpu::Solver& s) {
-    return s.prm.pressure_solver != SGPU_P_CG && s.prm.mg_mode != SGPU_MG_TOLERANCE && !s.net;
+    return s.prm.pressure_solver != SGPU_P_CG && !s.net;
 }
 
 // start > 0: the run continues one whose first `start` iterations ran on the host (sampled timers),
@@ -1676,6 +1785,10 @@ static bool run_graphed(sgpu::Solver& s, int maxit, double* log, int print_every
         SGPU_CUDA(cudaMemcpy(log + 4 * static_cast<std::size_t>(start), g.bd.log + 4 * static_cast<std::size_t>(start),
                              sizeof(double) * 4 * static_cast<std::size_t>(done - start), cudaMemcpyDeviceToHost));
     g.count(done - start, done - start);
+    if (done > start) { // what iteration_enqueue notes on the host when it launches an iteration
+        s.tol_stats = s.prm.pressure_solver == SGPU_P_MG && s.prm.mg_mode == SGPU_MG_TOLERANCE;
+        if (s.mixed) s.p_links_stale = s.pc_stale = true;
+    }
     out.iterations = done;
     out.converged = conv == 1 ? 1 : 0;
     diverged = conv < 0;
@@ -1873,6 +1986,7 @@ int sgpu_last_solve_stats(sgpu_handle* h, int* cg_iterations, int* mg_vcycles, i
             s.last_rel = sc.rel;
             s.cg_stats_pending = false;
         }
+        s.fetch_tol();
         s.finish_stats();
         if (cg_iterations) *cg_iterations = s.last_cg_iterations;
         if (mg_vcycles) *mg_vcycles = s.last_vcycles;
@@ -2088,6 +2202,13 @@ int sgpu_set_mg_mode(sgpu_handle* h, int mg_mode, double pressure_tolerance, int
     return guarded([&] {
         sgpu::Solver& s = *h->s;
         s.sync();
+        s.fetch_tol();
+        // a captured iteration holds the old mode, tolerance and cap
+        if (s.run_graph && (s.prm.mg_mode != mg_mode || s.prm.pressure_tolerance != pressure_tolerance ||
+                            s.prm.pressure_maxit != pressure_maxit)) {
+            sgpu::destroy_iter_graph(s.run_graph);
+            s.run_graph = nullptr;
+        }
         s.prm.mg_mode = mg_mode;
         s.prm.pressure_tolerance = pressure_tolerance;
         s.prm.pressure_maxit = pressure_maxit;
@@ -2099,7 +2220,7 @@ int sgpu_warm_start_stats(sgpu_handle* h, long long* used, long long* fallbacks,
     sgpu::Solver& s = *h->s;
     if (used) *used = s.ws_used;
     if (fallbacks) *fallbacks = s.ws_fallbacks;
-    if (rel_initial) *rel_initial = s.last_rel_initial;
+    if (rel_initial) *rel_initial = s.tol_stats ? 1.0 : s.last_rel_initial; // (a graph's solves start from zero)
     return SGPU_OK;
 }
 

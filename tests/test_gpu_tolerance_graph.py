@@ -1,0 +1,49 @@
+"""mg_mode = tolerance in Solver.run: the V-cycle loop is a conditional node of the captured iteration. It takes
+the host loop's decisions: same cycles, residuals, fields and p' as outer_iteration, bit for bit, on grids with
+and without streamed levels, with one cycle and many, at the cycle cap, from rest, and across changes of mode."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import bit_equal, config_text, cuda_available, describe_diff, snapshot_config
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")]
+
+
+def _params(sgpu_mod, nx, ny, precision, **kw):
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x=str(nx), N_cells_y=str(ny), Re="600", momentum_solver="gs_multicolour", pressure_solver="mg",
+               precision=precision, maxit="100", error_tolerance="0", mg_mode="tolerance", **kw)
+    return sgpu_mod.params_from_config(config_text(cfg))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny,kw", [(16, 16, {}), (33, 20, {}), (64, 96, {"pressure_tolerance": "1e-8"}),
+                                      (160, 320, {"pressure_tolerance": "0.5"}),
+                                      (300, 280, {"pressure_tolerance": "1e-9", "pressure_maxit": "4"})])
+def test_run_equals_host_issued_iterations(sgpu_mod, precision, nx, ny, kw):
+    p = _params(sgpu_mod, nx, ny, precision, **kw)
+    fields = (0, 1, 2, sgpu_mod.F_PC)
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for n in (1, 3, 2):  # the second and third run replay the graph
+            _, log = a.run(n)
+            rows = np.array([b.outer_iteration() for _ in range(n)])
+            assert bit_equal(np.ascontiguousarray(log[:, 1:]), rows)
+            assert a.last_solve_stats() == b.last_solve_stats()
+            for f in fields:
+                assert bit_equal(a.download(f), b.download(f)), f"field {f}: " + describe_diff(a.download(f), b.download(f))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_run_follows_changes_of_mode(sgpu_mod, precision):
+    p = _params(sgpu_mod, 96, 64, precision)
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for mode in ((False,), (True, 1e-3, 50), (True, 1e-6, 50), (True, 1e-6, 2), (False,)):
+            a.set_mg_mode(*mode)
+            b.set_mg_mode(*mode)
+            _, log = a.run(2)
+            rows = np.array([b.outer_iteration() for _ in range(2)])
+            assert bit_equal(np.ascontiguousarray(log[:, 1:]), rows)
+            for f in (0, 1, 2, sgpu_mod.F_PC):
+                assert bit_equal(a.download(f), b.download(f)), f"{mode}, field {f}"
