@@ -29,4 +29,27 @@ __device__ __forceinline__ double block_sum(double v, double* s, int tid) {
     return t;
 }
 
+// The sum of part[0 .. n) as k_sum_partials forms it (value v goes to thread v mod 1024 of 32 warps), by a
+// block of 256 threads, each standing for four of those threads: the same bits. Valid in every thread; s: 33
+// doubles of shared memory. A kernel whose blocks each need a sum of few partial sums forms it itself
+// instead of waiting for a launch that does.
+__device__ __forceinline__ double partials_sum256(const double* __restrict__ part, int n, double* s, int tid) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        double a = 0.0;
+        for (int i = tid + 256 * k; i < n; i += 1024) a += part[i];
+        a = warp_sum(a);
+        if ((tid & 31) == 0) s[8 * k + (tid >> 5)] = a;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 32; ++w) t += s[w];
+        s[32] = t;
+    }
+    __syncthreads();
+    return s[32];
+}
+
 } // namespace sgpu

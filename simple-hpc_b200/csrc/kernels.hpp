@@ -39,8 +39,22 @@ void launch_ordered_sum(const float* vals, std::size_t plane_stride, int ld, int
 // out0 = the sum of part[0 .. n), and for K = 2 also out1 = the sum of part[plane .. plane + n).
 void launch_sum_partials(const double* part, int n, int K, int plane, double* out0, double* out1,
                          cudaStream_t st);
+// Up to four such sums in one launch.
+struct SumJobs {
+    static constexpr int kMax = 4;
+    const double* part[kMax];
+    double* out[kMax];
+    int n[kMax];
+    int count = 0;
+    void add(const double* p, int m, double* o) {
+        part[count] = p;
+        n[count] = m;
+        out[count++] = o;
+    }
+};
+void launch_sum_partials(const SumJobs& jobs, cudaStream_t st);
 // *out = the sum of an nr x nc FP32 array (row stride ld) in FP64; part holds tree_sum_partials(nr,
-// nc) doubles of scratch.
+// nc) doubles of scratch, and with out null the partial sums are left there.
 int tree_sum_partials(int nr, int nc);
 void launch_tree_sum(const float* vals, int ld, int nr, int nc, double* part, double* out, cudaStream_t st);
 
@@ -58,6 +72,7 @@ void launch_assemble_v(const DevParams& p, const double* u, const double* v, Coe
                        cudaStream_t st);
 void launch_bc_u(const DevParams& p, double* u, cudaStream_t st);
 void launch_bc_v(const DevParams& p, double* v, cudaStream_t st);
+void launch_bc_uv(const DevParams& p, double* u, double* v, cudaStream_t st); // both, in one launch
 // |R| of every residual cell into cells (compact rows of the residual range).
 void launch_residual_u_cells(const DevParams& p, Coef9Ptr cu, const double* u, const double* pf,
                              double* cells, cudaStream_t st);
@@ -239,15 +254,18 @@ void launch_correct_dc(const DevParams& p, const double* pc64, const double* sum
                        const double* pc64b = nullptr, const TolState* state = nullptr);
 void launch_dc_zero_if(const TolState* state, double* pc64, std::size_t n, double* sum_pc, cudaStream_t st);
 void launch_pc_from64(const DevParams& p, const double* src, const double* sum_pc, double* dst, cudaStream_t st);
+// jobs (not null): the sums are formed inside, sum_b being the output of the last job (see kFewPartials).
 void launch_b_to_f32(const DevParams& p, const double* bfield, const double* sum_b,
-                     const LevelView32& L0, cudaStream_t st);
+                     const LevelView32& L0, const SumJobs* jobs, cudaStream_t st);
 // pc64 = FP32 p' minus its FP64 mean over the p' cells (the field correct_mixed applied).
 void launch_pc_from32(const DevParams& p, const LevelView32& L0, const double* sum_pc, double* pc64,
                       cudaStream_t st);
-// correct with the FP32 level-0 p' minus its FP64 mean (the mixed iteration's last phase).
-void launch_correct_mixed(const DevParams& p, const LevelView32& L0, const double* sum_pc,
+// correct with the FP32 level-0 p' minus its FP64 mean (the mixed iteration's last phase). part (not null):
+// *sum_pc is formed inside from nparts partial sums.
+void launch_correct_mixed(const DevParams& p, const LevelView32& L0, double* sum_pc,
                           const double* APU, const double* APV, double* u, double* v, double* pf,
-                          cudaStream_t st);
+                          cudaStream_t st,
+                          const double* part = nullptr, int nparts = 0);
 
 // ---- fused fast path (fused.cu) ----
 // Rows per CTA segment of the streaming sweeps: one wave of blocks_per_sm resident CTAs per SM, at

@@ -562,13 +562,32 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// b32 = b - mean(b), rounded to FP32 (remove_mean0, multigrid.cpp:327-345, in FP64 first).
-__global__ void k_b_to_f32(DevParams p, const double* __restrict__ bfield, const double* __restrict__ sum_b,
-                           LevelView32 L0) {
+// b32 = b - mean(b), rounded to FP32 (remove_mean0, multigrid.cpp:327-345, in FP64 first). jobs.count > 0: the
+// residual sums and the sum of b (the last job) are formed here, by block 0 and by every block.
+__global__ void __launch_bounds__(256)
+    k_b_to_f32(DevParams p, const double* __restrict__ bfield, const double* __restrict__ sum_b, LevelView32 L0,
+               SumJobs jobs) {
+    __shared__ double s_sum[33];
+    double sb = 0.0;
+    if (jobs.count > 0) {
+        const int tid = static_cast<int>(threadIdx.y * 32 + threadIdx.x);
+        const bool lead = blockIdx.x == 0 && blockIdx.y == 0;
+        if (lead)
+            for (int k = 0; k + 1 < jobs.count; ++k) {
+                const double t = partials_sum256(jobs.part[k], jobs.n[k], s_sum, tid);
+                if (tid == 0) *jobs.out[k] = t;
+                __syncthreads();
+            }
+        const int last = jobs.count - 1;
+        sb = partials_sum256(jobs.part[last], jobs.n[last], s_sum, tid);
+        if (lead && tid == 0) *jobs.out[last] = sb;
+    } else {
+        sb = *sum_b;
+    }
     const int J = static_cast<int>(blockIdx.x * 32 + threadIdx.x);
     const int I0 = static_cast<int>(blockIdx.y * kTileRows + threadIdx.y);
     if (J >= p.NY) return;
-    const double m = *sum_b / (static_cast<double>(p.NX) * p.NY);
+    const double m = sb / (static_cast<double>(p.NX) * p.NY);
 #pragma unroll
     for (int k = 0; k < kRowsPerThread; ++k) { // rows I0, I0 + 8, ...: more loads in flight per thread
         const int I = I0 + 8 * k;
@@ -584,16 +603,25 @@ __global__ void k_b_to_f32(DevParams p, const double* __restrict__ bfield, const
 // load instructions and double the bytes each one has in flight: 0.17 ms.
 __global__ void __launch_bounds__(256)
     k_correct_mixed(DevParams p, const float* __restrict__ pc32, int ld32,
-                          const double* __restrict__ sum_pc, const double* __restrict__ APU,
+                          double* __restrict__ sum_pc, const double* __restrict__ APU,
                           const double* __restrict__ APV, double* __restrict__ u, double* __restrict__ v,
-                          double* __restrict__ pf) {
+                          double* __restrict__ pf, const double* __restrict__ part, int nparts) {
+    __shared__ double s_sum[33];
+    double sp;
+    if (part) { // the mean of p' from its partial sums, by every block
+        const int tid = static_cast<int>(threadIdx.y * 32 + threadIdx.x);
+        sp = partials_sum256(part, nparts, s_sum, tid);
+        if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *sum_pc = sp;
+    } else {
+        sp = *sum_pc;
+    }
     const int H = p.H;
     const int j = pair_col0(p) + 2 * static_cast<int>(blockIdx.x * 32 + threadIdx.x);
     const int I = static_cast<int>(blockIdx.y * 8 + threadIdx.y);
     if (I >= p.NX || j > p.NY + H) return;
     const int i = H + I;
     const std::size_t q = ix(p, i, j);
-    const double m = *sum_pc / (static_cast<double>(p.NX) * p.NY);
+    const double m = sp / (static_cast<double>(p.NX) * p.NY);
     const double2 pp = *reinterpret_cast<const double2*>(pf + q);
     const double2 uu = *reinterpret_cast<const double2*>(u + q);
     const double2 au = *reinterpret_cast<const double2*>(APU + q);
@@ -921,9 +949,9 @@ int mixed_partials(const DevParams& p) {
 }
 
 void launch_b_to_f32(const DevParams& p, const double* bfield, const double* sum_b,
-                     const LevelView32& L0, cudaStream_t st) {
+                     const LevelView32& L0, const SumJobs* jobs, cudaStream_t st) {
     const dim3 grid((p.NY + 31) / 32, (p.NX + kTileRows - 1) / kTileRows);
-    k_b_to_f32<<<grid, dim3(32, 8), 0, st>>>(p, bfield, sum_b, L0);
+    k_b_to_f32<<<grid, dim3(32, 8), 0, st>>>(p, bfield, sum_b, L0, jobs ? *jobs : SumJobs{});
     SGPU_LAUNCH();
 }
 
@@ -971,11 +999,11 @@ void launch_pc_from64(const DevParams& p, const double* src, const double* sum_p
     SGPU_LAUNCH();
 }
 
-void launch_correct_mixed(const DevParams& p, const LevelView32& L0, const double* sum_pc,
+void launch_correct_mixed(const DevParams& p, const LevelView32& L0, double* sum_pc,
                           const double* APU, const double* APV, double* u, double* v, double* pf,
-                          cudaStream_t st) {
+                          cudaStream_t st, const double* part, int nparts) {
     const dim3 grid((pair_count(p) + 31) / 32, (p.NX + 7) / 8);
-    k_correct_mixed<<<grid, dim3(32, 8), 0, st>>>(p, L0.x, L0.stride, sum_pc, APU, APV, u, v, pf);
+    k_correct_mixed<<<grid, dim3(32, 8), 0, st>>>(p, L0.x, L0.stride, sum_pc, APU, APV, u, v, pf, part, nparts);
     SGPU_LAUNCH();
 }
 

@@ -95,6 +95,21 @@ __global__ void k_bc_v(DevParams p, double* v) {
     v[ix(p, i, p.NY + H + 1)] = -v[ix(p, i, p.NY + H)];
 }
 
+// Both (they touch different fields, and neither component's assembly reads the other's ghost cells).
+__global__ void k_bc_uv(DevParams p, double* u, double* v) {
+    const int H = p.H, k = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (k < p.NY) {
+        const int j = H + 1 + k;
+        u[ix(p, H - 1, j)] = 2 - u[ix(p, H, j)];
+        u[ix(p, p.NX + H, j)] = -u[ix(p, p.NX + H - 1, j)];
+    }
+    if (k < p.NX) {
+        const int i = H + k;
+        v[ix(p, i, H)] = -v[ix(p, i, H + 1)];
+        v[ix(p, i, p.NY + H + 1)] = -v[ix(p, i, p.NY + H)];
+    }
+}
+
 // residual_u (momentum_u.cpp:43-59): |R| per cell; the ordered sum runs after.
 __global__ void k_residual_u(DevParams p, Coef9Ptr cu, const double* __restrict__ u,
                              const double* __restrict__ pf, double* __restrict__ cells, Range r) {
@@ -306,6 +321,10 @@ void launch_bc_u(const DevParams& p, double* u, cudaStream_t st) {
 }
 void launch_bc_v(const DevParams& p, double* v, cudaStream_t st) {
     k_bc_v<<<(p.NX + 255) / 256, 256, 0, st>>>(p, v);
+    SGPU_LAUNCH();
+}
+void launch_bc_uv(const DevParams& p, double* u, double* v, cudaStream_t st) {
+    k_bc_uv<<<((p.NX > p.NY ? p.NX : p.NY) + 255) / 256, 256, 0, st>>>(p, u, v);
     SGPU_LAUNCH();
 }
 void launch_residual_u_cells(const DevParams& p, Coef9Ptr cu, const double* u, const double* pf,

@@ -172,17 +172,17 @@ void launch_sum(const TIn* vals, std::size_t plane_stride, int ld, int nr, int n
 
 // ---- deterministic FP64 tree sums (the mixed-precision path) ----
 
-// out_k = the sum of the n partial sums of plane k (block k): thread t adds values t, t + 1024, ...
-// in order, then the block tree.
-__global__ void __launch_bounds__(1024)
-    k_sum_partials(const double* __restrict__ part, int n, int plane, double* out0, double* out1) {
+// Block k: *jobs.out[k] = the sum of the jobs.n[k] partial sums at jobs.part[k]: thread t adds values t,
+// t + 1024, ... in order, then the block tree.
+__global__ void __launch_bounds__(1024) k_sum_partials(SumJobs jobs) {
     __shared__ double s[32];
-    const double* src = part + static_cast<std::size_t>(blockIdx.x) * plane;
+    const double* src = jobs.part[blockIdx.x];
+    const int n = jobs.n[blockIdx.x];
     double a = 0.0;
 #pragma unroll 8
     for (int i = static_cast<int>(threadIdx.x); i < n; i += 1024) a += src[i];
     const double t = block_sum<32>(a, s, static_cast<int>(threadIdx.x));
-    if (threadIdx.x == 0) *(blockIdx.x == 0 ? out0 : out1) = t;
+    if (threadIdx.x == 0) *jobs.out[blockIdx.x] = t;
 }
 
 constexpr int kTileRows = 32; // rows per block of k_tile_sum
@@ -208,11 +208,19 @@ __global__ void __launch_bounds__(256)
 
 } // namespace
 
+void launch_sum_partials(const SumJobs& jobs, cudaStream_t st) {
+    if (jobs.count < 1 || jobs.count > SumJobs::kMax) throw Error(SGPU_E_INVALID, "partial sums: 1 to 4 jobs");
+    k_sum_partials<<<jobs.count, 1024, 0, st>>>(jobs);
+    SGPU_LAUNCH();
+}
+
 void launch_sum_partials(const double* part, int n, int K, int plane, double* out0, double* out1,
                          cudaStream_t st) {
     if (K < 1 || K > 2 || (K == 2 && !out1)) throw Error(SGPU_E_INVALID, "partial sums: 1 or 2 planes");
-    k_sum_partials<<<K, 1024, 0, st>>>(part, n, plane, out0, out1);
-    SGPU_LAUNCH();
+    SumJobs jobs;
+    jobs.add(part, n, out0);
+    if (K == 2) jobs.add(part + plane, n, out1);
+    launch_sum_partials(jobs, st);
 }
 
 int tree_sum_partials(int nr, int nc) {
@@ -221,13 +229,13 @@ int tree_sum_partials(int nr, int nc) {
 
 void launch_tree_sum(const float* vals, int ld, int nr, int nc, double* part, double* out, cudaStream_t st) {
     if (nr <= 0 || nc <= 0) {
-        SGPU_CUDA(cudaMemsetAsync(out, 0, sizeof(double), st));
+        if (out) SGPU_CUDA(cudaMemsetAsync(out, 0, sizeof(double), st));
         return;
     }
     const dim3 grid((nc + 255) / 256, (nr + kTileRows - 1) / kTileRows);
     k_tile_sum<float><<<grid, 256, 0, st>>>(vals, ld, nr, nc, part);
     SGPU_LAUNCH();
-    launch_sum_partials(part, static_cast<int>(grid.x * grid.y), 1, 0, out, nullptr, st);
+    if (out) launch_sum_partials(part, static_cast<int>(grid.x * grid.y), 1, 0, out, nullptr, st);
 }
 
 void launch_ordered_sum(const double* vals, std::size_t plane_stride, int ld, int nr, int nc, int K,

@@ -281,8 +281,7 @@ struct Solver {
         double* AP = vcomp ? cv.a[8] : cu.a[8];
         // Phase attribution: the prep pass is the assembly, the ordered sum the residual.
         mark(vcomp ? SGPU_PH_BC_V : SGPU_PH_BC_U);
-        if (vcomp) launch_bc_v(dp, v, st);
-        else launch_bc_u(dp, u, st);
+        if (!vcomp) launch_bc_uv(dp, u, v, st); // both: v's ghost cells are not read before its own phase
         double* cplane = cells + (vcomp ? plane : 0);
         const bool deferred = defer_sums();
         const int n = vcomp ? prm.maxit_inner_v : prm.maxit_inner_u;
@@ -541,23 +540,29 @@ struct Solver {
     // two full-grid arrays (allocated on first use); pc_dc_src is the last iteration's final iterate.
     double* dc[2] = {nullptr, nullptr};
     const double* pc_dc_src = nullptr;
-    double* part = nullptr;           // per-block partial sums of the FP64 tree sums
+    double* part = nullptr;           // per-block partial sums of the FP64 tree sums: u, v and p' in turn
+    std::size_t part_stride = 0;
+    // A launch that only adds partial sums costs 3 us and a gap, a fifth of a 128^2 iteration in all, so where
+    // there are few (a load and a half per thread of a block) the blocks of the next kernel add them
+    // themselves: 128^2 mixed, 125.0 against 123.2 us an iteration.
+    static constexpr int kFewPartials = 640; // assemble_p's blocks, up to about 512^2
+    static constexpr int kFewTiles = 64;     // the p' tiles, up to about 700^2
     float* e32[2] = {nullptr, nullptr}; // correction ping-pong
     std::vector<LevelView32> lv32;    // FP32 multigrid hierarchy (level 0: the p' operator)
     std::vector<float*> mg32_x2;
     MgLevelsT<float> mgl32{};
 
-    void mixed_momentum(bool vcomp, double* res) {
+    // Its residual sum joins `jobs`, which one launch forms after assemble_p.
+    void mixed_momentum(bool vcomp, double* res, SumJobs& jobs) {
         double* x = vcomp ? v : u;
         const double* oth = vcomp ? u : v;
         double* AP = vcomp ? cv.a[8] : cu.a[8];
         mark(vcomp ? SGPU_PH_BC_V : SGPU_PH_BC_U);
-        if (vcomp) launch_bc_v(dp, v, st);
-        else launch_bc_u(dp, u, st);
+        if (!vcomp) launch_bc_uv(dp, u, v, st); // both: v's ghost cells are not read before its own phase
         mark(vcomp ? SGPU_PH_ASSEMBLE_V : SGPU_PH_ASSEMBLE_U);
-        const int nparts = launch_mom_prep_mixed(dp, vcomp, x, oth, pf, AP, part, rec32, st);
+        double* pp = part + (vcomp ? part_stride : 0);
+        jobs.add(pp, launch_mom_prep_mixed(dp, vcomp, x, oth, pf, AP, pp, rec32, st), res); // res_u / res_v: FP64 tree
         mark(vcomp ? SGPU_PH_RESIDUAL_V : SGPU_PH_RESIDUAL_U);
-        launch_sum_partials(part, nparts, 1, 0, res, nullptr, st); // res_u / res_v: FP64 tree
         mark(vcomp ? SGPU_PH_SWEEP_V : SGPU_PH_SWEEP_U);
         const int n = vcomp ? prm.maxit_inner_v : prm.maxit_inner_u;
         int cur = 0; // e32[cur] holds the current correction (zero before the first sweep)
@@ -578,12 +583,18 @@ struct Solver {
     void mixed_iteration_enqueue(double* res3) {
         p_links_stale = true;
         pc_stale = true;
-        mixed_momentum(false, res3 + 0);
-        mixed_momentum(true, res3 + 1);
+        SumJobs jobs;
+        mixed_momentum(false, res3 + 0, jobs);
+        mixed_momentum(true, res3 + 1, jobs);
         mark(SGPU_PH_ASSEMBLE_P);
-        const int nparts = launch_assemble_p_mixed(dp, cu.a[8], cv.a[8], u, v, w.b, lv32[0], part, st);
+        double* const part_p = part + 2 * part_stride;
+        const int nparts = launch_assemble_p_mixed(dp, cu.a[8], cv.a[8], u, v, w.b, lv32[0], part_p, st);
         // res_p = the sum of |b|, and the sum of b (its mean), from the blocks' partial sums
-        launch_sum_partials(part, nparts, 2, nparts, res3 + 2, sums + 25, st);
+        jobs.add(part_p, nparts, res3 + 2);
+        jobs.add(part_p + nparts, nparts, sums + 25);
+        const bool dc_mode = prm.mg_mode == SGPU_MG_TOLERANCE;
+        const bool few = !dc_mode && nparts <= kFewPartials; // then k_b_to_f32 forms them
+        if (!few) launch_sum_partials(jobs, st);
         mark(SGPU_PH_SOLVE_P);
         // The coarse operators are built inside the V-cycle (fused_build: by the down kernel of the
         // level above for the streamed levels, by the tail for its own), unless a warm start reads them
@@ -591,14 +602,13 @@ struct Solver {
         const bool fused_build = !net;
         if (!fused_build)
             for (std::size_t l = 1; l < lv32.size(); ++l) launch_mg_build<float>(lv32[l - 1], lv32[l], st);
-        const bool dc_mode = prm.mg_mode == SGPU_MG_TOLERANCE;
         pc_dc_src = nullptr;
         int nbb = 0;
         if (dc_mode) {
             need_dc();
             nbb = launch_dc_rhs0(dp, w.b, sums + 25, lv32[0], part, st);
         } else {
-            launch_b_to_f32(dp, w.b, sums + 25, lv32[0], st);
+            launch_b_to_f32(dp, w.b, sums + 25, lv32[0], few ? &jobs : nullptr, st);
         }
         const LevelView32& L0 = lv32[0];
         // p' starts from zero. The streaming level kernels need no cleared array for that: the
@@ -639,9 +649,11 @@ struct Solver {
             launch_correct_dc(dp, pc_dc_src, sums + 26, cu.a[8], cv.a[8], u, v, pf, st);
         } else {
             last_vcycles = run_cycles(L0, !guess, vcycle32);
-            launch_tree_sum(L0.x, L0.stride, L0.nx, L0.ny, part, sums + 26, st); // the mean of p'
+            const int np = tree_sum_partials(L0.nx, L0.ny); // the mean of p'
+            const bool inside = np <= kFewTiles;
+            launch_tree_sum(L0.x, L0.stride, L0.nx, L0.ny, part, inside ? nullptr : sums + 26, st);
             mark(SGPU_PH_CORRECT);
-            launch_correct_mixed(dp, L0, sums + 26, cu.a[8], cv.a[8], u, v, pf, st);
+            launch_correct_mixed(dp, L0, sums + 26, cu.a[8], cv.a[8], u, v, pf, st, inside ? part : nullptr, np);
         }
         mark(SGPU_PH_COUNT);
     }
@@ -1061,7 +1073,8 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
         rec32.far_links = dalloc<float4>(nrec) + kRecFrontCols;
         rec32.diag = dalloc<float2>(nrec) + kRecFrontCols;
         corr_err = dalloc<unsigned>(1);
-        part = dalloc<double>(static_cast<std::size_t>(std::max(mixed_partials(dp), tree_sum_partials(p.NX, p.NY))));
+        part_stride = static_cast<std::size_t>(std::max(mixed_partials(dp), tree_sum_partials(p.NX, p.NY)));
+        part = dalloc<double>(3 * part_stride);
         e32[0] = dalloc<float>(g.elems());
         e32[1] = dalloc<float>(g.elems());
         const int nl = static_cast<int>(lv.size());
