@@ -138,7 +138,14 @@ struct Solver {
     // Minimum rows per CTA segment of the streaming kernels. A single solve owns the GPU and is
     // bound by each CTA's per-step latency on small grids, so it takes short segments (8 rows); a
     // batch fills the GPU with many cavities and keeps the kernels' defaults (0), which bound the
-    // halo and skew work per row (use_batch_shape).
+    // halo and skew work per row (use_batch_shape). A batch that does not fill the GPU is bound by the
+    // latency of its largest cavities, so while the batch has at most kBatchCells cells in all its
+    // kBatchLatency largest keep a single solve's shape (as many as the GPU holds 16-CTA tail clusters at
+    // once). Measured, us a round with the batch shape for all and with 8 excepted: 20 cavities of 64^2 to
+    // 512^2 (0.8 M cells) 612 and 441, four of 512^2 (1.05 M) 614 and 446, eight of 384^2 (1.2 M) 624 and 498,
+    // eight of 512^2 (2.1 M) 743 and 796, sixteen 1074 and 1404.
+    static constexpr int kBatchLatency = 8;
+    static constexpr std::size_t kBatchCells = 1200000;
     int min_seg = 8;
     void use_batch_shape() {
         min_seg = 0;
@@ -542,11 +549,11 @@ struct Solver {
     const double* pc_dc_src = nullptr;
     double* part = nullptr;           // per-block partial sums of the FP64 tree sums: u, v and p' in turn
     std::size_t part_stride = 0;
-    // A launch that only adds partial sums costs 3 us and a gap, a fifth of a 128^2 iteration in all, so where
-    // there are few (a load and a half per thread of a block) the blocks of the next kernel add them
-    // themselves: 128^2 mixed, 125.0 against 123.2 us an iteration.
-    static constexpr int kFewPartials = 640; // assemble_p's blocks, up to about 512^2
-    static constexpr int kFewTiles = 64;     // the p' tiles, up to about 700^2
+    // A launch that only adds partial sums costs 3 us and a gap, so where there are few the blocks of the next
+    // kernel add them themselves: 128^2 mixed, 125.0 against 123.2 us an iteration. From 512^2 on that costs
+    // more SM time than the launch (32 such cavities in a batch: 1.95 against 1.97 ms a round).
+    static constexpr int kFewPartials = 160; // assemble_p's blocks, up to 256^2
+    static constexpr int kFewTiles = 8;      // the p' tiles, up to 256^2
     float* e32[2] = {nullptr, nullptr}; // correction ping-pong
     std::vector<LevelView32> lv32;    // FP32 multigrid hierarchy (level 0: the p' operator)
     std::vector<float*> mg32_x2;
@@ -2280,8 +2287,16 @@ int sgpu_batch_create(const sgpu_params_t* params, int count, sgpu_batch** out) 
             if (p.warm_start)
                 throw sgpu::Error(SGPU_E_INVALID, who + "warm_start = cnn is not supported in a batch");
             b->s.push_back(std::make_unique<sgpu::Solver>(p, nullptr, nullptr, nullptr));
-            b->s.back()->use_batch_shape();
         }
+        std::vector<sgpu::Solver*> by_size;
+        for (auto& sv : b->s) by_size.push_back(sv.get());
+        std::stable_sort(by_size.begin(), by_size.end(), [](const sgpu::Solver* x, const sgpu::Solver* y) {
+            return x->plane > y->plane;
+        });
+        std::size_t cells = 0;
+        for (const sgpu::Solver* sv : by_size) cells += sv->plane;
+        const std::size_t first = cells <= sgpu::Solver::kBatchCells ? sgpu::Solver::kBatchLatency : 0;
+        for (std::size_t c = first; c < by_size.size(); ++c) by_size[c]->use_batch_shape();
         SGPU_CUDA(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking));
         b->seg_tuned.assign(count, 0);
         for (auto& sv : b->s) sv->sync();
