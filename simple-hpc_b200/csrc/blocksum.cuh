@@ -1,4 +1,5 @@
-// blocksum.cuh — deterministic block sums in FP64 (the mixed-precision path's residual sums).
+// blocksum.cuh — deterministic block sums in FP64 (the mixed-precision path's residual sums), and the serial
+// chain of the ordered ones.
 //
 // A fixed xor-shuffle tree inside each warp, then thread 0 adds the warps' sums in warp order. At
 // each tree step lane i forms v_i + v_(i^o) and its partner v_(i^o) + v_i, the same bits, so every
@@ -50,6 +51,38 @@ __device__ __forceinline__ double partials_sum256(const double* __restrict__ par
     }
     __syncthreads();
     return s[32];
+}
+
+// The serial sum of v[0 .. n) (ABS: of |v|) continued from a, the reference's order within a row; v is
+// 16-byte aligned shared memory. 16 values are loaded, two at a time, while 16 are added.
+template <bool ABS = false> __device__ __forceinline__ double ordered_chain(double a, const double* v, int n) {
+    double x[16], y[16];
+    auto load = [](double (&to)[16], const double* from) {
+#pragma unroll
+        for (int u = 0; u < 16; u += 2) {
+            const double2 d = *reinterpret_cast<const double2*>(from + u);
+            to[u] = d.x;
+            to[u + 1] = d.y;
+        }
+    };
+    auto add = [&](const double (&from)[16]) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) a += ABS ? fabs(from[u]) : from[u];
+    };
+    int t = 0;
+    if (n >= 16) {
+        load(x, v);
+        for (; t + 48 <= n; t += 32) {
+            load(y, v + t + 16);
+            add(x);
+            load(x, v + t + 32);
+            add(y);
+        }
+        add(x);
+        t += 16;
+    }
+    for (; t < n; ++t) a += ABS ? fabs(v[t]) : v[t];
+    return a;
 }
 
 } // namespace sgpu

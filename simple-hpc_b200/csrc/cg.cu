@@ -8,6 +8,7 @@
 // Grids whose rows fit the shared memory of one CTA per SM run the whole solve in one cooperative kernel
 // instead (k_cg_persist); the pass-by-pass kernels take the others.
 #include "kernels.hpp"
+#include "blocksum.cuh"
 
 #include <algorithm>
 
@@ -191,38 +192,6 @@ __global__ void k_cg_empty(unsigned long long* sums, int n) {
         sums[k] = kCgEmpty;
 }
 
-// The ordered sum of v[0 .. n) continued from a (v 16-byte aligned): 16 values are loaded, two at a time,
-// while 16 are added.
-__device__ __forceinline__ double chain(double a, const double* v, int n) {
-    double x[16], y[16];
-    auto load = [](double (&to)[16], const double* from) {
-#pragma unroll
-        for (int u = 0; u < 16; u += 2) {
-            const double2 d = *reinterpret_cast<const double2*>(from + u);
-            to[u] = d.x;
-            to[u + 1] = d.y;
-        }
-    };
-    auto add = [&](const double (&from)[16]) {
-#pragma unroll
-        for (int u = 0; u < 16; ++u) a += from[u];
-    };
-    int t = 0;
-    if (n >= 16) {
-        load(x, v);
-        for (; t + 48 <= n; t += 32) {
-            load(y, v + t + 16);
-            add(x);
-            load(x, v + t + 32);
-            add(y);
-        }
-        add(x);
-        t += 16;
-    }
-    for (; t < n; ++t) a += v[t];
-    return a;
-}
-
 __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void named_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory"); }
 
@@ -300,7 +269,7 @@ __global__ void __launch_bounds__(kCgWork + 128)
                 const int b = c % kCgBufs;
                 __syncwarp();
                 named_sync(1 + b, nt);
-                if (on) a = chain(a, stage + (b * 4 * R + k * R + r) * sld, min(cc, nc - c * cc));
+                if (on) a = ordered_chain(a, stage + (b * 4 * R + k * R + r) * sld, min(cc, nc - c * cc));
                 __syncwarp();
                 if (c + kCgBufs < nch) named_arrive(4 + b, nt);
             }
@@ -346,7 +315,7 @@ __global__ void __launch_bounds__(kCgWork + 128)
         __syncthreads();
         if (stop) return false;
         if (work) beside();
-        else if (tid - kCgWork < K) tot[tid - kCgWork] = chain(0.0, fin + (tid - kCgWork) * nrp, nr);
+        else if (tid - kCgWork < K) tot[tid - kCgWork] = ordered_chain(0.0, fin + (tid - kCgWork) * nrp, nr);
         __syncthreads();
         return true;
     };

@@ -29,9 +29,6 @@ void launch_ordered_sum_lean(const double* vals, int ld, int nr, int nc, double*
 // (res_p and the mean of b from the field b itself, without compact copies).
 void launch_ordered_sum_abs_pair(const double* vals, int ld, int nr, int nc, double* out, const SumScratch& s,
                                  cudaStream_t st);
-// The same order over FP32 values, each widened to double before it is added.
-void launch_ordered_sum(const float* vals, std::size_t plane_stride, int ld, int nr, int nc, int K,
-                        double* out, const SumScratch& s, const int* skip, cudaStream_t st);
 
 // Deterministic FP64 tree sums (the mixed-precision path, which is not tied to the reference's
 // rounding): a fixed shuffle tree per block, the blocks' partial sums added by one CTA in a fixed
