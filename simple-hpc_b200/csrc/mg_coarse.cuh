@@ -109,9 +109,13 @@ template <class T> struct CoarseCell {
 };
 
 // The update value of a cell from its neighbour sum. Double: b / AP (t0, formed once) + nb / AP, the
-// two statements of multigrid.cpp:61-63; float: as rb_value.
-__device__ __forceinline__ double coarse_value(double t0, double, double nb, double ap) { return div_sum(t0, nb, ap); }
-__device__ __forceinline__ float coarse_value(float, float b, float nb, float ap) { return rb_value(b, nb, ap); }
+// two statements of multigrid.cpp:61-63, y = inverse(AP); float: as rb_value.
+__device__ __forceinline__ double coarse_value(double t0, double, double nb, double ap, double y) {
+    return t0 + quotient(nb, ap, y);
+}
+__device__ __forceinline__ float coarse_value(float, float b, float nb, float ap, float) { return rb_value(b, nb, ap); }
+__device__ __forceinline__ double coarse_inverse(double ap) { return inverse(ap); }
+__device__ __forceinline__ float coarse_inverse(float) { return 0.0f; }
 __device__ __forceinline__ double coarse_t0(double b, double ap) { return b / ap; }
 __device__ __forceinline__ float coarse_t0(float, float) { return 0.0f; }
 
@@ -172,6 +176,7 @@ __device__ void coarse_solve(const Team& tm, int nx, int ny, int i0, int m, int 
         // rounding of the squares, the sum and the root; the float one that of the bound too)
         const T big = static_cast<T>(thr * (sizeof(T) == 8 ? 1.0 + 1e-9 : 1.0 + 1e-6));
         const T t0[2] = {coarse_t0(c[0].b, c[0].ap), coarse_t0(c[1].b, c[1].ap)};
+        const T y[2] = {coarse_inverse(c[0].ap), coarse_inverse(c[1].ap)};
         // This thread's cells are element o of each colour's array; the neighbours are o + odd (east),
         // o + odd - 1 (west), o + xstride (south) and o - xstride (north) of the other colour's.
         const int xs = sm.xstride, cs = static_cast<int>(sm.x[1] - sm.x[0]);
@@ -199,7 +204,7 @@ __device__ void coarse_solve(const Team& tm, int nx, int ny, int i0, int m, int 
         T f0 = flow(0), r0 = T(0), r1 = T(0);
         while (true) {
             // colour 0 of sweep sweeps + 1, and the test of sweep `sweeps`
-            const T v0 = coarse_value(t0[0], c[0].b, f0, c[0].ap);
+            const T v0 = coarse_value(t0[0], c[0].b, f0, c[0].ap, y[0]);
             put(0, v0);
             const bool above = (ok[0] && !(fabs(r0) < big)) || (ok[1] && !(fabs(r1) < big));
             if (!tm.vote(sweeps == 0 || above, sweeps, sm.bcast)) {
@@ -207,7 +212,7 @@ __device__ void coarse_solve(const Team& tm, int nx, int ny, int i0, int m, int 
             }
             c[0].x = v0;
             const T f1 = flow(1);
-            c[1].x = coarse_value(t0[1], c[1].b, f1, c[1].ap);
+            c[1].x = coarse_value(t0[1], c[1].b, f1, c[1].ap, y[1]);
             put(1, c[1].x);
             tm.sync();
             if (++sweeps == kCoarseSweeps) break;
