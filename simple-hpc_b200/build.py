@@ -40,6 +40,7 @@ SOURCES = {
     "cg.cu": EXACT,
     "fused.cu": EXACT,
     "mg_fast.cu": EXACT,
+    "mg_sweep.cu": EXACT,
     "mixed.cu": EXACT,
     "io.cpp": EXACT,
     "noalloc.cu": EXACT,

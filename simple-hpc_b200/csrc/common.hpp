@@ -145,19 +145,25 @@ __device__ __forceinline__ double inverse(double ap) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(ap)); // the sign bit fails the test too
     return (hi >> 20) - 923u <= 200u ? 1.0 / ap : 0.0;             // 2^-100 <= AP < 2^101
 }
-__device__ __forceinline__ double quotient(double a, double ap, double y) {
+// The quotient, or slow set where it takes a division.
+__device__ __forceinline__ double quotient_try(double a, double ap, double y, bool& slow) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(a));
     const bool zero = ((hi << 1) | static_cast<unsigned>(__double2loint(a))) == 0u;
     const bool mid = ((hi >> 20) & 0x7ffu) - 123u <= 1800u; // 2^-900 <= |a| < 2^901
     double q = a * y;
     q = __fma_rn(__fma_rn(-ap, q, a), y, q);
     q = __fma_rn(__fma_rn(-ap, q, a), y, q);
-    if (zero) q = a; // AP > 0 keeps the sign
-    if (!(mid || zero) || __double2hiint(y) == 0) {
-        double n = a;
-        asm volatile("" : "+d"(n)); // the division stays inside the branch
-        q = n / ap;
-    }
+    slow |= !(mid || zero) || __double2hiint(y) == 0;
+    return zero ? a : q; // AP > 0 keeps a zero's sign
+}
+__device__ __forceinline__ double divided(double a, double ap) {
+    asm volatile("" : "+d"(a)); // the division stays inside the caller's branch
+    return a / ap;
+}
+__device__ __forceinline__ double quotient(double a, double ap, double y) {
+    bool slow = false;
+    double q = quotient_try(a, ap, y, slow);
+    if (slow) q = divided(a, ap);
     return q;
 }
 __device__ __forceinline__ float rb_value(float b, float nb, float ap) {

@@ -156,6 +156,17 @@ template <class T>
 void launch_mg_up(const LevelViewT<T>& C, const LevelViewT<T>& F, const T* xin, T* xout,
                   double omega, int post, int sms, int min_seg, cudaStream_t st);
 
+// Two red-black sweeps of a double level whose operator is symmetric and whose AP is the sum of its links
+// (the operators of assemble_p and mg_build), from AE, AN and b alone (mg_sweep.cu): as launch_mg_down and
+// launch_mg_up with two sweeps, and the sweeps by themselves on a level whose zero ring is implied
+// (parity 1: the cells with I + J odd are the first colour).
+void launch_sweeps_down(const LevelView& F, const LevelView& C, double* xout, bool x_zero, int sms, int min_seg,
+                        cudaStream_t st, bool build);
+void launch_sweeps_up(const LevelView& C, const LevelView& F, const double* xin, double* xout, double omega, int sms,
+                      int min_seg, cudaStream_t st);
+void launch_sweeps_plain(const LevelView& L, const double* xin, double* xout, bool x_zero, int parity, int sms,
+                         int min_seg, cudaStream_t st);
+
 // ---- conjugate gradient (cg.cu) ----
 struct CgScalars {
     double rz, nb, mz, alpha, beta, rel, mb;

@@ -280,6 +280,9 @@ struct Solver {
     // Set while the fast iteration's pressure solve runs: the ordered sum of b, formed by the |b| / b
     // pair sum in the same order, for the multigrid's mean removal of b.
     const double* b_sum = nullptr;
+    // Set with it: the p' links are the ones this iteration assembled (between per-phase calls a caller may
+    // upload any), so the double levels are symmetric and mg_sweep.cu's kernels apply.
+    bool own_links = false;
 
     // One momentum phase on the fused path: bc, residual + AP + frozen copy, n streaming sweeps.
     void fast_momentum(bool vcomp, double* res) {
@@ -435,7 +438,9 @@ struct Solver {
         launch_ordered_sum_abs_pair(w.b + p_origin(), g.pitch, prm.NX, prm.NY, res3 + 2, ss, st);
         mark(SGPU_PH_SOLVE_P);
         b_sum = res3 + 3; // the multigrid's mean of b reuses the pair's sum of b
+        own_links = true;
         solve_p();
+        own_links = false;
         b_sum = nullptr;
         mark(SGPU_PH_CORRECT);
         correct();
@@ -1178,7 +1183,17 @@ void Solver::sweep_v(int n) {
 // solve_pc_redblack (pressure.cpp:114-134).
 void Solver::solve_redblack() {
     SGPU_CUDA(cudaMemsetAsync(w.pc, 0, g.bytes(), st));
-    for (int k = 0; k < prm.maxit_inner_p; ++k)
+    int k = 0;
+    if (own_links) { // two sweeps per pass, to the other of pc and tmp each time and to pc at last
+        const std::size_t o = p_origin();
+        LevelView L{prm.NX, prm.NY, g.pitch, w.AEP + o, nullptr, w.ANP + o, nullptr, nullptr, w.b + o, nullptr, nullptr};
+        const int passes = prm.maxit_inner_p / 2;
+        for (int n = passes; n > 0; --n, k += 2) {
+            double* const out = (n & 1 ? w.pc : tmp) + o;
+            launch_sweeps_plain(L, (n & 1 ? tmp : w.pc) + o, out, n == passes, 1, sms, min_seg, st);
+        }
+    }
+    for (; k < prm.maxit_inner_p; ++k)
         for (int c = 0; c < 2; ++c) launch_pc_redblack(dp, w, c, st);
 }
 
@@ -1321,14 +1336,20 @@ template <class T> void Solver::sample_pair(std::vector<LevelViewT<T>>& L, float
 // mg_vcycle with the streaming level kernels: levels [0, mg_tail64) go down and up in one pass each, the
 // rest (and the coarse solve) in a tail kernel.
 void Solver::mg_vcycle_fast(bool x_is_zero, bool build) {
-    for (int l = 0; l < mg_tail64; ++l)
-        launch_mg_down(lv[l], lv[l + 1], mg_x2[l], prm.mg_pre, x_is_zero || l > 0, sms, min_seg, st, build);
+    for (int l = 0; l < mg_tail64; ++l) {
+        const bool zero = x_is_zero || l > 0;
+        if (own_links && prm.mg_pre == 2) launch_sweeps_down(lv[l], lv[l + 1], mg_x2[l], zero, sms, min_seg, st, build);
+        else launch_mg_down(lv[l], lv[l + 1], mg_x2[l], prm.mg_pre, zero, sms, min_seg, st, build);
+    }
     if (mg_tail64 == mg_tail || !launch_mg_tail_cluster(mgl, mg_tail64, prm.mg_pre, prm.mg_post, prm.mg_omega,
                                                         kCoarseTol64, stats, st, build))
         launch_mg_tail(mgl, mg_tail64, prm.mg_pre, prm.mg_post, prm.mg_omega, kCoarseTol64, coarse_rowbuf,
                        stats, st, build);
-    for (int l = mg_tail64 - 1; l >= 0; --l)
-        launch_mg_up(lv[l + 1], lv[l], mg_x2[l], lv[l].x, prm.mg_omega, prm.mg_post, sms, min_seg, st);
+    for (int l = mg_tail64 - 1; l >= 0; --l) {
+        if (own_links && prm.mg_post == 2)
+            launch_sweeps_up(lv[l + 1], lv[l], mg_x2[l], lv[l].x, prm.mg_omega, sms, min_seg, st);
+        else launch_mg_up(lv[l + 1], lv[l], mg_x2[l], lv[l].x, prm.mg_omega, prm.mg_post, sms, min_seg, st);
+    }
 }
 
 void Solver::solve_p() {
