@@ -16,7 +16,9 @@
 //    common.hpp), which a cell's first sweep forms and passes to its second in registers, and a step reads
 //    all it needs before it stores (its cells' neighbours lie on rows and columns that no thread updates in
 //    the same step), so the two sweeps' chains overlap.
-// Measured: FIGURES
+// Measured, the streamed levels of a V(2,2) cycle at 4096^2: descent 670 -> 460 us, ascent 540 -> 395 us; 8 sweeps
+// of the red-black solver at 1531 x 2047: 470 us (16 launches, a colour each) -> 192 us. It is now bound by
+// issue slots and shared-memory wavefronts (60% of each; DRAM 25%).
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -26,13 +28,17 @@ namespace sgpu {
 namespace {
 
 constexpr int kNT = 128;        // threads: loaded columns of a strip
-constexpr int kCtas = 3;        // per SM: the four rings take 65 KB
-constexpr int kRing = 16;       // rows of each ring
+constexpr int kRing = 16;       // rows of the x ring
 constexpr int kHalo = 6;        // of a strip: one cell per colour pass, one for the residual, kept even
 constexpr int kLag = 8;         // rows between a step and the row whose two sweeps it completes
-constexpr int kSmem = (4 * kRing * kNT + 2) * 8; // and a pad: the first column's west neighbour
 
 enum Job { kDown, kUp, kPlain };
+// Rows of the rings of AE, AN and b: without a residual they are last read two rows behind the step. With
+// them at 8 rows four CTAs fit an SM (41 KB each), otherwise three (65 KB).
+__host__ __device__ constexpr int coef_ring(Job j) { return j == kDown ? 16 : 8; }
+__host__ __device__ constexpr int ctas(Job j) { return j == kDown ? 3 : 4; }
+// and a pad: the first column's west neighbour
+__host__ __device__ constexpr int smem_bytes(Job j) { return ((kRing + 3 * coef_ring(j)) * kNT + 2) * 8; }
 
 __device__ __forceinline__ void cp_async(double* smem, const double* gmem) {
     const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -50,16 +56,16 @@ struct Swept {
 
 // parity: 0 where the first colour is the cells with I + J even, 1 where it is the others.
 template <Job JOB>
-__global__ void __launch_bounds__(kNT, kCtas)
+__global__ void __launch_bounds__(kNT, ctas(JOB))
     k_level_sweeps(LevelView L, LevelView C, const double* __restrict__ xin, double* __restrict__ xout,
                    double omega, int x_zero, int parity, int seg_rows, int build) {
     // Rows copied beyond the ones a step reads: a step refills the slot of a row last read before it.
-    constexpr int LA = JOB == kUp ? 2 : 1, PF = JOB == kDown ? 4 : 5;
+    constexpr int LA = JOB == kUp ? 2 : 1, RC = coef_ring(JOB), PF = JOB == kDown ? 4 : JOB == kUp ? 2 : 3;
     extern __shared__ __align__(16) double sm[];
     double* const X = sm + 2;
     double* const AE = X + kRing * kNT;
-    double* const AN = AE + kRing * kNT;
-    double* const B = AN + kRing * kNT;
+    double* const AN = AE + RC * kNT;
+    double* const B = AN + RC * kNT;
     const int tid = threadIdx.x, nx = L.nx, ny = L.ny, ls = L.stride;
     constexpr int W = kNT - 2 * kHalo;
     const int R0 = blockIdx.y * seg_rows, R1 = min(R0 + seg_rows, nx);            // owned rows
@@ -77,22 +83,23 @@ __global__ void __launch_bounds__(kNT, kCtas)
         return ((cols >> k) & 1u) && I >= lo + (cut_top ? k : 0) && I <= hi - (cut_bot ? k : 0);
     };
     auto at = [&](int I) { return (I & (kRing - 1)) * kNT + tid; };
+    auto cat = [&](int I) { return (I & (RC - 1)) * kNT + tid; };
 
     int next = L0;
     auto issue = [&]() {
         if (next < L1 && cload) {
-            const int q = at(next);
+            const int q = at(next), k = cat(next);
             const bool in = cint && next >= 0 && next < nx;
             const long long c = static_cast<long long>(next) * ls + Jc;
             if (x_zero || (JOB == kPlain && !in)) X[q] = 0.0;
             else cp_async(X + q, xin + c);
             if (in) {
-                cp_async(AE + q, L.AE + c);
-                cp_async(AN + q, L.AN + c);
-                cp_async(B + q, L.b + c);
+                cp_async(AE + k, L.AE + c);
+                cp_async(AN + k, L.AN + c);
+                cp_async(B + k, L.b + c);
             } else { // the west and south links of the cells along the walls
-                AE[q] = 0.0;
-                AN[q] = 0.0;
+                AE[k] = 0.0;
+                AN[k] = 0.0;
             }
         }
         cp_async_commit();
@@ -128,11 +135,12 @@ __global__ void __launch_bounds__(kNT, kCtas)
         const int q0 = at(I0), q0n = at(I0 - 1), q0s = at(I0 + 1);
         const int q1 = at(I1), q1n = at(I1 - 1), q1s = at(I1 + 1);
         Swept z;
-        z.e = AE[q0];
-        z.w = AE[q0 - 1];
-        z.n = AN[q0];
-        z.s = AN[q0s];
-        const double b0 = B[q0];
+        const int k0 = cat(I0);
+        z.e = AE[k0];
+        z.w = AE[k0 - 1];
+        z.n = AN[k0];
+        z.s = AN[cat(I0 + 1)];
+        const double b0 = B[k0];
         const double nb0 = z.e * X[q0 + 1] + z.w * X[q0 - 1] + z.s * X[q0s] + z.n * X[q0n];
         const double nb1 = sw.e * X[q1 + 1] + sw.w * X[q1 - 1] + sw.s * X[q1s] + sw.n * X[q1n];
         z.ap = ok0 ? z.e + z.w + z.n + z.s : 1.0;
@@ -208,16 +216,16 @@ void launch(const LevelView& L, const LevelView& C, const double* xin, double* x
     auto kernel = k_level_sweeps<JOB>;
     static PerDeviceOnce once;
     const int blocks = once.get([&] {
-        SGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        SGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(JOB)));
         int n = 0;
-        SGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kNT, kSmem));
+        SGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kNT, smem_bytes(JOB)));
         return n < 1 ? 1 : n;
     });
     constexpr int W = kNT - 2 * kHalo;
     const int strips = (L.ny + W - 1) / W, want = std::max(1, blocks * sms / strips);
     int seg = ((L.nx + want - 1) / want + 1) & ~1;
     seg = std::max(seg, min_seg > 0 ? std::max(2, min_seg & ~1) : 2 * kHalo + 8);
-    kernel<<<dim3(strips, (L.nx + seg - 1) / seg), kNT, kSmem, st>>>(L, C, xin, xout, omega, x_zero ? 1 : 0, parity, seg,
+    kernel<<<dim3(strips, (L.nx + seg - 1) / seg), kNT, smem_bytes(JOB), st>>>(L, C, xin, xout, omega, x_zero ? 1 : 0, parity, seg,
                                                                    build ? 1 : 0);
     SGPU_LAUNCH();
 }
