@@ -20,6 +20,7 @@
 // Pressure assembly (assemble_p, pressure.cpp:14-54) is one kernel with the wall zeros folded in.
 #include "kernels.hpp"
 #include "bulk.cuh"
+#include "prep_walk.cuh"
 #include "stencil.cuh"
 
 #include <cooperative_groups.h>
@@ -415,65 +416,38 @@ __global__ void __launch_bounds__(NT, PF == 0 ? 2 : 3)
 // The recomputing sweep is bound by instruction issue (about 400 a cell, half of the slots busy, DRAM at
 // 17%), and its CTAs' halo and skew rows cost as much as their own. Records cost 72 B/cell once per
 // component and 56 B/cell more per sweep, but a third of the instructions, and up to about 1024^2 they
-// stay in L2. Measured, prep and four sweeps of one component: 178 us at 1024^2 and 1570 us at 4096^2,
-// against 206 and 1810 us (a sweep: 37 and 262 us against 47 and 390; the prep, bound by the latency of
-// its loads, 31 and 520 us against 18 and 260).
+// stay in L2. Measured, prep and four sweeps of one component: 175 us at 1024^2 and 1400 us at 4096^2,
+// against 206 and 1810 us (a sweep: 37 and 262 us against 47 and 390; the prep
+// 27 and 350 us against 18 and 260).
 
-constexpr int kRecTileRows = 16; // rows of a prep block's tile: 40 KB of records in shared memory
-
-// Prep over the update range: |R|, AP and the records. A block of 32 x 8 threads stages the records of a
-// tile of 32 columns x kRecTileRows rows in shared memory and then writes whole step rows (the cells of
-// one step row lie on up to five field rows; a step row shared with the neighbouring tile is written in
-// part by each). At 4096^2: 0.52 ms; a tile of 16 x 32 0.55, 80 registers and three CTAs an SM 0.55, 48 and
-// five 0.58.
+// Prep over the update range: |R|, AP and the records (prep_walk.cuh), 350 us at 4096^2
+// and 27 at 1024^2; from tiles assembled in global memory 505 and 31. It is bound by memory now (120 B a cell:
+// 307 us).
 template <int NCOL, bool V>
 __global__ void __launch_bounds__(256, 4)
     k_mom_prep_rec(DevParams p, const double* __restrict__ x, const double* __restrict__ oth,
                    const double* __restrict__ pf, double* __restrict__ AP, double* __restrict__ cells, MomRec64 rec,
-                   Range ur) {
-    constexpr int NK = NCOL == 5 ? 5 : 3;
-    __shared__ double2 s[NK][kRecTileRows][32];
-    const int lane = static_cast<int>(threadIdx.x), wy = static_cast<int>(threadIdx.y);
-    const int j = ur.j0 + static_cast<int>(blockIdx.x) * 32 + lane;
-    const int ib = ur.i0 + static_cast<int>(blockIdx.y) * kRecTileRows;
-    if (j <= ur.j1) {
-#pragma unroll 1
-        for (int ti = wy; ti < kRecTileRows; ti += 8) {
-            const int i = ib + ti;
-            if (i > ur.i1) break;
-            const std::size_t q = ix(p, i, j), ld = p.pitch;
-            const Coef9 c = V ? coef_v(p, oth, x, i, j) : coef_u(p, x, oth, i, j);
-            const double nb = (c.AE * x[q + 1] + c.AW * x[q - 1] + c.AN * x[q - ld] + c.AS * x[q + ld]) +
-                              (c.AEE * x[q + 2] + c.AWW * x[q - 2] + c.ANN * x[q - 2 * ld] + c.ASS * x[q + 2 * ld]);
-            const double pt = V ? (pf[q] - pf[q - ld]) * p.dx : (pf[q] - pf[q + 1]) * p.dy;
-            cells[static_cast<std::size_t>(i - ur.i0) * ur.cols() + (j - ur.j0)] = fabs(nb + pt - c.AP * x[q]);
-            AP[q] = c.AP;
-            s[0][ti][lane] = make_double2(c.AE, c.AW);
-            s[1][ti][lane] = make_double2(c.AN, c.AS);
+                   Range ur, int rows) {
+    extern __shared__ __align__(16) unsigned char prep_sm[];
+    PrepWalk<V, double2>& walk = *reinterpret_cast<PrepWalk<V, double2>*>(prep_sm);
+    const int R0 = ur.i0 + static_cast<int>(blockIdx.y) * rows, R1 = min(R0 + rows, ur.i1 + 1);
+    walk.template run<NCOL>(
+        p, x, oth, pf, ur, prep_first(ur) + static_cast<int>(blockIdx.x) * 32, R0, R1,
+        [&](int st, int, int j, const Coef9& c, double nb, double pt, double own) {
+            const std::size_t q = static_cast<std::size_t>(st) * p.pitch + j;
+            rec.r[0][q] = make_double2(c.AE, c.AW);
+            rec.r[1][q] = make_double2(c.AN, c.AS);
             if (NCOL == 5) {
-                s[2][ti][lane] = make_double2(c.AEE, c.AWW);
-                s[NK - 2][ti][lane] = make_double2(c.ANN, c.ASS);
+                rec.r[2][q] = make_double2(c.AEE, c.AWW);
+                rec.r[3][q] = make_double2(c.ANN, c.ASS);
             }
-            s[NK - 1][ti][lane] = make_double2(c.AP, pt);
-        }
-    }
-    __syncthreads();
-    if (j > ur.j1) return;
-    const int nsteps = kRecTileRows + 2 * (NCOL - 1);
-    for (int k = wy; k < nsteps; k += 8) {
-        const int st = ib + k;
-        const int c = NCOL == 5 ? (2 * st + j) % 5 : (st + j) & 1; // the colour of step st in column j
-        const int ti = k - 2 * c;
-        if (ti < 0 || ti >= kRecTileRows || ib + ti > ur.i1) continue;
-        const std::size_t q = static_cast<std::size_t>(st) * p.pitch + j;
-        rec.r[0][q] = s[0][ti][lane];
-        rec.r[1][q] = s[1][ti][lane];
-        if (NCOL == 5) {
-            rec.r[2][q] = s[2][ti][lane];
-            rec.r[3][q] = s[NK - 2][ti][lane];
-        }
-        rec.r[4][q] = s[NK - 1][ti][lane];
-    }
+            rec.r[4][q] = make_double2(c.AP, pt);
+            return make_double2(c.AP, fabs(nb + pt - c.AP * own));
+        },
+        [&](int i, int j, const double2& v) {
+            AP[ix(p, i, j)] = v.x;
+            cells[static_cast<std::size_t>(i - ur.i0) * ur.cols() + (j - ur.j0)] = v.y;
+        });
 }
 
 // Threads of the record sweep's CTAs, and the resident CTAs its registers are bounded for: the x ring and
@@ -1019,21 +993,31 @@ void launch_mom_sweep(const DevParams& p, bool v_component, const double* xin, d
     else launch_stream_v<false, kStreamPF>(p, xin, xout, xF, oth, pf, seg_rows, st);
 }
 
+namespace {
+template <int NCOL, bool V>
+void launch_prep_rec(const DevParams& p, const double* x, const double* oth, const double* pf, double* AP, double* cells,
+                     MomRec64 rec, const Range& ur, cudaStream_t st) {
+    constexpr int smem = sizeof(PrepWalk<V, double2>);
+    static PerDeviceOnce once;
+    const int rows = prep_rows(ur, prep_resident(k_mom_prep_rec<NCOL, V>, smem, once));
+    const dim3 grid(prep_strips(ur), (ur.rows() + rows - 1) / rows);
+    k_mom_prep_rec<NCOL, V><<<grid, dim3(32, kPrepSteps), smem, st>>>(p, x, oth, pf, AP, cells, rec, ur, rows);
+    SGPU_LAUNCH();
+}
+} // namespace
 void launch_mom_prep_rec(const DevParams& p, bool v_component, const double* x, const double* oth, const double* pf,
                          double* AP, double* cells, MomRec64 rec, cudaStream_t st) {
     Range ur, cr;
     if (v_component) prep_ranges<true>(p, ur, cr);
     else prep_ranges<false>(p, ur, cr);
     if (ur.rows() <= 0 || ur.cols() <= 0) return;
-    const dim3 grid((ur.cols() + 31) / 32, (ur.rows() + kRecTileRows - 1) / kRecTileRows), block(32, 8);
     if (p.ncol == 5) {
-        if (v_component) k_mom_prep_rec<5, true><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
-        else k_mom_prep_rec<5, false><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
+        if (v_component) launch_prep_rec<5, true>(p, x, oth, pf, AP, cells, rec, ur, st);
+        else launch_prep_rec<5, false>(p, x, oth, pf, AP, cells, rec, ur, st);
     } else {
-        if (v_component) k_mom_prep_rec<2, true><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
-        else k_mom_prep_rec<2, false><<<grid, block, 0, st>>>(p, x, oth, pf, AP, cells, rec, ur);
+        if (v_component) launch_prep_rec<2, true>(p, x, oth, pf, AP, cells, rec, ur, st);
+        else launch_prep_rec<2, false>(p, x, oth, pf, AP, cells, rec, ur, st);
     }
-    SGPU_LAUNCH();
 }
 
 void launch_mom_sweep_rec(const DevParams& p, bool v_component, const double* xin, double* xout, MomRec64 rec,

@@ -228,7 +228,8 @@ struct MomRec32 {
 // FP64 prep over the update range: AP (FP64), the cell's FP32 record, and one partial sum of |R|
 // per block into part; returns the number of partial sums (for launch_sum_partials).
 int launch_mom_prep_mixed(const DevParams& p, bool v_component, const double* x, const double* oth,
-                          const double* pf, double* AP, double* part, MomRec32 rec, cudaStream_t st);
+                          const double* pf, double* AP, double* part, MomRec32 rec,
+                          cudaStream_t st);
 // One FP32 multicolour correction sweep e_in -> e_out (e_zero: e_in is zero and not read).
 // xfinal != null: the last sweep of a component adds e to the FP64 field x over the update range
 // (x += e in FP64) instead of writing eout. *err (a device word) gets a nonzero bit if one of the
