@@ -48,6 +48,7 @@ SOURCES = {
     "conv_tc.cu": FAST,
     "mg32.cu": FAST,
     "mg_fast32.cu": FAST,
+    "mg_sweep32.cu": FAST,
     "mixed32.cu": FAST,
 }
 DRIVER = ["driver.cpp"]

@@ -160,9 +160,11 @@ void launch_mg_up(const LevelViewT<T>& C, const LevelViewT<T>& F, const T* xin, 
 // (the operators of assemble_p and mg_build), from AE, AN and b alone (mg_sweep.cu): as launch_mg_down and
 // launch_mg_up with two sweeps, and the sweeps by themselves on a level whose zero ring is implied
 // (parity 1: the cells with I + J odd are the first colour).
-void launch_sweeps_down(const LevelView& F, const LevelView& C, double* xout, bool x_zero, int sms, int min_seg,
+template <class T>
+void launch_sweeps_down(const LevelViewT<T>& F, const LevelViewT<T>& C, T* xout, bool x_zero, int sms, int min_seg,
                         cudaStream_t st, bool build);
-void launch_sweeps_up(const LevelView& C, const LevelView& F, const double* xin, double* xout, double omega, int sms,
+template <class T>
+void launch_sweeps_up(const LevelViewT<T>& C, const LevelViewT<T>& F, const T* xin, T* xout, double omega, int sms,
                       int min_seg, cudaStream_t st);
 void launch_sweeps_plain(const LevelView& L, const double* xin, double* xout, bool x_zero, int parity, int sms,
                          int min_seg, cudaStream_t st);

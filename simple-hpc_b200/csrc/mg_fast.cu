@@ -440,7 +440,10 @@ void launch_mg_down(const LevelViewT<T>& F, const LevelViewT<T>& C, T* xout, int
                     int sms, int min_seg, cudaStream_t st, bool build) {
     switch (pre) {
     case 1: down_t<1>(F, C, xout, x_zero, build, sms, min_seg, st); break;
-    case 2: down_t<2>(F, C, xout, x_zero, build, sms, min_seg, st); break;
+    case 2: // in float always mg_sweep.cu's kernel; in double its caller decides (symmetric operators)
+        if constexpr (sizeof(T) == 4) launch_sweeps_down<T>(F, C, xout, x_zero, sms, min_seg, st, build);
+        else down_t<2>(F, C, xout, x_zero, build, sms, min_seg, st);
+        break;
     case 3: down_t<3>(F, C, xout, x_zero, build, sms, min_seg, st); break;
     case 4: down_t<4>(F, C, xout, x_zero, build, sms, min_seg, st); break;
     default: throw Error(SGPU_E_INVALID, "streaming multigrid supports mg_pre 1..4");
@@ -453,7 +456,10 @@ void launch_mg_up(const LevelViewT<T>& C, const LevelViewT<T>& F, const T* xin, 
     switch (post) {
     case 0: up_t<0>(C, F, xin, xout, omega, sms, min_seg, st); break;
     case 1: up_t<1>(C, F, xin, xout, omega, sms, min_seg, st); break;
-    case 2: up_t<2>(C, F, xin, xout, omega, sms, min_seg, st); break;
+    case 2:
+        if constexpr (sizeof(T) == 4) launch_sweeps_up<T>(C, F, xin, xout, omega, sms, min_seg, st);
+        else up_t<2>(C, F, xin, xout, omega, sms, min_seg, st);
+        break;
     case 3: up_t<3>(C, F, xin, xout, omega, sms, min_seg, st); break;
     case 4: up_t<4>(C, F, xin, xout, omega, sms, min_seg, st); break;
     default: throw Error(SGPU_E_INVALID, "streaming multigrid supports mg_post 0..4");
