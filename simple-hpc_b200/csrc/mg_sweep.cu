@@ -17,10 +17,10 @@
 //    of AP there and every division goes through it (quotient() in common.hpp). A step reads all it needs
 //    before it stores (its cells' neighbours lie on rows and columns that no thread updates in the same
 //    step), so the two sweeps' chains overlap.
-// Measured, the streamed levels of a V(2,2) cycle at 4096^2: double, descent 670 -> 460 us and ascent 540 ->
-// 395 us; float, 309 -> 262 and 263 -> 244 us; float at 1024^2, 51 -> 32 and 47 -> 38 us. 8 sweeps of the
-// red-black solver at 1531 x 2047: 470 us (16 launches, a colour each) -> 192 us. The double passes are bound
-// by issue slots and shared-memory wavefronts (60% of each; DRAM 25%).
+// Measured, the streamed levels of a V(2,2) cycle at 4096^2: double, descent 670 -> 448 us and ascent 540 ->
+// 381 us; float, 309 -> 260 and 263 -> 219 us; float at 1024^2, 51 -> 31 and 47 -> 36 us. 8 sweeps of the
+// red-black solver at 1531 x 2047: 470 us (16 launches, a colour each) -> 184 us. The passes are bound by issue
+// slots (float: 3.0 instructions a cycle; double: 2.4, and 60% of the shared-memory wavefronts; DRAM 25%).
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -66,7 +66,7 @@ template <class T, int RC> struct Operator;
 template <int RC> struct Operator<double, RC> {
     double *AE, *AN, *B;
     __device__ explicit Operator(double* p) : AE(p), AN(p + RC * kNT), B(p + 2 * RC * kNT) {}
-    __device__ __forceinline__ void fetch(const LevelView& L, int k, long long c, bool in) const {
+    __device__ __forceinline__ void fetch(const LevelView& L, int k, int c, bool in) const {
         if (in) {
             cp_async(AE + k, L.AE + c);
             cp_async(AN + k, L.AN + c);
@@ -88,7 +88,7 @@ template <int RC> struct Operator<float, RC> {
     float4* K;
     float *P, *B;
     __device__ explicit Operator(float* p) : K(reinterpret_cast<float4*>(p)), P(p + 4 * RC * kNT), B(p + 5 * RC * kNT) {}
-    __device__ __forceinline__ void fetch(const LevelView32& L, int k, long long c, bool in) const {
+    __device__ __forceinline__ void fetch(const LevelView32& L, int k, int c, bool in) const {
         if (!in) return;
         cp_async(K + k, reinterpret_cast<const float4*>(L.L4) + c);
         cp_async(P + k, static_cast<const float*>(L.AP) + c);
@@ -106,27 +106,27 @@ template <int RC> struct Operator<float, RC> {
 
 // The updates of a step's two cells (multigrid.cpp:61-63) from their neighbour sums: of z, in its first sweep, whose
 // b is given, and of sw, in its second.
-__device__ __forceinline__ void update(bool ok0, bool ok1, double b0, double nb0, double nb1, Swept<double>& z,
-                                       const Swept<double>& sw, double& v0, double& v1) {
-    if (!ok0) z.ap = 1.0; // not a cell of this pass: nothing that would take the division's long path
-    z.y = inverse(z.ap);
-    bool slow0 = false, slow1 = false;
-    z.t0 = quotient_try(b0, z.ap, z.y, slow0);
-    v0 = quotient_try(nb0, z.ap, z.y, slow0);
-    v1 = quotient_try(nb1, sw.ap, sw.y, slow1);
-    if ((ok0 && slow0) || (ok1 && slow1)) {
-        z.t0 = divided(b0, z.ap);
-        v0 = divided(nb0, z.ap);
-        v1 = divided(nb1, sw.ap);
+template <class T>
+__device__ __forceinline__ void update(bool ok0, bool ok1, T b0, T nb0, T nb1, Swept<T>& z, const Swept<T>& sw, T& v0, T& v1) {
+    if constexpr (sizeof(T) == 8) {
+        if (!ok0) z.ap = 1.0; // not a cell of this pass: nothing that would take the division's long path
+        z.y = inverse(z.ap);
+        bool slow0 = false, slow1 = false;
+        z.t0 = quotient_try(b0, z.ap, z.y, slow0);
+        v0 = quotient_try(nb0, z.ap, z.y, slow0);
+        v1 = quotient_try(nb1, sw.ap, sw.y, slow1);
+        if ((ok0 && slow0) || (ok1 && slow1)) {
+            z.t0 = divided(b0, z.ap);
+            v0 = divided(nb0, z.ap);
+            v1 = divided(nb1, sw.ap);
+        }
+        v0 = z.t0 + v0;
+        v1 = sw.t0 + v1;
+    } else {
+        z.t0 = b0;
+        v0 = rb_value(b0, nb0, z.ap);
+        v1 = rb_value(sw.t0, nb1, sw.ap);
     }
-    v0 = z.t0 + v0;
-    v1 = sw.t0 + v1;
-}
-__device__ __forceinline__ void update(bool, bool, float b0, float nb0, float nb1, Swept<float>& z, const Swept<float>& sw,
-                                       float& v0, float& v1) {
-    z.t0 = b0;
-    v0 = rb_value(b0, nb0, z.ap);
-    v1 = rb_value(sw.t0, nb1, sw.ap);
 }
 
 // parity: 0 where the first colour is the cells with I + J even, 1 where it is the others.
@@ -147,63 +147,83 @@ __global__ void __launch_bounds__(kNT, (Shape<T, JOB>::ctas))
     const int J0 = blockIdx.x * W, C0 = J0 - kHalo, Jc = C0 + tid;                // owned, loaded, own column
     const bool cload = Jc >= -1 && Jc <= ny, cint = Jc >= 0 && Jc < ny;
     const bool cown = cint && Jc >= J0 && Jc < J0 + W;
-    // Pass k (colour k & 1 of sweep k / 2; 4: the residual) is computable k + 1 cells inside a cut edge.
+    // Pass k (colour k & 1 of sweep k / 2; 4: the residual) is computable k + 1 cells inside a cut edge: the
+    // thread's steps for it are the span's, of a column where it never is none. All of a step's tests are one
+    // subtraction and one unsigned comparison, and what differs between a thread's two colours is formed here,
+    // since the instructions of a step are what bounds the pass.
     const bool cut_top = L0 > -1, cut_bot = L1 < nx + 1, cut_left = C0 > -1, cut_right = C0 + kNT < ny + 1;
-    unsigned cols = 0;
-    for (int k = 0; k <= 4; ++k)
-        if (cint && (!cut_left || tid >= 1 + k) && (!cut_right || tid <= kNT - 2 - k)) cols |= 1u << k;
     const int lo = cut_top ? L0 + 1 : 0, hi = cut_bot ? L1 - 2 : nx - 1;
-    auto ok = [&](int I, int k) {
-        return ((cols >> k) & 1u) && I >= lo + (cut_top ? k : 0) && I <= hi - (cut_bot ? k : 0);
+    struct Span {
+        int first;
+        unsigned len;
+        __device__ __forceinline__ bool has(int t) const { return static_cast<unsigned>(t - first) < len; }
     };
-    auto at = [&](int I) { return (I & (kRing - 1)) * kNT + tid; };
-    auto cat = [&](int I) { return (I & (RC - 1)) * kNT + tid; };
+    auto span = [&](int k, int lag) { // the cell of step t is in row t - lag
+        const bool col = cint && (!cut_left || tid >= 1 + k) && (!cut_right || tid <= kNT - 2 - k);
+        const int a = lo + (cut_top ? k : 0), n = hi - (cut_bot ? k : 0) + 1 - a;
+        return Span{a + lag, col && n > 0 ? static_cast<unsigned>(n) : 0u};
+    };
+    auto rows = [&](bool col, int a, int b, int lag) { return Span{a + lag, col && b > a ? static_cast<unsigned>(b - a) : 0u}; };
+    auto wrap = [&](int e) { return e & (kRing * kNT - 1); };  // ring element of row I, column J: wrap(I * kNT + J)
+    auto cwrap = [&](int e) { return e & (RC * kNT - 1); };
 
-    int next = L0;
+    const Span loaded = rows(cload, L0, L1, 0), inside = rows(cint, 0, nx, 0);
+    int next = L0, c = L0 * ls + Jc; // the row to copy next, and its element of the level's arrays
     auto issue = [&]() {
-        if (next < L1 && cload) {
-            const int q = at(next), k = cat(next);
-            const bool in = cint && next >= 0 && next < nx;
-            const long long c = static_cast<long long>(next) * ls + Jc;
-            if (x_zero || (JOB == kPlain && !in)) X[q] = T(0);
-            else cp_async(X + q, xin + c);
-            A.fetch(L, k, c, in);
+        if (loaded.has(next)) {
+            const int e = next * kNT + tid;
+            const bool in = inside.has(next);
+            if (x_zero || (JOB == kPlain && !in)) X[wrap(e)] = T(0);
+            else cp_async(X + wrap(e), xin + c);
+            A.fetch(L, cwrap(e), c, in);
         }
         cp_async_commit();
         ++next;
+        c += ls;
     };
     for (int k = 0; k < LA + 1 + PF; ++k) issue();
 
     const int t0 = JOB == kUp ? L0 - 2 : L0;
     Swept<T> Q[4];
     T cx[4]; // kUp: the coarse correction of row t + 2 for the steps ahead
-    auto coarse_at = [&](int I) {
-        return cint && I >= 0 && I < nx && I < L1 ? __ldg(C.x + static_cast<long long>(I >> 1) * C.stride + (Jc >> 1)) : T(0);
+    const Span raised = rows(cint, 0, min(nx, L1), -2); // rows t + 2
+    auto coarse_at = [&](int t) {
+        return raised.has(t) ? __ldg(C.x + ((t + 2) >> 1) * C.stride + (Jc >> 1)) : T(0);
     };
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
         Q[d] = {T(0), T(0), T(0), T(0), T(1), T(1), T(0)};
-        if (JOB == kUp) cx[d] = coarse_at(t0 + d + 2);
+        if (JOB == kUp) cx[d] = coarse_at(t0 + d);
     }
     T r_prev = T(0), lp_e = T(0), lp_w = T(0), lp_n = T(0); // kDown: of the residual row before
 
-    auto step = [&](int t, Swept<T>& sw, T& cxt) {
+    // of the steps t0, t0 + 2, ..: colour col[0]; of the others: the other
+    const int col[2] = {(t0 + Jc + parity) & 1, (t0 + 1 + Jc + parity) & 1};
+    Span sp[2][2]; // first and second sweep
+    int ofs[2];    // ring element of the first sweep's cell, less t * kNT
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        sp[k][0] = span(col[k], 2 * col[k]);
+        sp[k][1] = span(2 + col[k], 2 * col[k] + 4);
+        ofs[k] = tid - 2 * col[k] * kNT;
+    }
+    const Span sp_res = span(4, kLag), sp_out = rows(cown, R0, R1, kLag - 1);
+
+    auto step = [&](int t, int d, Swept<T>& sw, T& cxt) {
         if (JOB == kUp && t < L0) cp_async_wait<PF + 1>();
         else cp_async_wait<PF>(); // rows <= t + LA have landed
         __syncthreads();
         if (JOB != kUp || t >= L0) issue();
         if (JOB == kUp) { // prolongation of row t + 2 (read first at step t + 1)
-            const int I = t + 2;
-            if (cint && I >= 0 && I < nx && I < L1) X[at(I)] += om * cxt;
+            if (raised.has(t)) X[wrap((t + 2) * kNT + tid)] += om * cxt;
         }
-        const int c = (t + Jc + parity) & 1;
-        const int I0 = t - 2 * c, I1 = I0 - 4;
-        const bool ok0 = ok(I0, c), ok1 = ok(I1, 2 + c);
-        const int q0 = at(I0), q0n = at(I0 - 1), q0s = at(I0 + 1);
-        const int q1 = at(I1), q1n = at(I1 - 1), q1s = at(I1 + 1);
+        const bool ok0 = sp[d & 1][0].has(t), ok1 = sp[d & 1][1].has(t);
+        const int e = t * kNT + ofs[d & 1];
+        const int q0 = wrap(e), q0n = wrap(e - kNT), q0s = wrap(e + kNT);
+        const int q1 = wrap(e - 4 * kNT), q1n = wrap(e - 5 * kNT), q1s = wrap(e - 3 * kNT);
         Swept<T> z;
-        const int k0 = cat(I0);
-        A.links(k0, cat(I0 + 1), z.e, z.w, z.n, z.s);
+        const int k0 = cwrap(e);
+        A.links(k0, cwrap(e + kNT), z.e, z.w, z.n, z.s);
         z.ap = A.ap(k0, z.e, z.w, z.n, z.s);
         const T nb0 = z.e * X[q0 + 1] + z.w * X[q0 - 1] + z.s * X[q0s] + z.n * X[q0n];
         const T nb1 = sw.e * X[q1 + 1] + sw.w * X[q1 - 1] + sw.s * X[q1s] + sw.n * X[q1n];
@@ -214,12 +234,12 @@ __global__ void __launch_bounds__(kNT, (Shape<T, JOB>::ctas))
         sw = z;
         if (JOB == kDown) {
             // Residual of row Ir (multigrid.cpp:84-85); its neighbours' updates are earlier steps'.
-            const int Ir = t - kLag, q = at(Ir), qn = at(Ir - 1), qs = at(Ir + 1);
-            T r = T(0), e = T(0), w = T(0), n = T(0), s = T(0);
-            if (ok(Ir, 4)) {
-                A.links(q, qs, e, w, n, s); // the rings are of the same height here
-                const T ap = A.ap(q, e, w, n, s);
-                r = A.B[q] - (ap * X[q] - (e * X[q + 1] + w * X[q - 1] + s * X[qs] + n * X[qn]));
+            const int Ir = t - kLag, er = Ir * kNT + tid, q = wrap(er), qn = wrap(er - kNT), qs = wrap(er + kNT);
+            T r = T(0), ke = T(0), kw = T(0), kn = T(0), ks = T(0);
+            if (sp_res.has(t)) {
+                A.links(q, qs, ke, kw, kn, ks); // the rings are of the same height here
+                const T ap = A.ap(q, ke, kw, kn, ks);
+                r = A.B[q] - (ap * X[q] - (ke * X[q + 1] + kw * X[q - 1] + ks * X[qs] + kn * X[qn]));
             }
             // Restriction of the rows Ir - 1 and Ir, C.b = r[f] + r[f+1] + r[f+fs] + r[f+fs+1], and with
             // build the coarse cell's links as mg_build adds them (the odd column from the next lane).
@@ -228,9 +248,9 @@ __global__ void __launch_bounds__(kNT, (Shape<T, JOB>::ctas))
                 T ep_odd = T(0), e_odd = T(0), np_odd = T(0), s_odd = T(0);
                 if (build) {
                     ep_odd = __shfl_down_sync(0xffffffffu, lp_e, 1);
-                    e_odd = __shfl_down_sync(0xffffffffu, e, 1);
+                    e_odd = __shfl_down_sync(0xffffffffu, ke, 1);
                     np_odd = __shfl_down_sync(0xffffffffu, lp_n, 1);
-                    s_odd = __shfl_down_sync(0xffffffffu, s, 1);
+                    s_odd = __shfl_down_sync(0xffffffffu, ks, 1);
                 }
                 const int Rc = Ir >> 1;
                 if (cown && !(Jc & 1) && Ir - 1 >= R0 && Ir < R1 && Rc < C.nx) {
@@ -238,26 +258,26 @@ __global__ void __launch_bounds__(kNT, (Shape<T, JOB>::ctas))
                     C.b[cq] = r_prev + rp_odd + r + r_odd;
                     C.x[cq] = T(0);
                     if (build) {
-                        const T ae = ep_odd + e_odd, aw = lp_w + w, an = lp_n + np_odd, as = s + s_odd;
+                        const T ae = ep_odd + e_odd, aw = lp_w + kw, an = lp_n + np_odd, as = ks + s_odd;
                         set_links(C, cq, ae, aw, an, as);
                         C.AP[cq] = ae + aw + an + as;
                     }
                 }
             }
             r_prev = r;
-            lp_e = e;
-            lp_w = w;
-            lp_n = n;
+            lp_e = ke;
+            lp_w = kw;
+            lp_n = kn;
         }
-        const int rw = t - kLag + 1; // had its last update at step t - 1
-        if (cown && rw >= R0 && rw < R1) xout[static_cast<long long>(rw) * ls + Jc] = X[at(rw)];
-        if (JOB == kUp) cxt = coarse_at(t + 4 + 2);
+        // row t - kLag + 1 had its last update at step t - 1
+        if (sp_out.has(t)) xout[(t - kLag + 1) * ls + Jc] = X[wrap((t - kLag + 1) * kNT + tid)];
+        if (JOB == kUp) cxt = coarse_at(t + 4);
     };
     const int t_last = R1 - 1 + kLag;
     for (int t = t0; t <= t_last; t += 4) {
 #pragma unroll
         for (int d = 0; d < 4; ++d)
-            if (t + d <= t_last) step(t + d, Q[d], cx[d]);
+            if (t + d <= t_last) step(t + d, d, Q[d], cx[d]);
     }
     cp_async_wait<0>();
 }
