@@ -121,7 +121,7 @@ void launch_mg_sub_mean(const LevelView& L, double* x, const double* sum, cudaSt
 template <class T>
 void launch_mg_coarse(const LevelViewT<T>& L, double* rowbuf, double tol, int* sweeps_out,
                       cudaStream_t st);
-// The whole hierarchy, by value, for the single-CTA tail kernel.
+// The whole hierarchy, by value, for the tail kernels.
 template <class T> struct MgLevelsT {
     LevelViewT<T> L[24];
     int n;

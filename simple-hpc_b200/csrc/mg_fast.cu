@@ -14,7 +14,9 @@
 //  * k_mg_up: prolongation with over-correction (:106-116) applied to each row as it arrives,
 //    followed by `post` red-black sweeps, in the same streaming order.
 // The smoothed iterate goes to a second buffer (CTAs read their neighbours' rows as halo). Levels
-// below a size threshold and the coarsest solve run in one CTA (k_mg_tail in mg.cu).
+// below a size threshold and the coarsest solve run in a tail kernel on one CTA or a cluster (mg.cu).
+// With two sweeps (the default) the float levels, and the double ones whose operator the solver itself
+// assembled, run on mg_sweep.cu's kernel; these take the other counts and operators.
 #include "kernels.hpp"
 
 #include <algorithm>

@@ -118,7 +118,7 @@ struct Solver {
     std::vector<LevelView> lv;
     double* mg_r0 = nullptr;
     double* coarse_rowbuf = nullptr;
-    bool mg_fast = false;            // streaming level kernels (mg_fast.cu) + single-CTA tail
+    bool mg_fast = false;            // streaming level kernels (mg_sweep.cu, mg_fast.cu) + a tail
     int mg_tail = 0;                 // first level handled by the tail kernel
     // first level of the float and of the double V-cycle's tail: the cluster tail's (mg.cu,
     // k_mg_tail_cluster) where the device and the grid allow it, else mg_tail
@@ -438,9 +438,14 @@ struct Solver {
         launch_ordered_sum_abs_pair(w.b + p_origin(), g.pitch, prm.NX, prm.NY, res3 + 2, ss, st);
         mark(SGPU_PH_SOLVE_P);
         b_sum = res3 + 3; // the multigrid's mean of b reuses the pair's sum of b
-        own_links = true;
-        solve_p();
-        own_links = false;
+        {
+            struct Scope { // cleared also where the solve throws
+                bool& flag;
+                ~Scope() { flag = false; }
+            } scope{own_links};
+            own_links = true;
+            solve_p();
+        }
         b_sum = nullptr;
         mark(SGPU_PH_CORRECT);
         correct();
