@@ -29,7 +29,7 @@ namespace sgpu {
 
 namespace {
 
-constexpr int kNT = 128;        // threads: loaded columns of a strip
+constexpr int kNT = 128;        // threads: loaded columns of a strip (a power of two: ring elements wrap by a mask)
 constexpr int kRing = 16;       // rows of the x ring
 constexpr int kHalo = 6;        // of a strip: one cell per colour pass, one for the residual, kept even
 constexpr int kLag = 8;         // rows between a step and the row whose two sweeps it completes
