@@ -67,7 +67,11 @@ struct CoarseCta {
     }
     // a barrier that also tells whether v holds for any thread
     __device__ __forceinline__ bool vote(bool v, int, double*) const {
-        if (nt == 32) return __any_sync(0xffffffffu, v) != 0;
+        if (nt == 32) {
+            const bool any = __any_sync(0xffffffffu, v) != 0;
+            __syncwarp(); // a vote alone orders no memory
+            return any;
+        }
         unsigned o;
         asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.or.pred q, 1, %2, p;\n"
                      " selp.u32 %0, 1, 0, q;\n}\n"

@@ -76,3 +76,18 @@ def test_coarse_solve_fp32(sgpu_mod, nx, ny):
     x = x[1:-1, 1:-1].astype(float)
     x -= x.mean()
     assert np.max(np.abs(pc - x)) <= 1e-4 * np.max(np.abs(x))
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (1, 60), (7, 8), (8, 8), (10, 6), (32, 1), (28, 28), (128, 64), (5, 12)])
+def test_one_warp_solve(sgpu_mod, oracle_mod, nx, ny):
+    """Coarsest levels of at most 32 cell pairs, which one warp solves: its vote is also the barrier between a
+    colour's stores and the other colour's loads. Alone, inside the one-CTA tail and inside the cluster tail."""
+    p = sgpu_mod.params_from_config(_cfg(nx, ny))
+    o = oracle_mod.Oracle(p)
+    _, _, olog = o.run(3)
+    with sgpu_mod.Solver(p) as g:
+        _, log = g.run(3)
+        assert bit_equal(log, olog), describe_diff(log, olog)
+        for f in (0, 1, 2, sgpu_mod.F_PC):
+            assert bit_equal(g.download(f), o.get(f)), f"field {f}: " + describe_diff(g.download(f), o.get(f))
+        assert g.last_solve_stats()["coarse_sweeps"] == o.mg_last_coarse_sweeps()
