@@ -191,11 +191,20 @@ using LevelView32 = LevelViewT<float>;
 template <class T> struct Links {
     T e, w, n, s;
 };
+// Through the read-only path: for operators that the running kernel does not write.
 __device__ __forceinline__ Links<double> links(const LevelViewT<double>& L, int q) {
     return {__ldg(L.AE + q), __ldg(L.AW + q), __ldg(L.AN + q), __ldg(L.AS + q)};
 }
 __device__ __forceinline__ Links<float> links(const LevelViewT<float>& L, int q) {
     const float4 v = __ldg(reinterpret_cast<const float4*>(L.L4) + q);
+    return {v.x, v.y, v.z, v.w};
+}
+// With plain loads: for operators that the running kernel may itself have formed (set_links).
+__device__ __forceinline__ Links<double> links_written(const LevelViewT<double>& L, int q) {
+    return {L.AE[q], L.AW[q], L.AN[q], L.AS[q]};
+}
+__device__ __forceinline__ Links<float> links_written(const LevelViewT<float>& L, int q) {
+    const float4 v = reinterpret_cast<const float4*>(L.L4)[q];
     return {v.x, v.y, v.z, v.w};
 }
 __device__ __forceinline__ void set_links(const LevelViewT<double>& L, int q, double e, double w, double n,

@@ -155,7 +155,7 @@ template <class T> __device__ void cta_smooth_colour(const LevelViewT<T>& L, int
         const int I = k / L.ny, J = k % L.ny;
         if (((I + J) & 1) != colour) continue;
         const int q = I * s + J;
-        const Links<T> k4 = links(L, q);
+        const Links<T> k4 = links_written(L, q);
         x[q] = rb_value(L.b[q], k4.e * x[q + 1] + k4.w * x[q - 1] + k4.s * x[q + s] + k4.n * x[q - s], L.AP[q]);
     }
     __syncthreads();
@@ -166,7 +166,7 @@ template <class T> __device__ void cta_residual(const LevelViewT<T>& L) {
     const T* x = L.x;
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const int I = k / L.ny, J = k % L.ny, q = I * s + J;
-        const Links<T> k4 = links(L, q);
+        const Links<T> k4 = links_written(L, q);
         L.r[q] = L.b[q] - (L.AP[q] * x[q] - (k4.e * x[q + 1] + k4.w * x[q - 1] + k4.s * x[q + s] + k4.n * x[q - s]));
     }
     __syncthreads();
@@ -189,7 +189,8 @@ template <class T> __device__ void cta_build(const LevelViewT<T>& F, const Level
     const int n = C.nx * C.ny, fs = F.stride;
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const int I = k / C.ny, J = k % C.ny, f = 2 * I * fs + 2 * J;
-        build_cell(C, I * C.stride + J, links(F, f), links(F, f + 1), links(F, f + fs), links(F, f + fs + 1));
+        build_cell(C, I * C.stride + J, links_written(F, f), links_written(F, f + 1),
+                   links_written(F, f + fs), links_written(F, f + fs + 1));
     }
     __syncthreads();
 }
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(kCoarseThreads)
 // A level in global memory as coarse_solve's cells.
 template <class T> __device__ CoarseCell<T> coarse_load(const LevelViewT<T>& L, int I, int J) {
     const int q = I * L.stride + J;
-    const Links<T> k = links(L, q);
+    const Links<T> k = links_written(L, q);
     return {k.e, k.w, k.n, k.s, L.AP[q], L.b[q], L.x[q]};
 }
 

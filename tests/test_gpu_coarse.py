@@ -91,3 +91,18 @@ def test_one_warp_solve(sgpu_mod, oracle_mod, nx, ny):
         for f in (0, 1, 2, sgpu_mod.F_PC):
             assert bit_equal(g.download(f), o.get(f)), f"field {f}: " + describe_diff(g.download(f), o.get(f))
         assert g.last_solve_stats()["coarse_sweeps"] == o.mg_last_coarse_sweeps()
+
+
+@pytest.mark.parametrize("nx,ny", [(52, 52), (56, 56), (60, 60), (64, 64), (80, 48), (62, 66)])
+def test_tail_in_global_memory(sgpu_mod, oracle_mod, nx, ny):
+    """FP64 tails that do not fit one CTA's shared memory form their coarse operators in global memory and read
+    them back in the same kernel. Alone, and as the cavity of a batch that takes the batch shape."""
+    p = sgpu_mod.params_from_config(_cfg(nx, ny))
+    o = oracle_mod.Oracle(p)
+    o.run(3)
+    with sgpu_mod.Solver(p) as g, sgpu_mod.Batch([sgpu_mod.params_from_config(_cfg(128, 128))] * 8 + [p]) as b:
+        g.run(3)
+        b.run(3)
+        for f in (0, 1, 2, sgpu_mod.F_PC):
+            for got in (g.download(f), b.download(8, f)):
+                assert bit_equal(got, o.get(f)), f"field {f}: " + describe_diff(got, o.get(f))
