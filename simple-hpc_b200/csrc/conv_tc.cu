@@ -245,32 +245,34 @@ __global__ void __launch_bounds__(kThreadsConv)
                 const bool live = r < pl.rb && c < pl.cw && y0 + r < H && x0 + c < W;
                 const long o = (image + static_cast<long>(y0 + r) * W + x0 + c) * Cout + co0 + k0;
                 float v[16];
+                __syncwarp(); // tcgen05.ld takes the whole warp, converged
                 tmem_ld16(tmem + lane_base + static_cast<uint32_t>(b * pl.nt + k0), v);
-                if (!live) continue;
-                uint4 q[2], y[2];
-                if (mask) {
-                    y[0] = __ldg(reinterpret_cast<const uint4*>(mask + o));
-                    y[1] = __ldg(reinterpret_cast<const uint4*>(mask + o) + 1);
-                }
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    float v0 = v[2 * k] + (bias ? bias[co0 + k0 + 2 * k] : 0.0f);
-                    float v1 = v[2 * k + 1] + (bias ? bias[co0 + k0 + 2 * k + 1] : 0.0f);
-                    if (relu) {
-                        v0 = fmaxf(v0, 0.0f);
-                        v1 = fmaxf(v1, 0.0f);
-                    }
-                    __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+                if (live) {
+                    uint4 q[2], y[2];
                     if (mask) {
-                        h = relu_mask((&y[0].x)[k], h);
-                        sum[2 * k] += __low2float(h);
-                        sum[2 * k + 1] += __high2float(h);
+                        y[0] = __ldg(reinterpret_cast<const uint4*>(mask + o));
+                        y[1] = __ldg(reinterpret_cast<const uint4*>(mask + o) + 1);
                     }
-                    (&q[0].x)[k] = *reinterpret_cast<const uint32_t*>(&h);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        float v0 = v[2 * k] + (bias ? bias[co0 + k0 + 2 * k] : 0.0f);
+                        float v1 = v[2 * k + 1] + (bias ? bias[co0 + k0 + 2 * k + 1] : 0.0f);
+                        if (relu) {
+                            v0 = fmaxf(v0, 0.0f);
+                            v1 = fmaxf(v1, 0.0f);
+                        }
+                        __nv_bfloat162 h = __floats2bfloat162_rn(v0, v1);
+                        if (mask) {
+                            h = relu_mask((&y[0].x)[k], h);
+                            sum[2 * k] += __low2float(h);
+                            sum[2 * k + 1] += __high2float(h);
+                        }
+                        (&q[0].x)[k] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                    uint4* dst = reinterpret_cast<uint4*>(Y + o);
+                    dst[0] = q[0];
+                    dst[1] = q[1];
                 }
-                uint4* dst = reinterpret_cast<uint4*>(Y + o);
-                dst[0] = q[0];
-                dst[1] = q[1];
             }
             if (mask) { // (uniform) the bias gradient of the masked output
 #pragma unroll
@@ -441,6 +443,7 @@ __global__ void __launch_bounds__(kThreadsTc)
         if (warp * 32 < Cout) // uniform in the warp
             for (int c0 = 0; c0 < nt * Cin; c0 += 16) { // 16 columns of one tap (Cin is a multiple of 16)
                 float v[16];
+                __syncwarp(); // (as above)
                 tmem_ld16(tmem + lane_base + static_cast<uint32_t>(c0), v);
                 if (co < Cout) {
                     float* dst = dW + (static_cast<long>(co) * 9 + t0) * Cin + c0;

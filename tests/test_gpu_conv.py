@@ -34,3 +34,24 @@ def test_convolutions_at_tile_edges(sgpu_mod, n, h, w, base):
     for (cin, cout, _), (wo, bo) in zip(o.convs, o.offs):
         assert rel_l2(g[wo:bo], rg[wo:bo]) < 1e-2
         assert rel_l2(g[bo:bo + cout], rg[bo:bo + cout]) < 1e-2
+
+
+@pytest.mark.parametrize("n,h,w,base", [(1, 40, 50, 16), (2, 61, 9, 32), (1, 200, 130, 16), (5, 19, 35, 64)])
+def test_epilogue_of_partly_live_warps(sgpu_mod, n, h, w, base):
+    """Tiles of several blocks of 128 pixels in which some lanes of a warp have an output pixel and others do not
+    (halo columns, columns and rows past the image), with the masked input gradient too. Bounds as above."""
+    import cnn_oracle
+    params = cnn_oracle.init_params(base, 1, seed=h + w)
+    rng = np.random.default_rng(11)
+    x = rng.normal(size=(n, h, w, 2)).astype(np.float32)
+    t = rng.normal(size=(n, h, w)).astype(np.float32)
+    with sgpu_mod.Cnn(base, 1) as net:
+        net.set_params(params)
+        out = net.forward(x)
+        _, g = net.loss_grad(x, t)
+    o = cnn_oracle.UNetOracle(base, 1)
+    _, rg, ref = o.loss_grad(params, x, t)
+    assert rel_l2(out, ref) < 5e-3
+    for (cin, cout, _), (wo, bo) in zip(o.convs, o.offs):
+        assert rel_l2(g[wo:bo], rg[wo:bo]) < 1e-2
+        assert rel_l2(g[bo:bo + cout], rg[bo:bo + cout]) < 1e-2
