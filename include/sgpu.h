@@ -196,6 +196,11 @@ int sgpu_memory_bytes(sgpu_handle* h, size_t* bytes);
  * through the same bounded-wait helper the mixed mode's correction sweep uses. *gave_up = 1 when the
  * wait ended by giving up and reported it, as it must; the GPU context stays usable. */
 int sgpu_selftest_bounded_wait(int polls, int* gave_up);
+/* The same for the reporting (no counterpart in the reference): leaves the handle's error words as a wait
+ * that gave up leaves them, so that its next sgpu_solve_p, sgpu_outer_iteration or sgpu_run must return
+ * SGPU_E_TIMEOUT, and the one after it run normally. Nothing is launched. SGPU_E_INVALID for a handle
+ * without such waits. */
+int sgpu_selftest_set_timeout(sgpu_handle* h);
 /* Number of multigrid levels and the dims of level l (mg_level_dims, multigrid.cpp:143-151). */
 int sgpu_mg_levels(int NX, int NY, int* nlevels, int* dims /* 2 * 64 ints, may be NULL */);
 /* Statistics of the last solve_p: CG iterations, MG V-cycles, coarsest-level sweeps. */

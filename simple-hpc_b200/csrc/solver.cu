@@ -112,7 +112,7 @@ struct Solver {
     double* res_dev = nullptr; // res_u, res_v, res_p of the current iteration
     SumScratch ss;
     int* stats = nullptr;      // device ints: [0] coarse sweeps
-    double* host_res = nullptr; // pinned: 3 residuals
+    double* host_res = nullptr; // pinned: 3 residuals, [4] CG iterations, [6] error words
 
     // multigrid
     std::vector<LevelView> lv;
@@ -531,27 +531,38 @@ struct Solver {
     }
     MomRec32 rec32{};                 // per-cell FP32 records: coefficients, 1/AP, R
     unsigned* corr_err = nullptr;     // device word: a record sweep's bounded wait gave up
-    // Raises SGPU_E_TIMEOUT if a record sweep since the last check gave up waiting for its
-    // record copies (its results are then not to be trusted); clears the word.
-    void check_pipeline() {
+    // Every call that runs a solve or a sweep reports a bounded wait that gave up since the last check (its
+    // results are then not to be trusted) as SGPU_E_TIMEOUT: fetch_errors before the call's synchronisation,
+    // raise_errors after it, which clears the words.
+    unsigned* host_err() { return reinterpret_cast<unsigned*>(host_res + 6); } // pinned: corr_err, cg_err
+    void fetch_errors() {
+        unsigned* const dev[2] = {corr_err, cg_err};
+        for (int k = 0; k < 2; ++k) {
+            host_err()[k] = 0;
+            if (dev[k]) SGPU_CUDA(cudaMemcpyAsync(host_err() + k, dev[k], sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        }
+    }
+    void raise_errors() {
         if (net) net->check_error(st);
-        if (cg_err) {
-            unsigned h = 0;
-            SGPU_CUDA(cudaMemcpyAsync(&h, cg_err, sizeof h, cudaMemcpyDeviceToHost, st));
-            sync();
-            if (h) {
-                SGPU_CUDA(cudaMemsetAsync(cg_err, 0, sizeof h, st));
-                throw Error(SGPU_E_TIMEOUT, "conjugate gradients: a bounded wait for the other blocks' sums ran out");
-            }
-        }
-        if (!corr_err) return;
-        unsigned h = 0;
-        SGPU_CUDA(cudaMemcpyAsync(&h, corr_err, sizeof h, cudaMemcpyDeviceToHost, st));
+        const unsigned corr = host_err()[0], cg_wait = host_err()[1];
+        host_err()[0] = host_err()[1] = 0;
+        if (corr) SGPU_CUDA(cudaMemsetAsync(corr_err, 0, sizeof(unsigned), st));
+        if (cg_wait) SGPU_CUDA(cudaMemsetAsync(cg_err, 0, sizeof(unsigned), st));
+        if (cg_wait)
+            throw Error(SGPU_E_TIMEOUT, "conjugate gradients: a bounded wait for the other blocks' sums ran out");
+        if (corr) throw Error(SGPU_E_TIMEOUT, "momentum sweep: a bounded wait for its record copies ran out");
+    }
+    void check_pipeline() {
+        fetch_errors();
         sync();
-        if (h) {
-            SGPU_CUDA(cudaMemsetAsync(corr_err, 0, sizeof h, st));
-            throw Error(SGPU_E_TIMEOUT, "momentum sweep: a bounded wait for its record copies ran out");
-        }
+        raise_errors();
+    }
+    // The words as a wait that gave up leaves them; false for a solver that has no such wait.
+    bool set_errors() {
+        for (unsigned* w : {corr_err, cg_err})
+            if (w) SGPU_CUDA(cudaMemsetAsync(w, 1, sizeof(unsigned), st));
+        sync();
+        return corr_err || cg_err;
     }
     // FP64 defect correction of the p' solve in tolerance mode: the FP64 iterate ping-pongs between
     // two full-grid arrays (allocated on first use); pc_dc_src is the last iteration's final iterate.
@@ -1756,7 +1767,7 @@ int sgpu_solve_p(sgpu_handle* h) {
     SGPU_NEED_HANDLE(h);
     return guarded([&] {
         h->s->solve_p();
-        h->s->sync();
+        h->s->check_pipeline();
         h->s->finish_stats();
     });
 }
@@ -1774,9 +1785,11 @@ int sgpu_outer_iteration(sgpu_handle* h, double res[3], double* phase_seconds) {
         s.iteration_enqueue(s.res_dev);
         SGPU_CUDA(cudaMemcpyAsync(s.host_res, s.res_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost,
                                   s.st));
+        s.fetch_errors();
         s.sync();
         s.collect_phases(phase_seconds);
         s.profiling = was;
+        s.raise_errors();
         if (res) {
             res[0] = s.host_res[0];
             res[1] = s.host_res[1];
@@ -1994,6 +2007,14 @@ int sgpu_selftest_bounded_wait(int polls, int* gave_up) {
         }
         SGPU_CUDA(cudaFree(err));
         *gave_up = h != 0 ? 1 : 0;
+    });
+}
+
+int sgpu_selftest_set_timeout(sgpu_handle* h) {
+    SGPU_NEED_HANDLE(h);
+    return guarded([&] {
+        if (!h->s->set_errors())
+            throw sgpu::Error(SGPU_E_INVALID, "sgpu_selftest_set_timeout: this solver has no bounded waits");
     });
 }
 

@@ -109,6 +109,7 @@ def lib() -> C.CDLL:
             "sgpu_download": (I, [H, I, D]), "sgpu_upload": (I, [H, I, D]),
             "sgpu_memory_bytes": (I, [H, C.POINTER(C.c_size_t)]),
             "sgpu_selftest_bounded_wait": (I, [I, C.POINTER(I)]),
+            "sgpu_selftest_set_timeout": (I, [H]),
             "sgpu_mg_levels": (I, [I, I, C.POINTER(I), C.POINTER(I)]),
             "sgpu_last_solve_stats": (I, [H, C.POINTER(I), C.POINTER(I), C.POINTER(I), D]),
             "sgpu_ordered_sum": (I, [D, I, I, D]),
@@ -460,6 +461,10 @@ class Solver:
         n = C.c_size_t()
         _check(lib().sgpu_memory_bytes(self._h, C.byref(n)))
         return n.value
+
+    def selftest_set_timeout(self) -> None:
+        """Leave the error words as a bounded wait that gave up does: the next solve must report it."""
+        _check(lib().sgpu_selftest_set_timeout(self._h))
 
     def set_profiling(self, on) -> None:
         """False / True (every iteration timed per phase), or "sampled" (the first 10 iterations of a

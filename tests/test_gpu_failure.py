@@ -37,3 +37,42 @@ def test_selftest_rejects_bad_arguments(sgpu_mod):
     for polls in (0, -3, (1 << 20) + 1):
         with pytest.raises(sgpu_mod.SgpuError, match="polls"):
             sgpu_mod.selftest_bounded_wait(polls)
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+@pytest.mark.parametrize("call", ["solve_p", "outer_iteration", "run"])
+@pytest.mark.parametrize("n,kw", [(40, {"pressure_solver": "cg"}), (300, {"pressure_solver": "mg"}),
+                                  (48, {"pressure_solver": "mg", "precision": "mixed"})])
+def test_every_solving_call_reports_a_give_up(sgpu_mod, n, kw, call):
+    """A wait that gave up during a call is that call's error, whichever entry point it is; the call after it is a
+    solver's that never had one."""
+    cfg = snapshot_config("short_16")
+    cfg.update(N_cells_x=str(n), N_cells_y=str(n), momentum_solver="gs_multicolour", maxit="9", error_tolerance="0", **kw)
+    p = sgpu_mod.params_from_config(config_text(cfg))
+    go = {"solve_p": lambda s: s.solve_p(), "outer_iteration": lambda s: s.outer_iteration(), "run": lambda s: s.run(1)}[call]
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for s in (a, b):
+            s.assemble_u(), s.assemble_v(), s.assemble_p()
+        a.selftest_set_timeout()
+        with pytest.raises(sgpu_mod.SgpuError) as e:
+            go(a)
+        assert e.value.code == sgpu_mod.E_TIMEOUT
+        zero = a.download(0) * 0.0
+        for s in (a, b):  # the same fields in both, whatever the failed call left
+            for f in (0, 1, 2):
+                s.upload(f, zero)
+            s.assemble_u(), s.assemble_v(), s.assemble_p()
+            go(s)
+        for f in (0, 1, 2, sgpu_mod.F_PC):
+            assert (a.download(f) == b.download(f)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not cuda_available(), reason="needs a CUDA device")
+def test_no_bounded_wait_to_fail(sgpu_mod):
+    cfg = snapshot_config("short_16")
+    cfg.update(momentum_solver="jacobi", pressure_solver="jacobi")
+    with sgpu_mod.Solver(sgpu_mod.params_from_config(config_text(cfg))) as s:
+        with pytest.raises(sgpu_mod.SgpuError, match="no bounded waits"):
+            s.selftest_set_timeout()
