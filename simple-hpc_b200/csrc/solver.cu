@@ -1369,6 +1369,7 @@ void Solver::mg_vcycle_fast(bool x_is_zero, bool build) {
 }
 
 void Solver::solve_p() {
+    fetch_tol();      // statistics of a graph's last solve are not to replace this one's
     pc_stale = false; // the FP64 p' field is written by this solve
     switch (prm.pressure_solver) {
     case SGPU_P_JACOBI: solve_jacobi(); break;

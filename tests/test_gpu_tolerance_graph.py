@@ -47,3 +47,21 @@ def test_run_follows_changes_of_mode(sgpu_mod, precision):
             assert bit_equal(np.ascontiguousarray(log[:, 1:]), rows)
             for f in (0, 1, 2, sgpu_mod.F_PC):
                 assert bit_equal(a.download(f), b.download(f)), f"{mode}, field {f}"
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solve_p_after_run_has_its_own_statistics(sgpu_mod, precision):
+    """The statistics are those of the last p' solve, a per-phase one after a run included."""
+    p = _params(sgpu_mod, 64, 96, precision, pressure_tolerance="1e-7")
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        a.run(2)
+        for _ in range(2):
+            b.outer_iteration()
+        for s in (a, b):
+            for f in (0, 1):
+                s.upload(f, 1e3 * s.download(f))  # another solve than the run's last
+            s.assemble_u(), s.assemble_v(), s.assemble_p()
+            s.solve_p()
+        assert a.last_solve_stats() == b.last_solve_stats()
+        assert a.warm_start_stats() == b.warm_start_stats()
+        assert bit_equal(a.download(sgpu_mod.F_PC), b.download(sgpu_mod.F_PC))
