@@ -177,8 +177,11 @@ __device__ void coarse_solve(const Team& tm, int nx, int ny, int i0, int m, int 
     if (bb > 0.0) {
         const double bn = sqrt(bb), thr = tol * bn;
         // |r| >= big in any cell: sqrt of the sum of squares is not below thr (the margin covers the
-        // rounding of the squares, the sum and the root; the float one that of the bound too)
-        const T big = static_cast<T>(thr * (sizeof(T) == 8 ? 1.0 + 1e-9 : 1.0 + 1e-6));
+        // rounding of the squares, the sum and the root; the float one that of the bound too). That needs
+        // squares of normal size and a bound that T holds: below, the norm is formed after every sweep.
+        const T big = thr >= (sizeof(T) == 8 ? 1e-140 : 1e-30)
+                          ? static_cast<T>(thr * (sizeof(T) == 8 ? 1.0 + 1e-9 : 1.0 + 1e-6))
+                          : static_cast<T>(INFINITY);
         const T t0[2] = {coarse_t0(c[0].b, c[0].ap), coarse_t0(c[1].b, c[1].ap)};
         const T y[2] = {coarse_inverse(c[0].ap), coarse_inverse(c[1].ap)};
         // This thread's cells are element o of each colour's array; the neighbours are o + odd (east),

@@ -106,3 +106,22 @@ def test_tail_in_global_memory(sgpu_mod, oracle_mod, nx, ny):
         for f in (0, 1, 2, sgpu_mod.F_PC):
             for got in (g.download(f), b.download(8, f)):
                 assert bit_equal(got, o.get(f)), f"field {f}: " + describe_diff(got, o.get(f))
+
+
+@pytest.mark.parametrize("nx,ny", [(8, 8), (31, 33), (32, 32), (46, 45), (128, 128)])
+@pytest.mark.parametrize("scale", [1e-100, 1e-148, 1e-155, 1e-157, 1e-159, 1e-161])
+def test_right_hand_sides_whose_squares_underflow(sgpu_mod, oracle_mod, nx, ny, scale):
+    """The reference stops when the sum of squares is small, and squares of values below 1e-154 lose their digits
+    or vanish: it then stops earlier than the residuals themselves would say. Same sweep counts, same bits."""
+    p = sgpu_mod.params_from_config(_cfg(nx, ny))
+    o = oracle_mod.Oracle(p)
+    b = np.random.default_rng(nx).standard_normal((p.nrows, p.ncols)) * scale
+    with sgpu_mod.Solver(p) as g:
+        for s in (o, g):
+            s.assemble_u(), s.assemble_v(), s.assemble_p()
+        o.set(sgpu_mod.F_B, b)
+        g.upload(sgpu_mod.F_B, b)
+        o.solve_p()
+        g.solve_p()
+        assert g.last_solve_stats()["coarse_sweeps"] == o.mg_last_coarse_sweeps()
+        assert bit_equal(g.download(sgpu_mod.F_PC), o.get(sgpu_mod.F_PC))
