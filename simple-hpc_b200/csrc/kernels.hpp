@@ -194,10 +194,11 @@ bool launch_cg_solve(const DevParams& p, PressurePtr w, CgPtr cg, CgScalars* sc,
                      int sms, cudaStream_t st);
 
 // State of a tolerance-driven V-cycle loop that runs inside a graph (mg_mode = tolerance): the cycles of the
-// current p' solve, ||b||^2 and the relative residual after the last one.
+// current p' solve, ||b||^2 and the relative residual after the last one; the cycles of all solves so far.
 struct TolState {
     double bb, rel;
     int cycles;
+    long long total;
 };
 
 // ---- mixed precision (mixed.cu) ----

@@ -87,6 +87,7 @@ __global__ void k_tol_step(TolState* t, const double* rr, double tol, int maxc, 
     const double nb = sqrt(t->bb), nr = sqrt(*rr);
     t->rel = nr / nb;
     const int c = ++t->cycles;
+    ++t->total;
     cudaGraphSetConditional(h, !(nr <= tol * nb) && c < maxc ? 1u : 0u);
 }
 
@@ -740,6 +741,8 @@ struct Solver {
     bool capturing = false;
     TolState* tol = nullptr;   // device; its cycles and residual are the last solve's while tol_stats
     bool tol_stats = false;
+    long long cycle_launches = 0; // kernels of one pass of the captured loop
+    long long tol_total = 0;      // TolState::total at the end of the last graphed run
     // What a capture may not allocate.
     void before_capture() {
         if (prm.pressure_solver != SGPU_P_MG || prm.mg_mode != SGPU_MG_TOLERANCE) return;
@@ -778,9 +781,11 @@ struct Solver {
             SGPU_CUDA(cudaStreamBeginCaptureToGraph(inner, wp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                     cudaStreamCaptureModeRelaxed));
             st = inner;
+            const long long before = g_launches.load();
             cycle();
             k_tol_step<<<1, 1, 0, st>>>(tol, rr, prm.pressure_tolerance, prm.pressure_maxit, h);
             SGPU_LAUNCH();
+            cycle_launches = g_launches.load() - before;
             st = outer;
             SGPU_CUDA(cudaStreamEndCapture(inner, &got));
         } catch (...) {
@@ -1819,6 +1824,7 @@ static bool run_graphed(sgpu::Solver& s, int maxit, double* log, int print_every
     if (start > 0) g.resume(s.st, start, maxr);
     const int chunk = print_every > 0 ? print_every : maxit;
     int done = start, conv = 0;
+    sgpu::TolState tol{};
     std::vector<double> rows;
     while (done < maxit) {
         const int lim = std::min(maxit, done + chunk);
@@ -1826,6 +1832,7 @@ static bool run_graphed(sgpu::Solver& s, int maxit, double* log, int print_every
         int it = 0;
         SGPU_CUDA(cudaMemcpyAsync(&it, g.bd.iters, sizeof(int), cudaMemcpyDeviceToHost, s.st));
         SGPU_CUDA(cudaMemcpyAsync(&conv, g.bd.converged, sizeof(int), cudaMemcpyDeviceToHost, s.st));
+        if (s.tol) SGPU_CUDA(cudaMemcpyAsync(&tol, s.tol, sizeof tol, cudaMemcpyDeviceToHost, s.st));
         s.sync();
         if (print_every > 0 && it > done) {
             rows.resize(4 * static_cast<std::size_t>(it - done));
@@ -1847,6 +1854,11 @@ static bool run_graphed(sgpu::Solver& s, int maxit, double* log, int print_every
     g.count(done - start, done - start);
     if (done > start) { // what iteration_enqueue notes on the host when it launches an iteration
         s.tol_stats = s.prm.pressure_solver == SGPU_P_MG && s.prm.mg_mode == SGPU_MG_TOLERANCE;
+        if (s.tol_stats) { // an iteration's count holds one pass of its cycle loop
+            const long long cycles = tol.total - s.tol_total;
+            sgpu::count_launches((cycles - (done - start)) * s.cycle_launches);
+            s.tol_total = tol.total;
+        }
         if (s.mixed) s.p_links_stale = s.pc_stale = true;
     }
     out.iterations = done;

@@ -65,3 +65,25 @@ def test_solve_p_after_run_has_its_own_statistics(sgpu_mod, precision):
         assert a.last_solve_stats() == b.last_solve_stats()
         assert a.warm_start_stats() == b.warm_start_stats()
         assert bit_equal(a.download(sgpu_mod.F_PC), b.download(sgpu_mod.F_PC))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_launch_count_holds_every_cycle(sgpu_mod, precision):
+    """sgpu_launch_count counts the kernels of each cycle of a captured solve, not those of one: the launches of a
+    run grow with the cycles it does as those of host-issued iterations do."""
+    def launches(cap, host):
+        p = _params(sgpu_mod, 160, 96, precision, pressure_tolerance="1e-300", pressure_maxit=str(cap))
+        with sgpu_mod.Solver(p) as s:
+            s.run(2)  # builds the graph
+            before = sgpu_mod.launch_count()
+            if host:
+                for _ in range(5):
+                    s.outer_iteration()
+            else:
+                s.run(5)
+            assert s.last_solve_stats()["mg_vcycles"] == cap
+            return sgpu_mod.launch_count() - before
+    run = [launches(c, False) for c in (1, 2, 5)]
+    host = [launches(c, True) for c in (1, 2)]
+    assert run[2] - run[1] == 3 * (run[1] - run[0])
+    assert run[1] - run[0] >= host[1] - host[0] > 0
