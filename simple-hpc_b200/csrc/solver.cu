@@ -530,6 +530,11 @@ struct Solver {
         launch_p_links_app(dp, cu.a[8], cv.a[8], w, st);
         p_links_stale = false;
     }
+    // An uploaded field is not to be formed anew, nor the others from what it replaces.
+    void before_upload(int id) {
+        if (id == SGPU_F_PC) pc_stale = false;
+        else form_p_links_if_stale(id == SGPU_F_CU_AP || id == SGPU_F_CV_AP ? SGPU_F_APP : id);
+    }
     MomRec32 rec32{};                 // per-cell FP32 records: coefficients, 1/AP, R
     unsigned* corr_err = nullptr;     // device word: a record sweep's bounded wait gave up
     // Every call that runs a solve or a sweep reports a bounded wait that gave up since the last check (its
@@ -1991,6 +1996,7 @@ int sgpu_upload(sgpu_handle* h, int id, const double* host) {
         if (h->s->is_coef(id)) h->s->need_coefs();
         double* f = h->s->field_ptr(id);
         if (!f) throw sgpu::Error(SGPU_E_INVALID, "sgpu_upload: unknown field id " + std::to_string(id));
+        h->s->before_upload(id);
         h->s->upload(f, host);
         h->s->sync();
     });

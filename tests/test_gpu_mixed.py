@@ -200,3 +200,25 @@ def test_cluster_sweep_matches_streaming_sweep(sgpu_mod, monkeypatch, nx, ny, sc
     assert bit_equal(l0, l1)
     for a, b in zip(f0, f1):
         assert bit_equal(a, b)
+
+
+@pytest.mark.parametrize("runs", [1, 2])
+def test_uploaded_pressure_arrays_stay(sgpu_mod, runs):
+    """p' and the p' operator of a mixed iteration exist in FP64 only once somebody asks for them: what a caller
+    uploads is not formed over, and the arrays beside it are those of the run."""
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x="40", N_cells_y="56", momentum_solver="gs_multicolour", pressure_solver="mg", precision="mixed",
+               maxit="50", error_tolerance="0")
+    p = sgpu_mod.params_from_config(config_text(cfg))
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for _ in range(runs):
+            for s in (a, b):
+                s.run(3)
+                s.download(sgpu_mod.F_PC), s.download(sgpu_mod.F_APP)
+        a.run(2), b.run(2)
+        mine = np.random.default_rng(1).standard_normal((p.nrows, p.ncols))
+        for f in (sgpu_mod.F_PC, sgpu_mod.F_AEP, sgpu_mod.CU[8]):
+            a.upload(f, mine)
+            assert bit_equal(a.download(f), mine), f"field {f}"
+        for f in range(sgpu_mod.F_AEP + 1, sgpu_mod.F_PC):
+            assert bit_equal(a.download(f), b.download(f)), f"field {f}"
