@@ -96,7 +96,11 @@ struct Solver {
     DevParams dp{};
     Grid g;
     cudaStream_t st = nullptr;
-    std::vector<void*> allocs;
+    struct Alloc {
+        void* p;
+        std::size_t bytes;
+    };
+    std::vector<Alloc> allocs;
     std::size_t bytes = 0;
 
     double *u = nullptr, *v = nullptr, *pf = nullptr;
@@ -181,7 +185,7 @@ struct Solver {
         void* p = nullptr;
         const std::size_t nb = count * sizeof(T);
         SGPU_CUDA(cudaMalloc(&p, nb > 0 ? nb : 1));
-        allocs.push_back(p);
+        allocs.push_back({p, nb});
         bytes += nb;
         SGPU_CUDA(cudaMemsetAsync(p, 0, nb > 0 ? nb : 1, st));
         return static_cast<T*>(p);
@@ -353,8 +357,9 @@ struct Solver {
         }
     }
     void dfree(void* q) {
-        const auto it = std::find(allocs.begin(), allocs.end(), q);
+        const auto it = std::find_if(allocs.begin(), allocs.end(), [q](const Alloc& a) { return a.p == q; });
         if (it == allocs.end()) return;
+        bytes -= it->bytes;
         allocs.erase(it);
         cudaFree(q);
     }
@@ -1169,7 +1174,7 @@ Solver::~Solver() {
     }
     if (side) cudaStreamDestroy(side);
 
-    for (void* q : allocs) cudaFree(q);
+    for (const Alloc& a : allocs) cudaFree(a.p);
     if (host_res) cudaFreeHost(host_res);
     if (st) cudaStreamDestroy(st);
 }

@@ -69,3 +69,34 @@ def test_coefficient_arrays_appear_with_the_per_phase_calls(sgpu_mod, oracle_mod
         for f in sgpu_mod.CU:
             a, b = (x[p.H:p.H + 250, p.H:p.H + 241].copy() for x in (g.download(f), o.get(f)))
             assert bit_equal(a, b), f"field {f}: " + describe_diff(a, b)
+
+
+def test_records_given_up_for_the_coefficient_arrays(sgpu_mod):
+    """A device that has no memory left for the coefficient arrays of a per-phase call: the handle gives up its
+    records (87 MB here) for them, accounts for both, and goes on with the same bits."""
+    import torch
+    n = 1024
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x=str(n), N_cells_y=str(n), momentum_solver="gs_multicolour", pressure_solver="mg", maxit="9",
+               error_tolerance="0")
+    p = sgpu_mod.params_from_config(config_text(cfg))
+    field = p.nrows * (-(-p.ncols // 32) * 32) * 8
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for s in (a, b):
+            s.run(1)
+        b.assemble_u()
+        before = a.memory_bytes()
+        free = torch.cuda.mem_get_info()[0]
+        hog = torch.empty(free - (100 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            a.assemble_u()
+            after = a.memory_bytes()
+            a.run(2)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        b.run(2)
+        assert b.memory_bytes() == before + 16 * field
+        assert before - 5 * 2 * field * 1.1 < after - 16 * field <= before - 5 * 2 * field
+        for f in (0, 1, 2, sgpu_mod.F_PC, sgpu_mod.CU[0], sgpu_mod.CU[7]):
+            assert bit_equal(a.download(f), b.download(f)), f"field {f}"
