@@ -125,6 +125,7 @@ void launch_mg_coarse(const LevelViewT<T>& L, double* rowbuf, double tol, int* s
 template <class T> struct MgLevelsT {
     LevelViewT<T> L[24];
     int n;
+    bool clusters; // cluster kernels may take its tail and its coarsest level (mg_clusters_enabled)
 };
 using MgLevels = MgLevelsT<double>;
 // Levels [first, n) of one V-cycle in one CTA: down-leg, coarse solve, up-leg (mg_vcycle order). x of
@@ -139,6 +140,9 @@ void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double
 // the device or the grid does not allow it. launch_mg_tail_cluster returns false (and launches nothing)
 // where it does not apply from `first`.
 template <class T> int mg_cluster_tail_first(const MgLevelsT<T>& lv, int fallback);
+// False with SGPU_MG_CLUSTER=0: the solvers created while it is set run their tail as streamed levels and on one
+// CTA, the coarsest level on one CTA, as on a device without such clusters.
+bool mg_clusters_enabled();
 template <class T>
 bool launch_mg_tail_cluster(const MgLevelsT<T>& lv, int first, int pre, int post, double omega, double tol,
                             int* sweeps_out, cudaStream_t st, bool build);

@@ -659,7 +659,7 @@ constexpr int kCoarseSmemMax = 160 * 1024;
 // portable cluster. 37 x 37 FP64, 200 sweeps: 0.28 ms (one warp on shared memory: 6.31 ms); 75 x 125
 // FP32, 200 sweeps: 0.23 ms in a cluster of 8 (one CTA on global memory: 5.63 ms).
 template <class T>
-bool launch_coarse_pairs(const LevelViewT<T>& L, double tol, int* sweeps_out, cudaStream_t st) {
+bool launch_coarse_pairs(const LevelViewT<T>& L, bool clusters, double tol, int* sweeps_out, cudaStream_t st) {
     CoarseBands pl{};
     auto plan = [&](int ctas) {
         pl.rows = (L.nx + ctas - 1) / ctas;
@@ -679,6 +679,7 @@ bool launch_coarse_pairs(const LevelViewT<T>& L, double tol, int* sweeps_out, cu
         SGPU_LAUNCH();
         return true;
     }
+    if (!clusters) return false;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -729,7 +730,7 @@ template <class T>
 void launch_mg_tail(const MgLevelsT<T>& lv, int first, int pre, int post, double omega, double tol,
                     double* rowbuf, int* sweeps_out, cudaStream_t st, bool build) {
     const LevelViewT<T>& Lc = lv.L[lv.n - 1];
-    if (first == lv.n - 1 && launch_coarse_pairs(Lc, tol, sweeps_out, st)) return;
+    if (first == lv.n - 1 && launch_coarse_pairs(Lc, lv.clusters, tol, sweeps_out, st)) return;
     // pair solve inside the tail: a thread of the block per pair
     const bool pairs = static_cast<long long>(Lc.nx) * coarse_hp(Lc.ny) <= kCoarseThreads;
     TailSmem ts{};
@@ -801,6 +802,10 @@ void launch_mg_sub_mean(const LevelView& L, double* x, const double* sum, cudaSt
     k_mg_sub_mean<<<grid2(L.nx, L.ny), dim3(BX, BY), 0, st>>>(L, x, sum);
     SGPU_LAUNCH();
 }
+bool mg_clusters_enabled() {
+    const char* e = std::getenv("SGPU_MG_CLUSTER");
+    return !e || std::atoi(e) != 0;
+}
 #endif
 
 namespace {
@@ -845,11 +850,7 @@ template <class T> bool cluster_tail_plan(const MgLevelsT<T>& lv, int first, Clu
 
 // Whether this device runs the cluster tail: its function attributes set (the dynamic shared memory
 // and the non-portable cluster size, once per device) and at least one such cluster resident.
-// SGPU_MG_CLUSTER=0 turns it off for the solvers created while it is set (their tail then runs as
-// streamed levels and the single-CTA tail, as without a cluster).
 template <class T> bool cluster_tail_available() {
-    if (const char* e = std::getenv("SGPU_MG_CLUSTER"))
-        if (std::atoi(e) == 0) return false;
     static PerDeviceOnce once;
     return once.get([] {
         // a device that refuses either attribute runs the kernels without a cluster
@@ -881,7 +882,7 @@ template <class T> bool cluster_tail_available() {
 } // namespace
 
 template <class T> int mg_cluster_tail_first(const MgLevelsT<T>& lv, int fallback) {
-    if (!cluster_tail_available<T>()) return fallback;
+    if (!lv.clusters || !cluster_tail_available<T>()) return fallback;
     int t = 0;
     while (t < lv.n - 1 && lv.L[t].nx * lv.L[t].ny > kClusterTailCells<T>) ++t;
     ClusterTailPlan pl{};

@@ -301,7 +301,7 @@ struct Solver {
         const bool deferred = defer_sums();
         const int n = vcomp ? prm.maxit_inner_v : prm.maxit_inner_u;
         // small grids: assembly, residual and sweeps in one cluster launch (timed as the sweeps)
-        if (n > 0 && mom_cluster_fits(dp, vcomp)) {
+        if (n > 0 && on_cluster[vcomp ? 1 : 0]) {
             mark(vcomp ? SGPU_PH_SWEEP_V : SGPU_PH_SWEEP_U);
             sweep_mark(vcomp, 0, n);
             launch_mom_cluster(dp, vcomp, x, oth, pf, AP, cplane, n, st);
@@ -333,8 +333,17 @@ struct Solver {
     // cluster. Where the device has no memory for them (or SGPU_MOM_RECORDS=0) the sweeps recompute the
     // coefficients: the same bits.
     MomRec64 rec64{};
+    // The components (u, v) that run on a cluster instead (k_mom_cluster). SGPU_MOM_CLUSTER=0: none, for the
+    // solvers created while it is set, as on a device without such clusters.
+    bool on_cluster[2] = {false, false};
+    void choose_cluster() {
+        if (!fast || mixed) return;
+        if (const char* e = std::getenv("SGPU_MOM_CLUSTER"))
+            if (std::atoi(e) == 0) return;
+        for (int k = 0; k < 2; ++k) on_cluster[k] = mom_cluster_fits(dp, k == 1);
+    }
     void alloc_records() {
-        if (!fast || mixed || (mom_cluster_fits(dp, false) && mom_cluster_fits(dp, true))) return;
+        if (!fast || mixed || (on_cluster[0] && on_cluster[1])) return;
         if (const char* e = std::getenv("SGPU_MOM_RECORDS"))
             if (std::atoi(e) == 0) return;
         const std::size_t n =
@@ -1097,6 +1106,7 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
             }
         }
         mgl.n = nl;
+        mgl.clusters = mgl32.clusters = mg_clusters_enabled();
         for (int l = 0; l < nl && l < 24; ++l) mgl.L[l] = lv[l];
         mg_tail64 = mg_fast ? mg_cluster_tail_first(mgl, mg_tail) : mg_tail;
     }
@@ -1153,6 +1163,7 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
         net = own_net.get();
     }
 
+    choose_cluster();
     alloc_records(); // last: everything a solve cannot do without has its memory
     if (hu) upload(u, hu);
     if (hv) upload(v, hv);

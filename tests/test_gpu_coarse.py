@@ -125,3 +125,24 @@ def test_right_hand_sides_whose_squares_underflow(sgpu_mod, oracle_mod, nx, ny, 
         g.solve_p()
         assert g.last_solve_stats()["coarse_sweeps"] == o.mg_last_coarse_sweeps()
         assert bit_equal(g.download(sgpu_mod.F_PC), o.get(sgpu_mod.F_PC))
+
+
+@pytest.mark.parametrize("nx,ny", [(46, 45), (131, 133), (150, 250), (128, 128)])
+def test_without_clusters(sgpu_mod, oracle_mod, monkeypatch, nx, ny):
+    """SGPU_MG_CLUSTER=0 (and a device without clusters): the coarsest levels of more pairs than one CTA has threads
+    on the general loop, tails on one CTA. Bit for bit the oracle's, and other launches than with clusters."""
+    p = sgpu_mod.params_from_config(_cfg(nx, ny))
+    o = oracle_mod.Oracle(p)
+    _, _, olog = o.run(2)
+    seconds = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("SGPU_MG_CLUSTER", on)
+        with sgpu_mod.Solver(p) as g:
+            _, log = g.run(2)
+            assert bit_equal(log, olog), describe_diff(log, olog)
+            for f in (0, 1, 2, sgpu_mod.F_PC):
+                assert bit_equal(g.download(f), o.get(f)), f"field {f}: " + describe_diff(g.download(f), o.get(f))
+            assert g.last_solve_stats()["coarse_sweeps"] == o.mg_last_coarse_sweeps()
+            seconds.append(min(g.run(10)[0].seconds for _ in range(3)))
+    if nx != 128:  # one CTA on global memory takes several times the cluster's time: the switch was heeded
+        assert seconds[1] > 1.5 * seconds[0], seconds

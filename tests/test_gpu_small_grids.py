@@ -100,3 +100,28 @@ def test_records_given_up_for_the_coefficient_arrays(sgpu_mod):
         assert before - 5 * 2 * field * 1.1 < after - 16 * field <= before - 5 * 2 * field
         for f in (0, 1, 2, sgpu_mod.F_PC, sgpu_mod.CU[0], sgpu_mod.CU[7]):
             assert bit_equal(a.download(f), b.download(f)), f"field {f}"
+
+
+@pytest.mark.parametrize("nx,ny,scheme,order,inner", [(3, 200, "QUICK", 2, 3), (50, 90, "QUICK", 2, 2), (130, 101, "QUICK", 4, 5),
+                                                      (96, 96, "UDS", 2, 4)])
+def test_small_grids_without_the_cluster(sgpu_mod, oracle_mod, monkeypatch, nx, ny, scheme, order, inner):
+    """What a device without such clusters runs, and SGPU_MOM_CLUSTER=0 selects: the sweeps from stored and from
+    recomputed coefficients, on grids that otherwise run on the cluster."""
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(N_cells_x=str(nx), N_cells_y=str(ny), Re="700", convection_scheme=scheme, diffusion_order=str(order),
+               momentum_solver="gs_multicolour", pressure_solver="gs_redblack", maxit="6", error_tolerance="0",
+               maxit_inner_u=str(inner), maxit_inner_v=str(inner))
+    p = sgpu_mod.params_from_config(config_text(cfg))
+    o = oracle_mod.Oracle(p)
+    _, _, olog = o.run(6)
+    bytes_held = []
+    for cluster, records in (("1", "1"), ("0", "1"), ("0", "0")):
+        monkeypatch.setenv("SGPU_MOM_CLUSTER", cluster)
+        monkeypatch.setenv("SGPU_MOM_RECORDS", records)
+        with sgpu_mod.Solver(p) as g:
+            _, log = g.run(6)
+            assert bit_equal(log, olog), describe_diff(log, olog)
+            for f in (0, 1, 2, sgpu_mod.F_PC):
+                assert bit_equal(g.download(f), o.get(f)), f"field {f}: " + describe_diff(g.download(f), o.get(f))
+            bytes_held.append(g.memory_bytes())
+    assert bytes_held[0] == bytes_held[2] < bytes_held[1]  # the second one did take the records
