@@ -201,6 +201,10 @@ int sgpu_selftest_bounded_wait(int polls, int* gave_up);
  * SGPU_E_TIMEOUT, and the one after it run normally. Nothing is launched. SGPU_E_INVALID for a handle
  * without such waits. */
 int sgpu_selftest_set_timeout(sgpu_handle* h);
+/* Diagnostic: out[i] = a[i] / ap[i], i < n, on the current device as the FP64 red-black updates form the
+ * quotient (from an inverse of ap, several ranges of exponents); equal bit for bit to the IEEE division. Host
+ * arrays. */
+int sgpu_selftest_quotient(const double* a, const double* ap, int n, double* out);
 /* Number of multigrid levels and the dims of level l (mg_level_dims, multigrid.cpp:143-151). */
 int sgpu_mg_levels(int NX, int NY, int* nlevels, int* dims /* 2 * 64 ints, may be NULL */);
 /* Statistics of the last solve_p: CG iterations, MG V-cycles, coarsest-level sweeps. */

@@ -140,12 +140,12 @@ __device__ __forceinline__ double rb_value(double b, double nb, double ap) { ret
 // (P. Markstein, IBM J. Res. Dev. 34(1), 1990); a y can be two ulps off, so the step is taken twice, the
 // first bringing q within one. Five dependent operations, 41 cycles against the division's 113, and no
 // branch that keeps two of them from overlapping. The exponent bounds keep y, q and r normal numbers;
-// outside them (inverse returns 0 for such an AP), and for infinities and NaN, it divides.
+// outside them (inverse returns 0 for such an AP), and for infinities and NaN, see quotient_rare.
 __device__ __forceinline__ double inverse(double ap) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(ap)); // the sign bit fails the test too
     return (hi >> 20) - 923u <= 200u ? 1.0 / ap : 0.0;             // 2^-100 <= AP < 2^101
 }
-// The quotient, or slow set where it takes a division.
+// The quotient, or slow set where it takes quotient_rare.
 __device__ __forceinline__ double quotient_try(double a, double ap, double y, bool& slow) {
     const unsigned hi = static_cast<unsigned>(__double2hiint(a));
     const bool zero = ((hi << 1) | static_cast<unsigned>(__double2loint(a))) == 0u;
@@ -156,14 +156,30 @@ __device__ __forceinline__ double quotient_try(double a, double ap, double y, bo
     slow |= !(mid || zero) || __double2hiint(y) == 0;
     return zero ? a : q; // AP > 0 keeps a zero's sign
 }
-__device__ __forceinline__ double divided(double a, double ap) {
-    asm volatile("" : "+d"(a)); // the division stays inside the caller's branch
+// The quotient where quotient_try gave none. A red-black solve of a cavity started from rest has p' falling off
+// over hundreds of decades ahead of what the sweeps have reached, so dividends too small for the steps above are
+// common there, and the division takes its long path for them (in the level sweeps three in a row: a red-black
+// iteration on 1024 x 128, UDS, 20 to 60 iterations from rest 275 -> 243 us, QUICK 400 -> 360). So they are scaled: a 2^300 and its quotient q are normal
+// numbers, q 2^-300 rounds once more only where it is subnormal, and that gives another number than one rounding
+// only from a q half way between two subnormal ones (q is the rounded quotient and such a point is a number
+// itself, so any other q lies on the quotient's side of it), where it divides.
+__device__ __forceinline__ double quotient_rare(double a, double ap, double y) {
+    asm volatile("" : "+d"(a)); // stays inside the caller's branch
+    const unsigned hi = static_cast<unsigned>(__double2hiint(a));
+    if (((hi >> 20) & 0x7ffu) < 123u && __double2hiint(y) != 0) {
+        const double s = a * 0x1p300;
+        double q = s * y;
+        q = __fma_rn(__fma_rn(-ap, q, s), y, q);
+        q = __fma_rn(__fma_rn(-ap, q, s), y, q);
+        const double r = q * 0x1p-300;
+        if (fabs(q - r * 0x1p300) != 0x1p-775) return a == 0.0 ? a : r;
+    }
     return a / ap;
 }
 __device__ __forceinline__ double quotient(double a, double ap, double y) {
     bool slow = false;
     double q = quotient_try(a, ap, y, slow);
-    if (slow) q = divided(a, ap);
+    if (slow) q = quotient_rare(a, ap, y);
     return q;
 }
 __device__ __forceinline__ float rb_value(float b, float nb, float ap) {

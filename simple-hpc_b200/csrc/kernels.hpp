@@ -143,6 +143,8 @@ template <class T> int mg_cluster_tail_first(const MgLevelsT<T>& lv, int fallbac
 // False with SGPU_MG_CLUSTER=0: the solvers created while it is set run their tail as streamed levels and on one
 // CTA, the coarsest level on one CTA, as on a device without such clusters.
 bool mg_clusters_enabled();
+// out[i] = a[i] / ap[i] as the FP64 red-black updates form it (quotient() in common.hpp), for a check of its own.
+void launch_quotient(const double* a, const double* ap, int n, double* out, cudaStream_t st);
 template <class T>
 bool launch_mg_tail_cluster(const MgLevelsT<T>& lv, int first, int pre, int post, double omega, double tol,
                             int* sweeps_out, cudaStream_t st, bool build);

@@ -802,6 +802,17 @@ void launch_mg_sub_mean(const LevelView& L, double* x, const double* sum, cudaSt
     k_mg_sub_mean<<<grid2(L.nx, L.ny), dim3(BX, BY), 0, st>>>(L, x, sum);
     SGPU_LAUNCH();
 }
+namespace {
+__global__ void k_quotient(const double* a, const double* ap, int n, double* out) {
+    const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < n) out[i] = quotient(a[i], ap[i], inverse(ap[i]));
+}
+} // namespace
+void launch_quotient(const double* a, const double* ap, int n, double* out, cudaStream_t st) {
+    if (n <= 0) return;
+    k_quotient<<<(n + 255) / 256, 256, 0, st>>>(a, ap, n, out);
+    SGPU_LAUNCH();
+}
 bool mg_clusters_enabled() {
     const char* e = std::getenv("SGPU_MG_CLUSTER");
     return !e || std::atoi(e) != 0;

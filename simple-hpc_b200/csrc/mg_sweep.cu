@@ -116,9 +116,9 @@ __device__ __forceinline__ void update(bool ok0, bool ok1, T b0, T nb0, T nb1, S
         v0 = quotient_try(nb0, z.ap, z.y, slow0);
         v1 = quotient_try(nb1, sw.ap, sw.y, slow1);
         if ((ok0 && slow0) || (ok1 && slow1)) {
-            z.t0 = divided(b0, z.ap);
-            v0 = divided(nb0, z.ap);
-            v1 = divided(nb1, sw.ap);
+            z.t0 = quotient_rare(b0, z.ap, z.y);
+            v0 = quotient_rare(nb0, z.ap, z.y);
+            v1 = quotient_rare(nb1, sw.ap, sw.y);
         }
         v0 = z.t0 + v0;
         v1 = sw.t0 + v1;

@@ -2045,6 +2045,25 @@ int sgpu_selftest_bounded_wait(int polls, int* gave_up) {
     });
 }
 
+int sgpu_selftest_quotient(const double* a, const double* ap, int n, double* out) {
+    if (!a || !ap || !out || n < 0) return sgpu::fail(SGPU_E_INVALID, "sgpu_selftest_quotient: bad arguments");
+    return guarded([&] {
+        double* d = nullptr;
+        const std::size_t nb = sizeof(double) * static_cast<std::size_t>(n);
+        SGPU_CUDA(cudaMalloc(&d, 3 * nb + 1));
+        try {
+            SGPU_CUDA(cudaMemcpy(d, a, nb, cudaMemcpyHostToDevice));
+            SGPU_CUDA(cudaMemcpy(d + n, ap, nb, cudaMemcpyHostToDevice));
+            sgpu::launch_quotient(d, d + n, n, d + 2 * static_cast<std::size_t>(n), nullptr);
+            SGPU_CUDA(cudaMemcpy(out, d + 2 * static_cast<std::size_t>(n), nb, cudaMemcpyDeviceToHost));
+        } catch (...) {
+            cudaFree(d);
+            throw;
+        }
+        SGPU_CUDA(cudaFree(d));
+    });
+}
+
 int sgpu_selftest_set_timeout(sgpu_handle* h) {
     SGPU_NEED_HANDLE(h);
     return guarded([&] {

@@ -110,6 +110,7 @@ def lib() -> C.CDLL:
             "sgpu_memory_bytes": (I, [H, C.POINTER(C.c_size_t)]),
             "sgpu_selftest_bounded_wait": (I, [I, C.POINTER(I)]),
             "sgpu_selftest_set_timeout": (I, [H]),
+            "sgpu_selftest_quotient": (I, [D, D, I, D]),
             "sgpu_mg_levels": (I, [I, I, C.POINTER(I), C.POINTER(I)]),
             "sgpu_last_solve_stats": (I, [H, C.POINTER(I), C.POINTER(I), C.POINTER(I), D]),
             "sgpu_ordered_sum": (I, [D, I, I, D]),
@@ -361,6 +362,16 @@ def selftest_bounded_wait(polls: int = 4096) -> bool:
     out = C.c_int(0)
     _check(lib().sgpu_selftest_bounded_wait(int(polls), C.byref(out)))
     return bool(out.value)
+
+
+def selftest_quotient(a: np.ndarray, ap: np.ndarray) -> np.ndarray:
+    """a / ap as the FP64 red-black updates form it (sgpu_selftest_quotient)."""
+    a, ap = (np.ascontiguousarray(x, dtype=np.float64).ravel() for x in (a, ap))
+    if a.size != ap.size:
+        raise ValueError(f"{a.size} dividends, {ap.size} divisors")
+    out = np.empty_like(a)
+    _check(lib().sgpu_selftest_quotient(_dptr(a), _dptr(ap), a.size, _dptr(out)))
+    return out
 
 
 def ordered_sum(values: np.ndarray) -> float:
