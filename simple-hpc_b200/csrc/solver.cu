@@ -274,6 +274,16 @@ struct Solver {
     void solve_p();
     void correct() { launch_correct(dp, w, cu.a[8], cv.a[8], u, v, pf, st); }
 
+    // The level sweeps walk 28 rows and more per CTA, 13 us a pass however small the grid, where a launch per colour
+    // takes 2 us while the grid is in L2. Measured, us a red-black iteration (8 sweeps of p') of a developed flow
+    // and of one near rest, sweeps / colours: 128^2 110 / 101 and 112 / 101 (UDS), 1024 x 128 280 / 268 and
+    // 361 / 320 (QUICK), 1024^2 527 / 536 and 625 / 603, 1200^2 634 / 656 and 739 / 719, 1300^2 700 / 777 and
+    // 811 / 838, 1900^2 1155 / 1505 and 1322 / 1597. Where cavities share the GPU, launches cost more than steps:
+    // 148 of 64^2 576 / 934 a round, 7 of 512^2 733 / 836, 256 of 64 to 512 a side 6371 / 9257 (but four of 64^2
+    // 144 / 138, a batch of no more cavities than keep a single solve's shape).
+    static constexpr std::size_t kSweepCells = 1200000;
+    bool shares_gpu = false;
+    bool sweeps_pay() const { return shares_gpu || plane > kSweepCells; }
     void solve_redblack();
     void solve_jacobi();
     void solve_cg();
@@ -1226,7 +1236,7 @@ void Solver::sweep_v(int n) {
 void Solver::solve_redblack() {
     SGPU_CUDA(cudaMemsetAsync(w.pc, 0, g.bytes(), st));
     int k = 0;
-    if (own_links) { // two sweeps per pass, to the other of pc and tmp each time and to pc at last
+    if (own_links && sweeps_pay()) { // two sweeps per pass, to the other of pc and tmp each time and to pc at last
         const std::size_t o = p_origin();
         LevelView L{prm.NX, prm.NY, g.pitch, w.AEP + o, nullptr, w.ANP + o, nullptr, nullptr, w.b + o, nullptr, nullptr};
         const int passes = prm.maxit_inner_p / 2;
@@ -2398,6 +2408,7 @@ int sgpu_batch_create(const sgpu_params_t* params, int count, sgpu_batch** out) 
         for (const sgpu::Solver* sv : by_size) cells += sv->plane;
         const std::size_t first = cells <= sgpu::Solver::kBatchCells ? sgpu::Solver::kBatchLatency : 0;
         for (std::size_t c = first; c < by_size.size(); ++c) by_size[c]->use_batch_shape();
+        for (sgpu::Solver* sv : by_size) sv->shares_gpu = first < by_size.size();
         SGPU_CUDA(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking));
         b->seg_tuned.assign(count, 0);
         for (auto& sv : b->s) sv->sync();

@@ -34,3 +34,28 @@ def test_red_black_solver(sgpu_mod, oracle_mod, nx, ny, sweeps):
                                             (360, 348, 2, 2), (2048, 20, 2, 2)])
 def test_v_cycle(sgpu_mod, oracle_mod, nx, ny, pre, post):
     _check(sgpu_mod, oracle_mod, nx, ny, 3, pressure_solver="mg", mg_pre=str(pre), mg_post=str(post))
+
+
+@pytest.mark.parametrize("nx,ny,sweeps", [(10400, 116, 2), (10300, 117, 3), (5200, 232, 4), (5170, 233, 5), (3450, 349, 8),
+                                          (40, 30011, 6)])
+def test_red_black_solver_in_two_sweep_passes(sgpu_mod, oracle_mod, nx, ny, sweeps):
+    """The same at the size from which a single solve takes two sweeps a pass (smaller ones launch a colour each)."""
+    assert nx * ny > 1200000
+    _check(sgpu_mod, oracle_mod, nx, ny, 2, pressure_solver="gs_redblack", maxit_inner_p=str(sweeps))
+
+
+@pytest.mark.parametrize("nx,ny,sweeps", [(1, 3, 1), (2, 2, 2), (20, 116, 2), (21, 117, 3), (41, 232, 4), (19, 233, 5),
+                                          (130, 349, 8), (349, 5, 6)])
+def test_red_black_solver_of_a_batch_cavity(sgpu_mod, oracle_mod, nx, ny, sweeps):
+    """The cavities of a batch of more than eight take two sweeps a pass at any size."""
+    cfg = dict(snapshot_config("short_16"))
+    cfg.update(Re="700", momentum_solver="gs_multicolour", maxit="4", error_tolerance="0", pressure_solver="gs_redblack",
+               maxit_inner_p=str(sweeps))
+    big = sgpu_mod.params_from_config(config_text(dict(cfg, N_cells_x="400", N_cells_y="300")))
+    p = sgpu_mod.params_from_config(config_text(dict(cfg, N_cells_x=str(nx), N_cells_y=str(ny))))
+    o = oracle_mod.Oracle(p)
+    o.run(4)
+    with sgpu_mod.Batch([big] * 8 + [p]) as b:
+        b.run(4)
+        for f in (0, 1, 2, sgpu_mod.F_PC):
+            assert bit_equal(b.download(8, f), o.get(f)), f"field {f}: " + describe_diff(b.download(8, f), o.get(f))
