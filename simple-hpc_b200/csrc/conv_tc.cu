@@ -472,40 +472,61 @@ constexpr int kWgSmemPair = 110 * 1024; // the weight gradient's share with two 
 // in flight, first MMA, epilogue), per CTA its bytes at about 60 B/ns, its MMAs (an MMA reads its 4 KB of
 // A in about 20 ns, more with many output channels) and its stores. Narrow tiles waste product rows on
 // halo columns, wide or tall ones leave SMs idle on a single image.
+// Where the weights of all output channels do not fit beside a tile (128 -> 128), that leaves one CTA of few
+// output channels on an SM, whose copies wait for nobody's MMAs. There 16 channels at a time, for 64 output
+// channels or more, are tried too: small tiles, several CTAs on an SM, one's copies beside another's MMAs, at
+// about 0.6 us a chunk; taken where the estimate is well below the other's. A base of 128 channels, one level,
+// us a forward call, all channels at once / 16 at a time: 2 x 16 x 1024 200 / 161, 1 x 128^2 138 / 126,
+// 1 x 256^2 291 / 217, 1 x 512^2 944 / 685 (8 x 32^2: 132 either way, all at once).
 ConvPlan conv_plan(int N, int H, int W, int cin, int cout) {
-    ConvPlan best{};
-    double best_ns = 1e30;
-    int kc = cin;
-    if (kc > 128)
-        for (kc = 128; cin % kc; kc -= 16) {}
+    int whole = cin;
+    if (whole > 128)
+        for (whole = 128; cin % whole; whole -= 16) {}
     const int wr = (W + 7) / 8 * 8;
-    for (int cw : {8, 16, 32, 48, 64, 96, 128}) {
-        if (cw > wr && cw != 8) continue;
-        const int P = cw + 2;
-        for (int tb : {1, 2, 3, 4, 6, 8}) {
-            const int rb = std::min(H, 128 * tb / P);
-            if (rb < 1 || (tb > 1 && 128 * (tb - 1) >= rb * P)) continue;
-            for (int nt = cout; nt >= 16; nt = nt % 32 ? nt - 16 : nt / 2) {
-                if (cout % nt || tb * nt > 512) continue;
-                const long lp = 128L * tb + 2 * P + 2; // pixels a shifted block may read
-                const long smem = lp * 16 * (kc / 8) + 9L * kc * nt * 2;
-                if (smem > kConvSmemMax) continue;
-                uint32_t cols = 32;
-                while (cols < static_cast<uint32_t>(tb * nt)) cols <<= 1;
-                const long occ = std::min({227L * 1024 / (smem + 1024), 512L / cols, 8L});
-                const long ct = (W + cw - 1) / cw, rc = (H + rb - 1) / rb;
-                const long ctas = ct * rc * N * (cout / nt), chunks = cin / kc;
-                const double bytes = static_cast<double>((rb + 2) * P * 2L * cin + 18L * cin * nt);
-                const double mma = 9.0 * (cin / 16) * tb * std::max(20.0, 0.3 * nt);
-                const double ns = static_cast<double>((ctas + 148 * occ - 1) / (148 * occ)) * (1000.0 + 1000.0 * chunks) +
-                                  static_cast<double>((ctas + 147) / 148) * (bytes / 60.0 + mma + tb * nt * 2.0);
-                if (ns < best_ns) {
-                    best_ns = ns;
-                    best = {cw, rb, tb, nt, kc, static_cast<int>(chunks), static_cast<int>(ct), static_cast<int>(rc),
-                            static_cast<unsigned>(lp * 16), static_cast<int>(smem), cols};
+    // the best plan that brings in kc channels at a time and forms at least nt_min output channels; its time in ns
+    auto search = [&](int kc, int nt_min, double& best_ns) {
+        ConvPlan best{};
+        best_ns = 1e30;
+        for (int cw : {8, 16, 32, 48, 64, 96, 128}) {
+            if (cw > wr && cw != 8) continue;
+            const int P = cw + 2;
+            for (int tb : {1, 2, 3, 4, 6, 8}) {
+                const int rb = std::min(H, 128 * tb / P);
+                if (rb < 1 || (tb > 1 && 128 * (tb - 1) >= rb * P)) continue;
+                for (int nt = cout; nt >= nt_min; nt = nt % 32 ? nt - 16 : nt / 2) {
+                    if (cout % nt || tb * nt > 512) continue;
+                    const long lp = 128L * tb + 2 * P + 2; // pixels a shifted block may read
+                    const long smem = lp * 16 * (kc / 8) + 9L * kc * nt * 2;
+                    if (smem > kConvSmemMax) continue;
+                    uint32_t cols = 32;
+                    while (cols < static_cast<uint32_t>(tb * nt)) cols <<= 1;
+                    const long occ = std::min({227L * 1024 / (smem + 1024), 512L / cols, 8L});
+                    const long ct = (W + cw - 1) / cw, rc = (H + rb - 1) / rb;
+                    const long ctas = ct * rc * N * (cout / nt), chunks = cin / kc;
+                    const double copies = static_cast<double>((rb + 2) * P * 2L * cin + 18L * cin * nt) / 60.0;
+                    const double mma = 9.0 * (cin / 16) * tb * std::max(20.0, 0.3 * nt);
+                    const double waves = static_cast<double>((ctas + 148 * occ - 1) / (148 * occ));
+                    const double per_sm = static_cast<double>((ctas + 147) / 148);
+                    const double together = std::min(static_cast<double>(occ), per_sm);
+                    const double ns =
+                        (kc == whole ? waves * (1000.0 + 1000.0 * chunks) + per_sm * (copies + mma)
+                                     : waves * std::max(1000.0 + 600.0 * chunks + copies + mma, together * std::max(copies, mma))) +
+                        per_sm * (tb * nt * 2.0);
+                    if (ns < best_ns) {
+                        best_ns = ns;
+                        best = {cw, rb, tb, nt, kc, static_cast<int>(chunks), static_cast<int>(ct), static_cast<int>(rc),
+                                static_cast<unsigned>(lp * 16), static_cast<int>(smem), cols};
+                    }
                 }
             }
         }
+        return best;
+    };
+    double ns = 0.0, ns16 = 0.0;
+    ConvPlan best = search(whole, 16, ns);
+    if (whole > 16 && 9L * whole * cout * 2 > kConvSmemMax) {
+        const ConvPlan chunked = search(16, 64, ns16);
+        if (ns16 < 0.7 * ns) best = chunked;
     }
     return best;
 }

@@ -55,3 +55,24 @@ def test_epilogue_of_partly_live_warps(sgpu_mod, n, h, w, base):
     for (cin, cout, _), (wo, bo) in zip(o.convs, o.offs):
         assert rel_l2(g[wo:bo], rg[wo:bo]) < 1e-2
         assert rel_l2(g[bo:bo + cout], rg[bo:bo + cout]) < 1e-2
+
+
+@pytest.mark.parametrize("n,h,w", [(4, 64, 64), (1, 70, 187), (2, 250, 50)])
+def test_wide_convolutions_in_channel_chunks(sgpu_mod, n, h, w):
+    """128 to 128 channels, whose weights do not fit beside a tile: images large enough to come in 16 channels at a
+    time. Bounds as above."""
+    import cnn_oracle
+    params = cnn_oracle.init_params(128, 1, seed=n + h + w)
+    rng = np.random.default_rng(3)
+    x = rng.normal(size=(n, h, w, 2)).astype(np.float32)
+    t = rng.normal(size=(n, h, w)).astype(np.float32)
+    with sgpu_mod.Cnn(128, 1) as net:
+        net.set_params(params)
+        out = net.forward(x)
+        _, g = net.loss_grad(x, t)
+    o = cnn_oracle.UNetOracle(128, 1)
+    _, rg, ref = o.loss_grad(params, x, t)
+    assert rel_l2(out, ref) < 5e-3
+    for (cin, cout, _), (wo, bo) in zip(o.convs, o.offs):
+        assert rel_l2(g[wo:bo], rg[wo:bo]) < 1e-2
+        assert rel_l2(g[bo:bo + cout], rg[bo:bo + cout]) < 1e-2
