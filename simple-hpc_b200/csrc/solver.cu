@@ -346,6 +346,8 @@ struct Solver {
     // The components (u, v) that run on a cluster instead (k_mom_cluster). SGPU_MOM_CLUSTER=0: none, for the
     // solvers created while it is set, as on a device without such clusters.
     bool on_cluster[2] = {false, false};
+    // Whether an iteration launches the streaming momentum sweep at all (a mixed one may).
+    bool streams_sweeps() const { return mixed || !(on_cluster[0] && on_cluster[1]); }
     void choose_cluster() {
         if (!fast || mixed) return;
         if (const char* e = std::getenv("SGPU_MOM_CLUSTER"))
@@ -2444,6 +2446,10 @@ int sgpu_batch_autotune(sgpu_batch* b, int* chosen) {
             if (it == best.end()) {
                 const int heur = sv.seg_rows;
                 std::vector<int> cand = {heur};
+                if (!sv.streams_sweeps()) { // nothing launches with this height: the heuristic's, untimed
+                    sv.seg_rows = b->seg_tuned[c] = best.emplace(key, heur).first->second;
+                    continue;
+                }
                 for (int k : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
                     if (8 * sv.dp.ncol * k <= sv.dp.nrows + 8 * sv.dp.ncol) cand.push_back(8 * sv.dp.ncol * k);
                 cudaEvent_t e0, e1;

@@ -144,3 +144,16 @@ def test_run_graph_equals_host_loop(sgpu_mod, extra, capfd):
     # the same progress lines from both paths
     half = len(printed) // 2
     assert printed[:half] == printed[half:] and printed[0].startswith("iter 1 ")
+
+
+def test_autotune_times_only_sweeps_that_run(sgpu_mod):
+    """FP64 cavities whose components run on a cluster launch no streaming sweep: the autotuner has nothing to time
+    there (and reports the heuristic's height); a larger one it times."""
+    small = [cavity(64, 300), cavity(96, 700)]
+    for cases, timed in ((small, False), (small + [cavity(300, 500)], True)):
+        with sgpu_mod.Batch([sgpu_mod.params_from_config(config_text(c)) for c in cases]) as b:
+            before = sgpu_mod.launch_count()
+            chosen = b.autotune()
+            assert (sgpu_mod.launch_count() > before) == timed
+            assert all(s > 0 for s in chosen)
+            b.run(3)
