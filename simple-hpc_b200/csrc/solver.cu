@@ -144,11 +144,16 @@ struct Solver {
     // bound by each CTA's per-step latency on small grids, so it takes short segments (8 rows); a
     // batch fills the GPU with many cavities and keeps the kernels' defaults (0), which bound the
     // halo and skew work per row (use_batch_shape). A batch that does not fill the GPU is bound by the
-    // latency of its largest cavities, so while the batch has at most kBatchCells cells in all its
+    // latency of its largest cavities, so while the batch has at most kBatchCells cells in all, its
     // kBatchLatency largest keep a single solve's shape (as many as the GPU holds 16-CTA tail clusters at
-    // once). Measured, us a round with the batch shape for all and with 8 excepted: 20 cavities of 64^2 to
-    // 512^2 (0.8 M cells) 612 and 441, four of 512^2 (1.05 M) 614 and 446, eight of 384^2 (1.2 M) 624 and 498,
-    // eight of 512^2 (2.1 M) 743 and 796, sixteen 1074 and 1404.
+    // once), as far as they are larger than the next one: it would bound the batch just as long, and the
+    // shape of the others would only take SM time from it. Measured, us a round with the batch shape for all, with the
+    // eight largest excepted and by this rule: 20 cavities of 64^2 to 512^2 (0.8 M cells) 563, 435 and 434 mixed,
+    // 715, 662 and 664 FP64; one of 512^2 and eight of 192^2 512, 359 and 347, 662, 505 and 446; four of 384^2 and ten of
+    // 128^2 536, 394 and 390, 672, 597 and 567; sixteen of 192^2 311, 340 and 311, 385, 467 and 385. Where the limit
+    // lies, batch shape and excepted: mixed, eight of 384^2 (1.18 M) 564 and 490, six of 512^2 (1.6 M) 611 and
+    // 587, seven (1.8 M) 634 and 676; FP64, six of 384^2 (0.9 M) 701 and 646, eight 739 and 826, five of 512^2 (1.3 M)
+    // 790 and 894.
     static constexpr int kBatchLatency = 8;
     static constexpr std::size_t kBatchCells = 1200000;
     int min_seg = 8;
@@ -2408,7 +2413,10 @@ int sgpu_batch_create(const sgpu_params_t* params, int count, sgpu_batch** out) 
         });
         std::size_t cells = 0;
         for (const sgpu::Solver* sv : by_size) cells += sv->plane;
-        const std::size_t first = cells <= sgpu::Solver::kBatchCells ? sgpu::Solver::kBatchLatency : 0;
+        const std::size_t next = sgpu::Solver::kBatchLatency;
+        const std::size_t bound = by_size.size() > next ? by_size[next]->plane : 0; // the largest that could not be excepted
+        std::size_t first = 0;
+        while (cells <= sgpu::Solver::kBatchCells && first < std::min(next, by_size.size()) && by_size[first]->plane > bound) ++first;
         for (std::size_t c = first; c < by_size.size(); ++c) by_size[c]->use_batch_shape();
         for (sgpu::Solver* sv : by_size) sv->shares_gpu = first < by_size.size();
         SGPU_CUDA(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking));

@@ -157,3 +157,28 @@ def test_autotune_times_only_sweeps_that_run(sgpu_mod):
             assert (sgpu_mod.launch_count() > before) == timed
             assert all(s > 0 for s in chosen)
             b.run(3)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_equal_cavities_take_one_shape(sgpu_mod, precision):
+    """The largest cavities of a small batch keep a single solve's kernels only where they are larger than the others:
+    equal ones all launch the same, however many they are (a mixture shows as another average). Same bits
+    as a single run in either shape."""
+    def per_cavity(sizes):
+        with sgpu_mod.Batch([sgpu_mod.params_from_config(config_text(cavity(n, 300, precision=precision))) for n in sizes]) as b:
+            b.run(1)
+            before = sgpu_mod.launch_count()
+            b.run(6)
+            u = b.download(0, 0)
+            return sgpu_mod.launch_count() - before, u
+    nine, u9 = per_cavity([256] * 9)
+    more, u14 = per_cavity([256] * 14)
+    fixed = 2 + 2 * 6  # the graph's own kernels
+    assert (nine - fixed) % (9 * 6) == 0 and (more - fixed) // (14 * 6) == (nine - fixed) // (9 * 6)
+    eight, _ = per_cavity([256] * 8)
+    assert (eight - fixed) // (8 * 6) < (nine - fixed) // (9 * 6)  # a single solve's shape: fewer, larger launches
+    p = sgpu_mod.params_from_config(config_text(cavity(256, 300, precision=precision)))
+    with sgpu_mod.Solver(p) as s:
+        s.run(7)
+        if precision == "fp64":
+            assert bit_equal(u9, s.download(0)) and bit_equal(u14, u9)
