@@ -87,3 +87,36 @@ def test_launch_count_holds_every_cycle(sgpu_mod, precision):
     host = [launches(c, True) for c in (1, 2)]
     assert run[2] - run[1] == 3 * (run[1] - run[0])
     assert run[1] - run[0] >= host[1] - host[0] > 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny", [(5, 1), (1, 1)])
+def test_solves_of_no_cycle(sgpu_mod, precision, nx, ny):
+    """One column of cells has no u cells, so the lid drives nothing: b is zero, the loop runs no cycle, and p' and
+    the statistics are those of the host's early return, not the previous solve's."""
+    p = _params(sgpu_mod, nx, ny, precision)
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for n in (1, 2):
+            _, log = a.run(n)
+            rows = np.array([b.outer_iteration() for _ in range(n)])
+            assert bit_equal(np.ascontiguousarray(log[:, 1:]), rows) and not rows[:, 2].any()
+            assert a.last_solve_stats() == b.last_solve_stats()
+            assert a.last_solve_stats()["mg_vcycles"] == 0
+            for f in (0, 1, 2, sgpu_mod.F_PC):
+                assert bit_equal(a.download(f), b.download(f)), f"field {f}"
+        # a solve of no cycle after one of several: its p' is zero again
+        for s in (a, b):
+            s.upload(sgpu_mod.F_V, np.random.default_rng(2).standard_normal(s.shape))
+        for n in (1, 1):
+            _, log = a.run(n)
+            assert bit_equal(np.ascontiguousarray(log[:, 1:]), np.array([b.outer_iteration()]))
+            assert a.last_solve_stats() == b.last_solve_stats()
+            assert bit_equal(a.download(sgpu_mod.F_PC), b.download(sgpu_mod.F_PC))
+        for s in (a, b):
+            for f in (0, 1, 2):
+                s.upload(f, np.zeros(s.shape))
+        _, log = a.run(1)
+        assert bit_equal(np.ascontiguousarray(log[:, 1:]), np.array([b.outer_iteration()]))
+        for f in (0, 1, 2, sgpu_mod.F_PC):
+            assert bit_equal(a.download(f), b.download(f)), f"field {f}"
+        assert not a.download(sgpu_mod.F_PC).any() and a.last_solve_stats()["mg_vcycles"] == 0
