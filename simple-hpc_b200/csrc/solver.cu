@@ -166,7 +166,14 @@ struct Solver {
     }
 
     int ncol = 5;
-    IterGraph* run_graph = nullptr; // sgpu_run's graph (built on first use)
+    // sgpu_run's graphs, by mg_mode, built on first use; the tolerance-driven one holds its tolerance and cap
+    IterGraph* run_graph[2] = {nullptr, nullptr};
+    double graph_tolerance = 0.0;
+    int graph_maxit = 0;
+    void destroy_graph(int mode) {
+        destroy_iter_graph(run_graph[mode]);
+        run_graph[mode] = nullptr;
+    }
 
     // learned warm start (warm_start = cnn, or a network attached through the C ABI)
     std::unique_ptr<UNet> own_net;
@@ -416,8 +423,7 @@ struct Solver {
                     if (q) dfree(q);
                 if (e.code != SGPU_E_NOMEM || attempt || !rec64.r[0]) throw;
                 sync();
-                destroy_iter_graph(run_graph); // it holds the records
-                run_graph = nullptr;
+                for (int mode : {0, 1}) destroy_graph(mode); // they hold the records
                 free_records();
                 set_seg_rows(min_seg);
             }
@@ -1190,7 +1196,7 @@ Solver::Solver(const sgpu_params_t& p, const double* hu, const double* hv, const
 
 Solver::~Solver() {
     if (st) cudaStreamSynchronize(st);
-    destroy_iter_graph(run_graph);
+    for (int mode : {0, 1}) destroy_graph(mode);
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : sw_ev)
@@ -1855,8 +1861,15 @@ static bool graphable(const sgpu::Solver& s) {
 static bool run_graphed(sgpu::Solver& s, int maxit, double* log, int print_every, sgpu_result_t& out,
                         bool& diverged, int start = 0, const double* maxr = nullptr) {
     if (s.profiling || maxit < 1 || start >= maxit || !graphable(s)) return false;
-    if (!s.run_graph) s.run_graph = new sgpu::IterGraph({&s}, maxit);
-    sgpu::IterGraph& g = *s.run_graph;
+    const bool tolerant = s.prm.mg_mode == SGPU_MG_TOLERANCE;
+    if (tolerant && (s.graph_tolerance != s.prm.pressure_tolerance || s.graph_maxit != s.prm.pressure_maxit)) s.destroy_graph(1);
+    sgpu::IterGraph*& graph = s.run_graph[tolerant ? 1 : 0];
+    if (!graph) graph = new sgpu::IterGraph({&s}, maxit);
+    if (tolerant) {
+        s.graph_tolerance = s.prm.pressure_tolerance;
+        s.graph_maxit = s.prm.pressure_maxit;
+    }
+    sgpu::IterGraph& g = *graph;
     g.ensure_log(maxit);
     g.reset(s.st);
     if (start > 0) g.resume(s.st, start, maxr);
@@ -1891,7 +1904,11 @@ static bool run_graphed(sgpu::Solver& s, int maxit, double* log, int print_every
                              sizeof(double) * 4 * static_cast<std::size_t>(done - start), cudaMemcpyDeviceToHost));
     g.count(done - start, done - start);
     if (done > start) { // what iteration_enqueue notes on the host when it launches an iteration
-        s.tol_stats = s.prm.pressure_solver == SGPU_P_MG && s.prm.mg_mode == SGPU_MG_TOLERANCE;
+        s.tol_stats = s.prm.pressure_solver == SGPU_P_MG && tolerant;
+        if (s.prm.pressure_solver == SGPU_P_MG && !tolerant) {
+            s.last_vcycles = s.prm.mg_cycles;
+            s.pc_dc_src = nullptr;
+        }
         if (s.tol_stats) { // an iteration's count holds one pass of its cycle loop
             const long long cycles = tol.total - s.tol_total;
             sgpu::count_launches((cycles - (done - start)) * s.cycle_launches);
@@ -2341,12 +2358,6 @@ int sgpu_set_mg_mode(sgpu_handle* h, int mg_mode, double pressure_tolerance, int
         sgpu::Solver& s = *h->s;
         s.sync();
         s.fetch_tol();
-        // a captured iteration holds the old mode, tolerance and cap
-        if (s.run_graph && (s.prm.mg_mode != mg_mode || s.prm.pressure_tolerance != pressure_tolerance ||
-                            s.prm.pressure_maxit != pressure_maxit)) {
-            sgpu::destroy_iter_graph(s.run_graph);
-            s.run_graph = nullptr;
-        }
         s.prm.mg_mode = mg_mode;
         s.prm.pressure_tolerance = pressure_tolerance;
         s.prm.pressure_maxit = pressure_maxit;

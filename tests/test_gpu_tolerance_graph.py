@@ -120,3 +120,23 @@ def test_solves_of_no_cycle(sgpu_mod, precision, nx, ny):
         for f in (0, 1, 2, sgpu_mod.F_PC):
             assert bit_equal(a.download(f), b.download(f)), f"field {f}"
         assert not a.download(sgpu_mod.F_PC).any() and a.last_solve_stats()["mg_vcycles"] == 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_graphs_of_both_modes_side_by_side(sgpu_mod, precision):
+    """Switching between the modes keeps each one's graph: runs of either between runs of the other, tolerances that
+    change and come back, and host-issued iterations in between give the host's results, p' and statistics too."""
+    p = _params(sgpu_mod, 64, 96, precision)
+    plan = [(False,), (True, 1e-6, 50), (False,), (True, 1e-6, 50), (False, 1e-3, 7), (True, 1e-2, 50), (True, 1e-6, 50), (False,)]
+    with sgpu_mod.Solver(p) as a, sgpu_mod.Solver(p) as b:
+        for k, mode in enumerate(plan):
+            a.set_mg_mode(*mode)
+            b.set_mg_mode(*mode)
+            for hosted in ((True, False) if k % 3 == 2 else (False,)):
+                rows = np.array([b.outer_iteration() for _ in range(2)])
+                log = np.array([a.outer_iteration() for _ in range(2)]) if hosted else np.ascontiguousarray(a.run(2)[1][:, 1:])
+                assert bit_equal(log, rows), f"{k}: {mode}"
+            got, want = a.last_solve_stats(), b.last_solve_stats()
+            assert got == want, f"{k}: {mode}"
+            for f in (0, 1, 2, sgpu_mod.F_PC):
+                assert bit_equal(a.download(f), b.download(f)), f"{k}: {mode}, field {f}"
