@@ -34,8 +34,9 @@ enum {
     SGPU_E_INVALID = -1,     /* bad argument, unsupported solver combination, bad config */
     SGPU_E_CUDA = -2,        /* a CUDA runtime call failed (message holds cudaGetErrorString) */
     SGPU_E_NOMEM = -3,       /* a device allocation failed */
-    SGPU_E_TIMEOUT = -4,     /* a bounded device-side wait ran out (persistent kernels; the mixed
-                                mode's correction sweep waiting for its record copies) */
+    SGPU_E_TIMEOUT = -4,     /* a bounded device-side wait ran out: a momentum sweep's for its record
+                                copies, the one-kernel CG solve's for the other blocks' sums, a
+                                convolution's for its MMAs */
     SGPU_E_NONFINITE = -5,   /* a residual became NaN or Inf: sgpu_run stopped the diverged run */
     SGPU_E_NODEVICE = -6     /* no CUDA device is visible */
 };
@@ -193,7 +194,7 @@ int sgpu_upload(sgpu_handle* h, int field_id, const double* host);
 int sgpu_memory_bytes(sgpu_handle* h, size_t* bytes);
 /* Diagnostic of the device-side failure detection (no counterpart in the reference): one warp on the
  * current device waits, at most `polls` polls (1 .. 1 << 20), on an mbarrier that nothing completes,
- * through the same bounded-wait helper the mixed mode's correction sweep uses. *gave_up = 1 when the
+ * through the same bounded-wait helper the momentum sweeps use. *gave_up = 1 when the
  * wait ended by giving up and reported it, as it must; the GPU context stays usable. */
 int sgpu_selftest_bounded_wait(int polls, int* gave_up);
 /* The same for the reporting (no counterpart in the reference): leaves the handle's error words as a wait
@@ -241,7 +242,8 @@ int sgpu_ordered_sum_noalloc(const double* values, int nrows_v, int ncols_v, int
  * sgpu_launch_count returns the number of kernel launches this library has issued in the process.
  * sgpu_sweep_seconds returns the device time of the streaming momentum sweep kernels alone (the
  * FP64 sweep, or the FP32 correction sweep with precision = mixed) and how many were launched, both
- * accumulated over the profiled iterations: the per-launch time of the dominant kernel.
+ * accumulated over the profiled iterations: the per-launch time of the dominant kernel. A small grid's
+ * cluster kernel holds all sweeps of a component (in FP64 its assembly too) and counts as that many launches.
  */
 /* on: 0 off; 1 every iteration host-issued between events (exact per-phase device times, slower);
  * 2 sampled: sgpu_run times the phases of its first 10 iterations that way, replays the captured
@@ -342,7 +344,8 @@ int sgpu_batch_create(const sgpu_params_t* params /* count */, int count, sgpu_b
 int sgpu_batch_destroy(sgpu_batch* b);
 int sgpu_batch_count(sgpu_batch* b, int* count);
 /* Autotuner: per distinct grid, times the candidate row-segment heights of the streaming momentum
- * sweep and keeps the fastest (chosen[count], 0 for cavities without that sweep; may be NULL). The
+ * sweep and keeps the fastest (chosen[count], 0 for cavities without that sweep; may be NULL). FP64
+ * cavities whose sweeps run on a cluster are not timed and report the heuristic's height. The
  * segment height changes no result bit. Call before sgpu_batch_run. */
 int sgpu_batch_autotune(sgpu_batch* b, int* chosen);
 /* Run every cavity to its tolerance or maxit iterations from its current fields. log_cap > 0 keeps
